@@ -138,7 +138,9 @@ struct DevPlan {
     int8_t tri[SGE_MAX_K];
     uint8_t trel[2];                              // relation of slot j in `tries`
     uint8_t tkey[2][3];                           // key levels of slot j, in the trie's key order
-    uint8_t ntrie, pad2_[3];
+    uint8_t ntrie;
+    uint8_t dcls;                                 // dense path: universe class + 1, 0 = lists only (dense.cuh)
+    uint8_t pad2_[2];
     // labeled matching (sge_plan_set_labels): vlab = the data graph's vertex
     // labels (null: unlabeled), lab[i] = the label of level i's pattern vertex
     const uint32_t *vlab;
@@ -1669,6 +1671,15 @@ __global__ void heavy_prefix_kernel(DevGraph g, const DevPlan *__restrict__ plan
     if (lane == 0) H.tot[p] = run;
 }
 
+// Root task t is counted on bitsets (dense.cuh): dskip holds, per sampled
+// root edge, the universe classes that were built.
+__device__ __forceinline__ bool dense_counts_root(const DevPlan &P, const uint8_t *dskip, unsigned long long t) {
+    const bool any = P.root_kind == SGE_ROOT_ANY, swap = any ? (t & 1) : P.root_kind == SGE_ROOT_DESC;
+    uint32_t c = P.dcls - 1u;   // N(m0) and N(m1) change places when the root runs reversed
+    if (swap && (c == 1u || c == 2u)) c = 3u - c;
+    return (__ldg(dskip + (any ? t >> 1 : t)) >> c) & 1u;
+}
+
 // Phase 0 counts every root, except that a root whose level-2 bound exceeds
 // split_H is appended to its plan's heavy list (while there is room) instead.
 // Phase 1 runs each heavy root as ceil(bound / S) × P3 tasks: task (c, q)
@@ -1684,7 +1695,8 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
                                                     uint32_t *scratch, uint32_t cap, uint32_t bufs_per_warp,
                                                     uint32_t tw, uint32_t tmode, unsigned long long deadline_ns,
                                                     uint32_t *flags, DevStats *stats, uint32_t phase, HeavyBuf H,
-                                                    uint32_t ntd, uint32_t cs, uint32_t nvs, uint32_t ntr) {
+                                                    uint32_t ntd, uint32_t cs, uint32_t nvs, uint32_t ntr,
+                                                    const uint8_t *dskip) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t lane = lane_id();
     const uint32_t wib = threadIdx.x >> 5;
@@ -1697,14 +1709,15 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
     c.set_ops = c.alg_bytes = c.partial = 0;
     WarpState &W = setup_warp(smem_raw, wib, tw, tmode, ntd, cs, nvs, c, ntr);
     unsigned long long roots = 0;
-    // The time budget covers both launch phases: phase 0's first block
-    // records its start next to the flags, and phase 1 measures from there.
+    // The time budget covers the whole launch: its first kernel (phase 0, or
+    // the selection of dense roots) records its start next to the flags, and
+    // the later ones measure from there.
     unsigned long long tstart = 0;
     unsigned long long *t0_slot = reinterpret_cast<unsigned long long *>(flags + 2);
     if (lane == 0) {
         tstart = globaltimer_ns();
-        if (phase == 0 && blockIdx.x == 0 && wib == 0) *t0_slot = tstart;
-        else if (phase == 1 && *(volatile unsigned long long *)t0_slot) tstart = *(volatile unsigned long long *)t0_slot;
+        if (phase == 0 && !dskip && blockIdx.x == 0 && wib == 0) *t0_slot = tstart;
+        else if ((phase == 1 || dskip) && *(volatile unsigned long long *)t0_slot) tstart = *(volatile unsigned long long *)t0_slot;
     }
     c.tstart = __shfl_sync(FULL_MASK, tstart, 0);
     c.deadline = deadline_ns;
@@ -1782,6 +1795,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
             continue;
         }
         for (unsigned long long t = t0; t < t1; ++t) {
+            if (dskip && P.dcls && dense_counts_root(P, dskip, t)) continue;
             const uint2 e = root_edge(g, P, t);
             if (!root_kept(g, P, e)) continue;
             ++roots;
@@ -1808,6 +1822,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
     }
 }
 
+#include "dense.cuh"
 
 // ------------------------------------------------------------ enumeration --
 // Writes every match of a plan (all k levels enumerated, no counting tail)
@@ -1922,6 +1937,8 @@ struct sge_graph {
     uint32_t hub_words = 0, hub_min = 0xFFFFFFFFu, hub_count = 0;
     uint64_t hub_bytes = 0;
     uint32_t *d_labels = nullptr;  // vertex labels (sge_graph_set_labels)
+    unsigned char *d_dense = nullptr;  // dense-root records and rows
+    size_t dense_bytes = 0;
 };
 
 namespace {
@@ -2136,6 +2153,20 @@ sge_status ensure_scratch(sge_graph *g, size_t bytes) {
     return SGE_OK;
 }
 
+// False when the device has no room: the launch then counts every root on lists.
+bool ensure_dense(sge_graph *g, size_t bytes) {
+    if (g->dense_bytes >= bytes) return true;
+    cudaFree(g->d_dense);
+    g->d_dense = nullptr;
+    g->dense_bytes = 0;
+    if (cudaMalloc(&g->d_dense, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    g->dense_bytes = bytes;
+    return true;
+}
+
 sge_status ensure_batch(sge_graph *g, size_t bytes) {
     if (g->batch_bytes >= bytes) return SGE_OK;
     if (g->d_batch) { cudaFree(g->d_batch); g->d_batch = nullptr; g->batch_bytes = 0; }
@@ -2240,7 +2271,74 @@ struct LaunchCfg {
     unsigned long long deadline = 0;
     size_t off_plans = 0, off_counts = 0, off_queue = 0, off_flags = 0, off_stats = 0, off_hcnt = 0, off_htot = 0,
            off_hids = 0, off_hpre = 0, off_ptime = 0, bytes_zeroed = 0, bytes = 0;
+    // dense roots (dense.cuh): the plans' universe classes and the layout of their buffer
+    // (header | edge classes | records | order | prefix | (plan, orientation) table | rows)
+    std::vector<DensePO> dpo;           // empty: every root is counted on lists
+    uint32_t dneed = 0, drows_both = 0, drec_cap = 0, dmaxdeg = 0;
+    unsigned long long dedges = 0, darena_units = 0, droot_offset = 0, droot_stride = 1;
+    size_t dense_blocks = 0, off_dskip = 256, off_drecs = 0, off_dorder = 0, off_dpre = 0, off_dpo = 0, off_darena = 0, dense_bytes = 0;
 };
+
+constexpr unsigned long long DENSE_ARENA_MAX = 1ull << 30;   // bytes of rows per launch
+constexpr uint32_t DENSE_REC_MAX = 1u << 17;                 // root edges per launch
+
+// No dense buffer: every root on lists.
+void drop_dense(LaunchCfg &L) {
+    L.dpo.clear();
+    for (auto &d : L.dps) d.dcls = 0;
+}
+
+// Chooses the plans whose dense roots are counted on bitsets and lays out
+// their buffer.  The instrumented kernel (its counters are defined on lists)
+// and runs with a caller's list capacity (which lists may overflow) keep to
+// the lists.
+void prepare_dense(const sge_graph *g, const sge_count_opts &o, size_t free_b, LaunchCfg &L) {
+    if (L.want_stats || o.max_level_capacity || g->max_deg < 2) return;
+    L.drows_both = 15u;
+    for (uint32_t i = 0; i < L.nplans; ++i) {
+        DevPlan &d = L.dps[i];
+        const int c = dense_class(d);
+        if (c < 0) continue;
+        d.dcls = (uint8_t)(c + 1);
+        const bool both = dense_rows_both(d);
+        for (uint32_t swap = 0; swap < 2; ++swap) {
+            if (d.root_kind != SGE_ROOT_ANY && swap != (d.root_kind == SGE_ROOT_DESC ? 1u : 0u)) continue;
+            const uint32_t ec = dense_edge_class((uint32_t)c, swap != 0);
+            L.dpo.push_back(DensePO{i, ec, swap});
+            L.dneed |= 1u << ec;
+            if (!both) L.drows_both &= ~(1u << ec);
+        }
+        L.droot_offset = d.root_offset;
+        L.droot_stride = d.root_stride;
+        L.dedges = d.root_kind == SGE_ROOT_ANY ? d.ntasks / 2 : d.ntasks;
+    }
+    if (L.dpo.empty() || !L.dedges) { L.dpo.clear(); return; }
+    L.dmaxdeg = o.root_max_degree;
+    const uint32_t deg = o.root_max_degree ? std::min(o.root_max_degree, g->max_deg) : g->max_deg;
+    unsigned long long units = 0;   // of one record whose universes are as large as the degrees allow
+    for (uint32_t c = 0; c < 4; ++c)
+        if ((L.dneed >> c) & 1u)
+            units += dense_units((uint32_t)std::min<unsigned long long>(DENSE_WORDS, (c == DENSE_UNION ? 2ull * deg : deg) / 32 + 3));
+    L.darena_units = std::min({L.dedges * units, DENSE_ARENA_MAX / 16, (unsigned long long)free_b / 16 / 16});
+    L.drec_cap = (uint32_t)std::min<unsigned long long>(L.dedges, DENSE_REC_MAX);
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    L.off_drecs = up(L.off_dskip + L.dedges);
+    L.off_dorder = up(L.off_drecs + sizeof(DenseRec) * (size_t)L.drec_cap);
+    L.off_dpre = up(L.off_dorder + 4 * (size_t)L.drec_cap);
+    L.off_dpo = up(L.off_dpre + 8 * (size_t)L.drec_cap);
+    L.off_darena = up(L.off_dpo + sizeof(DensePO) * L.dpo.size());
+    L.dense_bytes = L.off_darena + 16 * (size_t)L.darena_units;
+    int b = 0;
+    const size_t smem = 4 * sizeof(DenseWarp);
+    if (cudaFuncSetAttribute(dense_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, dense_count_kernel, 128, smem) != cudaSuccess || b < 1) {
+        cudaGetLastError();
+        drop_dense(L);
+        return;
+    }
+    if (o.blocks_per_sm) b = std::min<int>(b, (int)o.blocks_per_sm);
+    L.dense_blocks = (size_t)g->num_sms * b;
+}
 
 sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t nplans, const sge_count_opts &o,
                           size_t scratch_held, LaunchCfg &L) {
@@ -2385,13 +2483,14 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
     L.off_hpre = L.off_hids + (((size_t)L.heavy_cap * nplans * 4 + 255) & ~(size_t)255);
     L.bytes = L.off_hpre + (((size_t)L.heavy_cap * nplans * 8 + 255) & ~(size_t)255);
     if (o.time_budget_s > 0) L.deadline = std::max<unsigned long long>(1, (unsigned long long)(o.time_budget_s * 1e9));
+    prepare_dense(g, o, free_b, L);
     return SGE_OK;
 }
 
 // Stream-ordered: clear the counters, run phase 0 and (when roots may be
 // split) phase 1.  Capturable (no host synchronisation).
-sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, uint32_t *scratch, cudaStream_t s,
-                          uint32_t &launches) {
+sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, uint32_t *scratch, unsigned char *dense,
+                          cudaStream_t s, uint32_t &launches) {
     CUDA_TRY(cudaMemsetAsync(B + L.off_counts, 0, L.bytes_zeroed - L.off_counts, s));
     DevGraph dg = dev_graph(g, L.use_hubs);
     const DevPlan *dplans = reinterpret_cast<const DevPlan *>(B + L.off_plans);
@@ -2404,6 +2503,32 @@ sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, ui
                reinterpret_cast<unsigned long long *>(B + L.off_htot),
                reinterpret_cast<unsigned long long *>(B + L.off_ptime), L.heavy_cap};
     launches = 0;
+    const uint8_t *dskip = nullptr;
+    if (!L.dpo.empty()) {
+        DenseBuf D{};
+        D.hdr = reinterpret_cast<uint32_t *>(dense);
+        D.skip = dense + L.off_dskip;
+        D.recs = reinterpret_cast<DenseRec *>(dense + L.off_drecs);
+        D.order = reinterpret_cast<uint32_t *>(dense + L.off_dorder);
+        D.pre = reinterpret_cast<unsigned long long *>(dense + L.off_dpre);
+        D.po = reinterpret_cast<const DensePO *>(dense + L.off_dpo);
+        D.arena = reinterpret_cast<uint4 *>(dense + L.off_darena);
+        D.arena_units = L.darena_units;
+        D.rec_cap = L.drec_cap;
+        D.npo = (uint32_t)L.dpo.size();
+        D.need = L.dneed;
+        D.rows_both = L.drows_both;
+        dskip = D.skip;
+        CUDA_TRY(cudaMemsetAsync(dense, 0, L.off_dskip + L.dedges, s));
+        const unsigned sel = (unsigned)std::min<unsigned long long>((L.dedges + 7) / 8, 16ull * g->num_sms);
+        dense_select_kernel<<<sel, 256, 0, s>>>(dg, L.droot_offset, L.droot_stride, L.dedges, L.dmaxdeg, D, dflags);
+        dense_build_kernel<<<8u * g->num_sms, 256, 0, s>>>(dg, D);
+        dense_prefix_kernel<<<1, 256, 0, s>>>(D);
+        dense_count_kernel<<<(unsigned)L.dense_blocks, 128, 4 * sizeof(DenseWarp), s>>>(dplans, D, dcounts, H.ptime,
+                                                                                       L.deadline, dflags);
+        CUDA_TRY(cudaGetLastError());
+        launches += 4;
+    }
     for (uint32_t phase = 0; phase < (L.any_split ? 2u : 1u); ++phase) {
         if (phase == 1) {
             CUDA_TRY(cudaMemsetAsync(dqueue, 0, 8 * (size_t)L.nplans, s));
@@ -2414,11 +2539,11 @@ sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, ui
         if (L.want_stats)
             count_kernel<true><<<(unsigned)L.blocks, L.threads, L.smem, s>>>(
                 dg, dplans, L.nplans, dqueue, dcounts, scratch, L.cap, L.nbufs, L.tw, L.tmode, L.deadline, dflags,
-                dstats, phase, H, L.ntd, L.cs, L.nvs, L.ntr);
+                dstats, phase, H, L.ntd, L.cs, L.nvs, L.ntr, dskip);
         else
             count_kernel<false><<<(unsigned)L.blocks, L.threads, L.smem, s>>>(
                 dg, dplans, L.nplans, dqueue, dcounts, scratch, L.cap, L.nbufs, L.tw, L.tmode, L.deadline, dflags,
-                dstats, phase, H, L.ntd, L.cs, L.nvs, L.ntr);
+                dstats, phase, H, L.ntd, L.cs, L.nvs, L.ntr, dskip);
         CUDA_TRY(cudaGetLastError());
         ++launches;
     }
@@ -2681,6 +2806,7 @@ sge_status sge_graph_destroy(sge_graph *g) {
     cudaFree(g->d_hub_bits);
     cudaFree(g->d_hub_slot);
     cudaFree(g->d_labels);
+    cudaFree(g->d_dense);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
     if (g->stream) cudaStreamDestroy(g->stream);
@@ -2776,11 +2902,15 @@ static sge_status count_impl(sge_graph *g, const sge_plan *const *plans, uint32_
     if (st != SGE_OK) return st;
     if ((st = ensure_scratch(g, L.scratch_bytes)) != SGE_OK) return st;
     if ((st = ensure_batch(g, L.bytes)) != SGE_OK) return st;
+    if (!L.dpo.empty() && !ensure_dense(g, L.dense_bytes)) drop_dense(L);
     unsigned char *B = g->d_batch;
+    if (!L.dpo.empty())
+        CUDA_TRY(cudaMemcpyAsync(g->d_dense + L.off_dpo, L.dpo.data(), sizeof(DensePO) * L.dpo.size(),
+                                 cudaMemcpyHostToDevice, g->stream));
     CUDA_TRY(cudaMemcpyAsync(B + L.off_plans, L.dps.data(), sizeof(DevPlan) * nplans, cudaMemcpyHostToDevice, g->stream));
     CUDA_TRY(cudaEventRecord(g->ev0, g->stream));
     uint32_t launches = 0;
-    if ((st = enqueue_launch(g, L, B, g->d_scratch, g->stream, launches)) != SGE_OK) return st;
+    if ((st = enqueue_launch(g, L, B, g->d_scratch, g->d_dense, g->stream, launches)) != SGE_OK) return st;
     g->launched = true;
     CUDA_TRY(cudaEventRecord(g->ev1, g->stream));
     std::vector<unsigned long long> hc(nplans);
@@ -2853,6 +2983,7 @@ struct sge_batch {
     sge_count_opts o{};
     unsigned char *d_buf = nullptr;
     uint32_t *d_scratch = nullptr;
+    unsigned char *d_dense = nullptr;
     unsigned char *h_res = nullptr;  // pinned: counts | flags | stats
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -2871,6 +3002,7 @@ sge_status sge_batch_destroy(sge_batch *b) {
     if (b->ev1) cudaEventDestroy(b->ev1);
     cudaFree(b->d_buf);
     cudaFree(b->d_scratch);
+    cudaFree(b->d_dense);
     if (b->h_res) cudaFreeHost(b->h_res);
     delete b;
     return SGE_OK;
@@ -2894,12 +3026,21 @@ sge_status sge_batch_create(sge_graph *g, const sge_plan *const *plans, uint32_t
         (e = cudaMallocHost(&b->h_res, res_bytes)) != cudaSuccess || (e = cudaEventCreate(&b->ev0)) != cudaSuccess ||
         (e = cudaEventCreate(&b->ev1)) != cudaSuccess)
         return bail(fail(SGE_OOM, "sge_batch_create: %s", cudaGetErrorString(e)));
+    if (!b->L.dpo.empty() && cudaMalloc(&b->d_dense, b->L.dense_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        b->d_dense = nullptr;
+        drop_dense(b->L);
+    }
+    if (!b->L.dpo.empty() &&
+        (e = cudaMemcpy(b->d_dense + b->L.off_dpo, b->L.dpo.data(), sizeof(DensePO) * b->L.dpo.size(),
+                        cudaMemcpyHostToDevice)) != cudaSuccess)
+        return bail(fail(SGE_CUDA_ERROR, "sge_batch_create: plan upload: %s", cudaGetErrorString(e)));
     if ((e = cudaMemcpy(b->d_buf + b->L.off_plans, b->L.dps.data(), sizeof(DevPlan) * nplans, cudaMemcpyHostToDevice)) != cudaSuccess)
         return bail(fail(SGE_CUDA_ERROR, "sge_batch_create: plan upload: %s", cudaGetErrorString(e)));
     // capture: clear counters, both launch phases, read back counts/flags/stats
     if ((e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return bail(fail(SGE_CUDA_ERROR, "stream capture: %s", cudaGetErrorString(e)));
-    st = enqueue_launch(g, b->L, b->d_buf, b->d_scratch, g->stream, b->launches);
+    st = enqueue_launch(g, b->L, b->d_buf, b->d_scratch, b->d_dense, g->stream, b->launches);
     if (st == SGE_OK) {
         cudaMemcpyAsync(b->h_res, b->d_buf + b->L.off_counts, 8 * (size_t)nplans, cudaMemcpyDeviceToHost, g->stream);
         cudaMemcpyAsync(b->h_res + 8 * (size_t)nplans, b->d_buf + b->L.off_flags, 4, cudaMemcpyDeviceToHost, g->stream);

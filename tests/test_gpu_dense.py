@@ -1,0 +1,45 @@
+"""Roots counted on bitsets (csrc/dense.cuh) against the list path and the CPU
+oracle.  A run with an explicit list capacity (here the largest degree, which
+no list exceeds) keeps every root on lists, so the two paths are compared on
+the same plans: one and two words per lane, universes that do not fit, the
+three tail modes, both join styles, root samples and degree caps."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def rooted(sge, p, stats, **kw):
+    import bench
+    seq, root = bench.canonical_symmetry(p.k, p.edges)
+    return sge.plan(p, stats, symmetry_seq=seq, root_edge=root, **kw)
+
+
+@pytest.mark.parametrize("exploration", [False, True])
+@pytest.mark.parametrize("iep", [False, True])
+@pytest.mark.parametrize("scale,m,stride,cap", [(9, 4000, 11, 0), (11, 20000, 97, 300), (13, 90000, 4999, 0)])
+def test_dense_roots_count_as_lists(sge, scale, m, stride, cap, iep, exploration):
+    ks = [(5, 10), (5, 9), (5, 8)] + [(6, 9 + i % 6) for i in range(24)] + [(7, 14 + i % 6) for i in range(18)]
+    if cap == 0 and scale > 11:
+        ks = [(5, 10), (6, 13), (6, 14), (6, 12), (6, 15), (5, 9)]
+    pats = [sge.PatternGraph.random(k, e, 700 + i) for i, (k, e) in enumerate(ks)]
+    with sge.Engine(sge.gen_rmat(scale, m, seed=scale)) as eng:
+        plans = [rooted(sge, p, eng, iep=iep, exploration=exploration) for p in pats]
+        opts = dict(root_stride=stride, root_offset=3, root_max_degree=cap)
+        got, inst, st = eng.count(plans, **opts)
+        want, winst, _ = eng.count(plans, max_level_capacity=eng.info()["max_degree"], **opts)
+        with eng.batch(plans, **opts) as b:
+            again = [b.run()[0] for _ in range(2)]
+    assert st["gpu_launches"] >= 5  # the bitset kernels ran
+    assert got == want and inst == winst
+    assert again == [want, want]
+    assert sum(got) > 0
+
+
+@pytest.mark.parametrize("k,m", [(5, 10), (6, 12), (6, 14), (7, 17), (7, 21), (8, 24)])
+def test_dense_counts_match_the_oracle(sge, oracle, k, m):
+    g = sge.gen_chung_lu(600, 3000, 2.1, 150, seed=5)
+    plans = [sge.plan(sge.PatternGraph.random(k, m, s), g, iep=iep) for s in (1, 2) for iep in (False, True)]
+    with sge.Engine(g) as eng:
+        got, _, _ = eng.count(plans)
+    want = [oracle.count_plan(g.offsets, g.nbrs, b, threads=0)[0] * b.count_multiplier % 2 ** 64 for b in plans]
+    assert got == want
