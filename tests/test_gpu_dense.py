@@ -43,3 +43,31 @@ def test_dense_counts_match_the_oracle(sge, oracle, k, m):
         got, _, _ = eng.count(plans)
     want = [oracle.count_plan(g.offsets, g.nbrs, b, threads=0)[0] * b.count_multiplier % 2 ** 64 for b in plans]
     assert got == want
+
+
+MIRROR_PATTERNS = {
+    "triangle": (3, [(0, 1), (0, 2), (1, 2)]),
+    "cycle4": (4, [(0, 1), (1, 2), (2, 3), (0, 3)]),
+    "k4": (4, [(0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3)]),
+    "star3": (4, [(0, 1), (0, 2), (0, 3)]),
+    "house": (5, [(0, 1), (0, 2), (0, 4), (1, 3), (1, 4), (2, 3)]),
+    "k5_minus_e": (5, [(a, b) for a in range(5) for b in range(a + 1, 5) if (a, b) != (3, 4)]),
+    "bull": (5, [(0, 1), (0, 2), (1, 2), (1, 3), (2, 4)]),
+}
+
+
+@pytest.mark.parametrize("exploration", [False, True])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_counts_do_not_depend_on_the_id_order(sge, oracle, reverse, exploration):
+    """Hubs at low ids (the reversed restrictions run) and at high ids (the
+    plan's own), with and without inclusion-exclusion."""
+    g = sge.gen_rmat(9, 3000, seed=3)
+    if reverse:
+        g = sge.DataGraph.from_edges(g.num_vertices - 1 - g.edge_array().astype("int64"), g.num_vertices)
+    plans = [sge.plan(sge.PatternGraph.from_edges(k, e), g, iep=iep, exploration=exploration)
+             for k, e in MIRROR_PATTERNS.values() for iep in (False, True)]
+    with sge.Engine(g) as eng:
+        got, _, _ = eng.count(plans)
+        split, _, _ = eng.count(plans, heavy_threshold=32)
+    want = [oracle.count_plan(g.offsets, g.nbrs, b, threads=0)[0] * b.count_multiplier for b in plans]
+    assert got == want and split == want
