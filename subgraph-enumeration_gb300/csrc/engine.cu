@@ -2473,12 +2473,24 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         const uint32_t split_P3 = split3 ? (tu.level3_parts ? std::min(tu.level3_parts, 1024u)
                                                             : (d.ne >= 6 ? 16u : 8u))
                                          : 1u;
-        const uint32_t deep = d.ne > 4 ? std::min<uint32_t>(d.ne - 4, 3u) : 0u;
-        const uint32_t split_S = split3 ? 1u : std::max<uint32_t>(128u >> (2 * deep), 2u);
+        // up to four enumerated levels: a task takes S level-2 candidates and
+        // repeats the root's setup.  128 keep that small where the roots
+        // alone give every warp 64 tasks; a sample's few roots are cut finer,
+        // down to 8 (K4 on 31,000 roots of R-MAT 2^18: 128 -> 11.4, 32 ->
+        // 3.5, 8 -> 3.2 ms; on all 2M of them 35.6, 42.7, 79.7 ms)
+        const uint32_t split_S = split3 ? 1u
+            : (uint32_t)std::min<unsigned long long>(128, std::max<unsigned long long>(8, 2ull * d.ntasks / warps));
         const double share = (double)d.ntasks * mean_deg / (double)std::max<unsigned long long>(warps, 1);
         const uint32_t thr = tu.heavy_threshold ? tu.heavy_threshold : o.heavy_threshold;
-        const uint32_t split_H = thr ? std::max(thr, 4u * split_S)
+        uint32_t split_H = thr ? std::max(thr, 4u * split_S)
                                : (uint32_t)std::min(1e9, std::max(32.0, share / 4.0));
+        // three enumerated levels over N(m0) ∩ N(m1) with a tail inside it: a
+        // root's work is the square of its list, which the share by list
+        // length does not see (K4 over every root of R-MAT 2^18: one root ran
+        // 287 ms; split from 1,024 on, 36 ms).  (A split root's repeated
+        // setup would count in the instrumented kernel's totals.)
+        if (!thr && !L.want_stats && d.ne == 3 && (d.parents[2] & 3u) == 3u && (d.tail_par & 4u))
+            split_H = std::min(split_H, std::max(8u * split_S, 256u));
         if (d.ne >= 3 && g->max_deg > split_H) {
             d.split_S = split_S;
             d.split_H = split_H;
