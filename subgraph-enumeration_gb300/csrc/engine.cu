@@ -543,11 +543,13 @@ __device__ __forceinline__ void wcoj_base(const DevPlan &P, const WarpState &W, 
 }
 
 // Warp-cooperative filter of [bp, bp+blen) by membership in all parent lists
-// of `rest` and by the exclusion set of level i; stores the survivors (in
-// order) to out when STORE.  Returns the survivor count (warp-uniform).
+// of `rest`, by the exclusion set of level i and (vlab: labeled plans whose
+// list no other level reuses) by its label; stores the survivors (in order)
+// to out when STORE.  Returns the survivor count (warp-uniform).
 template <bool STATS, bool STORE, bool EXCLUDE = true>
 __device__ __forceinline__ uint32_t setop(const DevPlan &P, const WarpState &W, Ctx<STATS> &c, uint32_t i,
-                                          const uint32_t *bp, uint32_t blen, uint32_t rest, uint32_t *out) {
+                                          const uint32_t *bp, uint32_t blen, uint32_t rest, uint32_t *out,
+                                          const uint32_t *vlab = nullptr) {
     const uint32_t lane = lane_id();
     if (STATS) {
         c.set_ops += 1;
@@ -562,6 +564,7 @@ __device__ __forceinline__ uint32_t setop(const DevPlan &P, const WarpState &W, 
         uint32_t idx = off + lane;
         bool ok = idx < blen;
         uint32_t x = ok ? bp[idx] : 0u;
+        if (vlab && ok) ok = __ldg(vlab + x) == P.lab[i];
         for (uint32_t msk = rest; msk && ok; msk &= msk - 1) ok = in_level_list(W, c, __ffs(msk) - 1, x);
         if (EXCLUDE && ok) ok = !excluded(P, W, i, x);
         uint32_t bal = __ballot_sync(FULL_MASK, ok);
@@ -587,9 +590,13 @@ __device__ __forceinline__ bool build_level_wcoj(const DevPlan &P, WarpState &W,
     if (!keep) trim(bp, blen, b);
     const uint32_t *fp = bp;
     uint32_t fl = blen;
-    if (rest != 0) {
+    // a labeled plan stores the level's own list filtered by its label (also
+    // where nothing is intersected), so that the levels below it run over the
+    // few candidates that remain, 32 at a time
+    const uint32_t *vlab = keep ? nullptr : P.vlab;
+    if (rest != 0 || (vlab && blen <= c.cap)) {
         uint32_t *out = c.buf + (size_t)i * c.cap;
-        uint32_t n = setop<STATS, true>(P, W, c, i, bp, blen, rest, out);
+        uint32_t n = setop<STATS, true>(P, W, c, i, bp, blen, rest, out, vlab);
         if (n > c.cap) {
             if (lane_id() == 0) atomicOr(c.flags, FLAG_OVERFLOW);
             return false;
@@ -609,7 +616,8 @@ __device__ __forceinline__ bool build_level_wcoj(const DevPlan &P, WarpState &W,
 
 // Hoisting: a tail level whose parents are all matched before the last
 // enumerated level gets its full intersection computed once, right after its
-// last parent is matched (bounds and exclusions are applied at the leaf).
+// last parent is matched (bounds and exclusions are applied at the leaf; a
+// labeled plan's label here, so that the leaf may count the list by its length).
 template <bool STATS>
 __device__ __forceinline__ bool hoist_after(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t j) {
     for (uint32_t msk = P.hoist_mask; msk; msk &= msk - 1) {
@@ -638,7 +646,7 @@ __device__ __forceinline__ bool hoist_after(const DevPlan &P, WarpState &W, Ctx<
             rest = P.parents[i] & ~(1u << best);
         }
         uint32_t *out = c.buf + (size_t)i * c.cap;
-        const uint32_t n = setop<STATS, true, false>(P, W, c, i, bp, blen, rest, out);
+        const uint32_t n = setop<STATS, true, false>(P, W, c, i, bp, blen, rest, out, P.vlab);
         __syncwarp();
         if (lane_id() == 0) W.hcnt[i] = n;
         __syncwarp();
@@ -975,7 +983,9 @@ __device__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<STA
         // scan: range size minus the matched vertices inside it (numResults)
         // (the last inclusion–exclusion pass probes no other tail level, so it
         // is a plain count too)
-        const bool direct = (P.tail_mode != SGE_TAIL_IEP || t + 1 == T) && D.nsrc == 1 && !P.vlab;
+        // (a labeled plan's only where the list holds that label alone)
+        const bool direct = (P.tail_mode != SGE_TAIL_IEP || t + 1 == T) && D.nsrc == 1 &&
+                            (!P.vlab || ((P.hoist_mask >> (ne + tp)) & 1u));
         if (direct) {
             if (lane < ncand) {
                 const uint32_t *fp = td_ptr(D, L, 0, lane);
@@ -1254,7 +1264,7 @@ __device__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32
             tail_desc(P, W, *c.L, c, lc, P.ne, S.ptd);
         }
         __syncwarp();
-        inl = S.ptd.nsrc == 1;
+        inl = S.ptd.nsrc == 1 && (!P.vlab || ((P.hoist_mask >> P.ne) & 1u));
     }
     const TailDesc &D = S.ptd;
     const uint32_t ns = S.ns, xpar = S.xpar, nex = S.nex;
@@ -1268,7 +1278,7 @@ __device__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32
         const uint32_t idx = b0 + lane;
         bool valid = idx < n;
         const uint32_t xv = valid ? lst[idx] : 0u;
-        if (valid) valid = !excluded(P, W, a, xv);  // (labeled plans take no pair step)
+        if (valid) valid = !rejected(P, W, a, xv);
         const uint32_t bal = __ballot_sync(FULL_MASK, valid);
         const uint32_t nc = __popc(bal);
         if (valid) S.x[__popc(bal & ((1u << lane) - 1u))] = xv;
@@ -1381,6 +1391,7 @@ __device__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32
                 if (keep && xpar && bsrc != -1) keep = pair_in(W, c, S, -1, l, y);
                 for (uint32_t e = 0; e < nex && keep; ++e) keep = y != S.exv[e];
                 if (keep && ex_x) keep = y != S.x[l];
+                if (P.vlab && keep) keep = __ldg(P.vlab + y) == P.lab[i];
             }
             if (inl) {
                 if (keep) {
@@ -2057,10 +2068,8 @@ void to_devplan(const sge_plan_blob &b, DevPlan &d) {
     for (uint32_t i = 0; i < SGE_MAX_K; ++i) d.hoist_at[i] = xs.hoist_at[i];
     d.tail_par = 0;
     for (uint32_t i = b.num_enum; i < b.k; ++i) d.tail_par |= b.parents[i];
-    // (labeled plans check every candidate's label where it is taken, so
-    // they keep the level-by-level DFS: no pair step)
-    d.pair = xs.pair && !b.labeled ? 1u : 0u;
-    d.pair_direct = xs.pair_direct && !b.labeled ? 1u : 0u;
+    d.pair = xs.pair ? 1u : 0u;
+    d.pair_direct = xs.pair_direct ? 1u : 0u;
     // exploration: the running list of a tail level whose parents below the
     // leaf are exactly levels 0 and 1 is final once the root is matched;
     // it is pinned in the third table
