@@ -24,9 +24,14 @@ struct DeviceGuard {
     DeviceGuard &operator=(const DeviceGuard &) = delete;
 };
 
-// Exclusive prefix sum of n uint32 values in device memory (out may alias
-// nothing in `in`), ordered on stream s; temporary space is allocated here.
+// Exclusive prefix sum of n uint32 values in device memory (out may be
+// `in` itself), ordered on stream s; temporary space is allocated here.
 sge_status device_exclusive_scan(const uint32_t *in, uint32_t *out, uint64_t n, cudaStream_t s);
+
+// Sorts n 64-bit keys of `bits` bits in device memory on stream s (tmp: as
+// many); the result is in `keys`, which may have changed places with tmp.
+sge_status device_sort_keys(unsigned long long *&keys, unsigned long long *&tmp, uint64_t n, uint32_t bits,
+                            cudaStream_t s);
 
 // Wraps a CSR already in device memory on `device` (d_off: n+1 offsets,
 // d_adj: nnz neighbours; symmetric, lists strictly increasing, no

@@ -5,7 +5,7 @@
 // (relation/graph.cpp:143-173) inserts both directions of every edge and
 // sorts each list; loadDataGraph (graph.cpp:255-419) reads text or BINGRPH.
 // Here an edge list already in device memory becomes a CSR with one sort of
-// (src, dst) rows, a duplicate/self-loop filter, an ordered compaction and
+// (src, dst) keys, a duplicate/self-loop filter that compacts in order and
 // one binary search per vertex for the offsets.  The R-MAT generator draws
 // the same counter-based splitmix64 stream as the host generator
 // (sge_gen_rmat), so a seed gives the same graph on either side.
@@ -40,39 +40,67 @@ __device__ __forceinline__ uint64_t splitmix64_d(uint64_t x) {
     return x ^ (x >> 31);
 }
 
-// Both directions of every edge as (src, dst) rows; self-loops become
-// (NONE, NONE) rows, which sort last and are dropped.  An id >= n sets *bad.
-__global__ void directed_rows(const uint32_t *edges, unsigned long long m, uint32_t n, uint32_t *rows,
-                              uint32_t *bad) {
+// Both directions of every edge as keys src << bits | dst; a self-loop becomes
+// two all-ones keys, which no edge has (src = dst), sort last and are dropped.
+// An id >= n sets *bad.
+__global__ void directed_keys(const uint2 *edges, unsigned long long m, uint32_t n, uint32_t bits,
+                              ulonglong2 *keys, uint32_t *bad) {
     const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    const uint32_t u = edges[2 * i], v = edges[2 * i + 1];
-    uint32_t *r = rows + 4 * i;
+    const uint32_t u = edges[i].x, v = edges[i].y;
+    const unsigned long long none = bits == 32 ? ~0ull : (1ull << (2 * bits)) - 1;
     if (u >= n || v >= n) atomicOr(bad, 1u);
-    if (u == v || u >= n || v >= n) {
-        r[0] = r[1] = r[2] = r[3] = NONE;
-        return;
+    if (u == v || u >= n || v >= n) keys[i] = make_ulonglong2(none, none);
+    else keys[i] = make_ulonglong2((unsigned long long)u << bits | v, (unsigned long long)v << bits | u);
+}
+
+// Sorted keys -> (src, adj): the first of every run of equal edge keys, in
+// order.  A warp takes 512 consecutive keys; the first kernel counts the kept
+// ones per 4096-key tile, the second writes them behind the tiles before it.
+constexpr int DEDUP_TILE = 4096;
+__device__ __forceinline__ bool first_of_run(const unsigned long long *keys, unsigned long long i,
+                                             unsigned long long n, unsigned long long none) {
+    return i < n && keys[i] != none && (i == 0 || keys[i] != keys[i - 1]);
+}
+__global__ void __launch_bounds__(256) dedup_count(const unsigned long long *keys, unsigned long long n,
+                                                   unsigned long long none, uint32_t *tiles) {
+    __shared__ uint32_t sum;
+    if (threadIdx.x == 0) sum = 0;
+    __syncthreads();
+    const unsigned long long base = blockIdx.x * (unsigned long long)DEDUP_TILE;
+    uint32_t c = 0;
+    for (int r = 0; r < DEDUP_TILE / 256; ++r) c += first_of_run(keys, base + r * 256 + threadIdx.x, n, none);
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if ((threadIdx.x & 31u) == 0) atomicAdd(&sum, c);
+    __syncthreads();
+    if (threadIdx.x == 0) tiles[blockIdx.x] = sum;
+}
+__global__ void __launch_bounds__(256) dedup_write(const unsigned long long *keys, unsigned long long n,
+                                                   unsigned long long none, uint32_t bits, const uint32_t *tile_at,
+                                                   uint32_t *src, uint32_t *adj) {
+    __shared__ uint32_t wsum[8];
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const unsigned long long base = blockIdx.x * (unsigned long long)DEDUP_TILE + w * (DEDUP_TILE / 8);
+    uint32_t mask[DEDUP_TILE / 256], c = 0;   // a round's kept lanes
+#pragma unroll
+    for (int r = 0; r < DEDUP_TILE / 256; ++r) {
+        mask[r] = __ballot_sync(0xFFFFFFFFu, first_of_run(keys, base + r * 32 + lane, n, none));
+        c += __popc(mask[r]);
     }
-    r[0] = u;
-    r[1] = v;
-    r[2] = v;
-    r[3] = u;
-}
-
-// keep[i] = row i is a real edge and differs from row i-1 (rows sorted)
-__global__ void first_of_run(const uint32_t *rows, unsigned long long n, uint32_t *keep) {
-    const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t a = rows[2 * i], b = rows[2 * i + 1];
-    keep[i] = (a != NONE) && (i == 0 || a != rows[2 * i - 2] || b != rows[2 * i - 1]) ? 1u : 0u;
-}
-
-__global__ void compact_rows(const uint32_t *rows, unsigned long long n, const uint32_t *keep, const uint32_t *pos,
-                             uint32_t *src, uint32_t *adj) {
-    const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !keep[i]) return;
-    src[pos[i]] = rows[2 * i];
-    adj[pos[i]] = rows[2 * i + 1];
+    if (lane == 0) wsum[w] = c;
+    __syncthreads();
+    uint32_t at = tile_at[blockIdx.x];
+    for (uint32_t q = 0; q < w; ++q) at += wsum[q];
+#pragma unroll
+    for (int r = 0; r < DEDUP_TILE / 256; ++r) {
+        if ((mask[r] >> lane) & 1u) {
+            const unsigned long long k = keys[base + r * 32 + lane];
+            const uint32_t o = at + __popc(mask[r] & ((1u << lane) - 1u));
+            src[o] = (uint32_t)(k >> bits);
+            adj[o] = (uint32_t)(k & ((1ull << bits) - 1));
+        }
+        at += __popc(mask[r]);
+    }
 }
 
 // off[v] = first position whose source is >= v (std::lower_bound)
@@ -168,30 +196,39 @@ sge_status sge_graph_create_from_device_edges(const uint32_t *d_edges, uint64_t 
     DeviceGuard restore_device;
     CUDA_TRY(cudaSetDevice(device));
     const unsigned long long nd = 2 * m;  // directed rows
-    DevBuf rows, keep, pos, src, bad;
+    DevBuf keys, tmp, tiles, src, bad;
     uint32_t *d_off = nullptr, *d_adj = nullptr;
     CUDA_TRY(cudaMalloc(&bad.p, 4));
     CUDA_TRY(cudaMemset(bad.p, 0, 4));
     uint64_t nnz = 0;
+    uint32_t bits = 1;
+    while (bits < 32 && ((uint64_t)num_vertices - 1) >> bits) ++bits;
+    const unsigned long long none = bits == 32 ? ~0ull : (1ull << (2 * bits)) - 1;
+    const unsigned ntiles = (unsigned)((nd + DEDUP_TILE - 1) / DEDUP_TILE);
     if (m) {
-        CUDA_TRY(cudaMalloc(&rows.p, 8 * nd));
-        directed_rows<<<grid_for(m), 256>>>(d_edges, m, num_vertices, rows.as<uint32_t>(), bad.as<uint32_t>());
+        CUDA_TRY(cudaMalloc(&keys.p, 8 * nd));
+        directed_keys<<<grid_for(m), 256>>>(reinterpret_cast<const uint2 *>(d_edges), m, num_vertices, bits,
+                                            keys.as<ulonglong2>(), bad.as<uint32_t>());
         CUDA_TRY(cudaGetLastError());
         uint32_t hbad = 0;
         CUDA_TRY(cudaMemcpy(&hbad, bad.p, 4, cudaMemcpyDeviceToHost));
         if (hbad) return fail(SGE_BAD_INPUT, "edge list has a vertex id >= num_vertices (%u)", num_vertices);
-        sge_status st = sge_sort_tuples(rows.as<uint32_t>(), nd, 2);
+        CUDA_TRY(cudaMalloc(&tmp.p, 8 * nd));
+        unsigned long long *a = keys.as<unsigned long long>(), *b = tmp.as<unsigned long long>();
+        sge_status st = device_sort_keys(a, b, nd, 2 * bits, 0);
+        keys.p = a;
+        tmp.p = b;
         if (st != SGE_OK) return st;
-        CUDA_TRY(cudaMalloc(&keep.p, 4 * nd));
-        CUDA_TRY(cudaMalloc(&pos.p, 4 * nd));
-        first_of_run<<<grid_for(nd), 256>>>(rows.as<uint32_t>(), nd, keep.as<uint32_t>());
+        // tile counts (and one more, for the total), then their prefix over themselves
+        CUDA_TRY(cudaMalloc(&tiles.p, 4 * ((size_t)ntiles + 1)));
+        CUDA_TRY(cudaMemset(tiles.as<uint32_t>() + ntiles, 0, 4));
+        dedup_count<<<ntiles, 256>>>(a, nd, none, tiles.as<uint32_t>());
         CUDA_TRY(cudaGetLastError());
-        st = device_exclusive_scan(keep.as<uint32_t>(), pos.as<uint32_t>(), nd, 0);
+        st = device_exclusive_scan(tiles.as<uint32_t>(), tiles.as<uint32_t>(), (uint64_t)ntiles + 1, 0);
         if (st != SGE_OK) return st;
-        uint32_t last_pos = 0, last_keep = 0;
-        CUDA_TRY(cudaMemcpy(&last_pos, pos.as<uint32_t>() + nd - 1, 4, cudaMemcpyDeviceToHost));
-        CUDA_TRY(cudaMemcpy(&last_keep, keep.as<uint32_t>() + nd - 1, 4, cudaMemcpyDeviceToHost));
-        nnz = (uint64_t)last_pos + last_keep;
+        uint32_t kept = 0;
+        CUDA_TRY(cudaMemcpy(&kept, tiles.as<uint32_t>() + ntiles, 4, cudaMemcpyDeviceToHost));
+        nnz = kept;
     }
     CUDA_TRY(cudaMalloc(&src.p, 4 * std::max<uint64_t>(nnz, 1)));
     cudaError_t e;
@@ -201,8 +238,8 @@ sge_status sge_graph_create_from_device_edges(const uint32_t *d_edges, uint64_t 
         return fail(SGE_OOM, "device CSR allocation: %s", cudaGetErrorString(e));
     }
     if (nnz)
-        compact_rows<<<grid_for(nd), 256>>>(rows.as<uint32_t>(), nd, keep.as<uint32_t>(), pos.as<uint32_t>(),
-                                             src.as<uint32_t>(), d_adj);
+        dedup_write<<<ntiles, 256>>>(keys.as<unsigned long long>(), nd, none, bits, tiles.as<uint32_t>(),
+                                     src.as<uint32_t>(), d_adj);
     offsets_from_sources<<<grid_for((unsigned long long)num_vertices + 1), 256>>>(src.as<uint32_t>(), nnz,
                                                                                  num_vertices, d_off);
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) {
