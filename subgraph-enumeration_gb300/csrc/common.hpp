@@ -23,6 +23,10 @@ sge_status fail(sge_status st, const char *fmt, ...);
 // bag, and that the bags cover every vertex.
 sge_status parse_bag_text(uint32_t k, const char *text, std::vector<std::vector<uint32_t>> &bags);
 
+// Degree moments and extremes of a graph (everything of sge_graph_stats but
+// the clustering coefficient).
+void degree_stats(const uint32_t *off, uint32_t n, sge_graph_stats *out);
+
 // splitmix64: the deterministic counter-based generator behind every seeded
 // generator and sampler in the library (same stream on every host).
 static inline uint64_t splitmix64(uint64_t x) {

@@ -36,10 +36,11 @@ sge_status device_sort_keys(unsigned long long *&keys, unsigned long long *&tmp,
 // Wraps a CSR already in device memory on `device` (d_off: n+1 offsets,
 // d_adj: nnz neighbours; symmetric, lists strictly increasing, no
 // self-loops) as a graph, which takes ownership of both arrays (also on
-// failure).  The root-edge list is built on the device; the planner's
-// statistics are computed on the host, from h_off/h_adj when the caller has
-// the CSR in host memory, else from a copy.
+// failure).  The root-edge list and the wedge sample are built on the device;
+// the degree statistics on the host, from h_off when the caller has the CSR in
+// host memory, else from a copy of the offsets.  planner_stats = false leaves
+// out what only the planner reads.
 sge_status graph_adopt(uint32_t *d_off, uint32_t *d_adj, uint32_t n, uint64_t nnz, int device, sge_graph **out,
-                       const uint32_t *h_off = nullptr, const uint32_t *h_adj = nullptr);
+                       const uint32_t *h_off = nullptr, const uint32_t *h_adj = nullptr, bool planner_stats = true);
 
 }  // namespace sge

@@ -2105,6 +2105,10 @@ __global__ void hub_bits_kernel(const uint32_t *off, const uint32_t *adj, const 
     }
 }
 
+__global__ void hub_flags_kernel(const uint32_t *off, uint32_t n, uint32_t thr, uint32_t *flag);
+__global__ void hub_slots_kernel(const uint32_t *off, uint32_t n, uint32_t thr, const uint32_t *at, int32_t *slot,
+                                 uint32_t *hubs);
+
 sge_status build_hub_index(sge_graph *g, const uint32_t *off) {
     const uint32_t n = g->n;
     if (n == 0 || g->max_deg < 16) return SGE_OK;
@@ -2124,15 +2128,11 @@ sge_status build_hub_index(sge_graph *g, const uint32_t *off) {
         thr = d;
     }
     if (above == 0) return SGE_OK;
-    std::vector<int32_t> slot(n, -1);
-    std::vector<uint32_t> hubs;
-    hubs.reserve(above);
-    for (uint32_t v = 0; v < n; ++v)
-        if (off[v + 1] - off[v] >= thr) { slot[v] = (int32_t)hubs.size(); hubs.push_back(v); }
-    uint32_t *d_hubs = nullptr;
+    const uint32_t nh = (uint32_t)above;
+    uint32_t *d_hubs = nullptr;   // hubs[nh] | flags, then their prefix [n]
     if (cudaMalloc(&g->d_hub_slot, 4ull * n) != cudaSuccess ||
-        cudaMalloc(&g->d_hub_bits, 4ull * words * hubs.size()) != cudaSuccess ||
-        cudaMalloc(&d_hubs, 4ull * hubs.size()) != cudaSuccess) {
+        cudaMalloc(&g->d_hub_bits, 4ull * words * nh) != cudaSuccess ||
+        cudaMalloc(&d_hubs, 4ull * (nh + (uint64_t)n)) != cudaSuccess) {
         cudaFree(g->d_hub_slot);
         cudaFree(g->d_hub_bits);
         g->d_hub_slot = nullptr;
@@ -2140,18 +2140,24 @@ sge_status build_hub_index(sge_graph *g, const uint32_t *off) {
         cudaGetLastError();
         return SGE_OK;  // no index: every probe is a binary search
     }
-    CUDA_TRY(cudaMemcpyAsync(g->d_hub_slot, slot.data(), 4ull * n, cudaMemcpyHostToDevice, g->stream));
-    CUDA_TRY(cudaMemcpyAsync(d_hubs, hubs.data(), 4ull * hubs.size(), cudaMemcpyHostToDevice, g->stream));
-    CUDA_TRY(cudaMemsetAsync(g->d_hub_bits, 0, 4ull * words * hubs.size(), g->stream));
-    hub_bits_kernel<<<(unsigned)std::min<size_t>(hubs.size(), 65535), 256, 0, g->stream>>>(
-        g->d_off, g->d_adj, d_hubs, (uint32_t)hubs.size(), (uint32_t)words, g->d_hub_bits);
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaStreamSynchronize(g->stream));
+    const unsigned grid = (unsigned)(((uint64_t)n + 255) / 256);
+    cudaError_t e = cudaMemsetAsync(g->d_hub_bits, 0, 4ull * words * nh, g->stream);
+    hub_flags_kernel<<<grid, 256, 0, g->stream>>>(g->d_off, n, thr, d_hubs + nh);
+    const sge_status st = device_exclusive_scan(d_hubs + nh, d_hubs + nh, n, g->stream);
+    if (st == SGE_OK) {
+        hub_slots_kernel<<<grid, 256, 0, g->stream>>>(g->d_off, n, thr, d_hubs + nh, g->d_hub_slot, d_hubs);
+        hub_bits_kernel<<<std::min(nh, 65535u), 256, 0, g->stream>>>(g->d_off, g->d_adj, d_hubs, nh, (uint32_t)words,
+                                                                    g->d_hub_bits);
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    }
     cudaFree(d_hubs);
+    if (st != SGE_OK) return st;
+    if (e != cudaSuccess) return fail(SGE_CUDA_ERROR, "hub index: %s", cudaGetErrorString(e));
     g->hub_words = (uint32_t)words;
     g->hub_min = thr;
-    g->hub_count = (uint32_t)hubs.size();
-    g->hub_bytes = 4ull * words * hubs.size() + 4ull * n;
+    g->hub_count = nh;
+    g->hub_bytes = 4ull * words * nh + 4ull * n;
     return SGE_OK;
 }
 
@@ -2671,8 +2677,9 @@ int sge_device_count(void) {
     return n;
 }
 
-sge_status sge_graph_create(const uint32_t *offsets, const uint32_t *nbrs, uint32_t n, uint64_t nnz, int device,
-                            sge_graph **out) {
+// planner_stats: false for a graph that no plan will be made on.
+static sge_status graph_create(const uint32_t *offsets, const uint32_t *nbrs, uint32_t n, uint64_t nnz, int device,
+                               bool planner_stats, sge_graph **out) {
     using sge_csr_check::validate_csr_device;
     if (!offsets || (!nbrs && nnz) || !out) return fail(SGE_BAD_INPUT, "sge_graph_create: null argument");
     if (nnz % 2) return fail(SGE_BAD_INPUT, "odd number of directed edges (%llu)", (unsigned long long)nnz);
@@ -2710,7 +2717,12 @@ sge_status sge_graph_create(const uint32_t *offsets, const uint32_t *nbrs, uint3
             return st;
         }
     }
-    return graph_adopt(d_off, d_adj, n, nnz, device, out, offsets, nbrs);
+    return graph_adopt(d_off, d_adj, n, nnz, device, out, offsets, nbrs, planner_stats);
+}
+
+sge_status sge_graph_create(const uint32_t *offsets, const uint32_t *nbrs, uint32_t n, uint64_t nnz, int device,
+                            sge_graph **out) {
+    return graph_create(offsets, nbrs, n, nnz, device, true, out);
 }
 
 }  // extern "C"
@@ -2752,44 +2764,191 @@ __global__ void csr_check_kernel(const uint32_t *off, const uint32_t *adj, uint3
     }
 }
 
-// Root edges of a device CSR: directed edge e = (src(e), adj[e]) is a root
-// when adj[e] > src(e); pos[e] is its rank among the roots (CSR order).
-__global__ void root_flags_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, unsigned long long nnz,
-                                  uint32_t *flags) {
-    const unsigned long long e = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const uint32_t src = ub(off, n + 1, (uint32_t)e) - 1;
-    flags[e] = adj[e] > src ? 1u : 0u;
-}
-// Sums over the vertices of (neighbours above it)^2 and (below it)^2: the
-// lengths of the lists that lower and upper bounds leave, weighted by use.
-__global__ void side_sums_kernel(const uint32_t *off, const uint32_t *pos, uint32_t n, unsigned long long nnz,
-                                 unsigned long long m, unsigned long long *sums) {
-    unsigned long long up = 0, down = 0;
+constexpr uint32_t EDGE_TILE = 1024;   // entries per block
+// Neighbours above each vertex (a list is sorted: its upper part), and the
+// sums over the vertices of their squares and of those below: the lengths of
+// the lists that lower and upper bounds leave, weighted by use.
+__global__ void upper_parts_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, uint32_t *up,
+                                   unsigned long long *sums) {
+    unsigned long long su = 0, sd = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t a = off[v], b = off[v + 1];
-        const unsigned long long u = (b < nnz ? pos[b] : m) - (a < nnz ? pos[a] : m), d = b - a - u;
-        up += u * u;
-        down += d * d;
+        const uint32_t a = off[v], d = off[v + 1] - a;
+        const unsigned long long below = lb(adj + a, d, v), above = d - below;
+        up[v] = (uint32_t)above;
+        su += above * above;
+        sd += below * below;
     }
-    up = warp_sum_u64(up);
-    down = warp_sum_u64(down);
+    __syncwarp();
+    su = warp_sum_u64(su);
+    sd = warp_sum_u64(sd);
     if ((threadIdx.x & 31u) == 0) {
-        atomicAdd(sums, up);
-        atomicAdd(sums + 1, down);
+        atomicAdd(sums, su);
+        atomicAdd(sums + 1, sd);
     }
 }
-__global__ void root_scatter_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, unsigned long long nnz,
-                                    const uint32_t *flags, const uint32_t *pos, uint2 *edges) {
-    const unsigned long long e = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz || !flags[e]) return;
-    const uint32_t src = ub(off, n + 1, (uint32_t)e) - 1;
-    edges[pos[e]] = make_uint2(src, adj[e]);
+// Root edges of a device CSR: directed edge e = (src, adj[e]) is a root when
+// adj[e] > src.  The upper part of a list is its end, so the rank of e among
+// the roots (CSR order) is base[src] + e - (end of the list - up[src]), with
+// base the exclusive prefix of up: one pass over the edges, and the source is
+// searched among the few vertices of the block's 1,024 edges.  (Flagging,
+// scanning and scattering all 32M directed edges of R-MAT 2^20 took 0.98 ms,
+// this 0.25 ms.)
+__global__ void __launch_bounds__(256) root_edges_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n,
+                                                         unsigned long long nnz, const uint32_t *up,
+                                                         const uint32_t *base, uint2 *edges) {
+    __shared__ uint32_t span[2];
+    const unsigned long long e0 = blockIdx.x * (unsigned long long)EDGE_TILE;
+    if (threadIdx.x < 2) {
+        const unsigned long long e = threadIdx.x ? min(e0 + EDGE_TILE, nnz) - 1 : e0;
+        span[threadIdx.x] = ub(off, n + 1, (uint32_t)e) - 1;
+    }
+    __syncthreads();
+    const uint32_t s0 = span[0], len = span[1] - s0 + 1;
+#pragma unroll
+    for (uint32_t r = 0; r < EDGE_TILE / 256; ++r) {
+        const unsigned long long e = e0 + r * 256 + threadIdx.x;
+        if (e >= nnz) break;
+        const uint32_t src = s0 + ub(off + s0, len, (uint32_t)e) - 1, y = adj[e];
+        if (y > src) edges[base[src] + ((uint32_t)e - (off[src + 1] - up[src]))] = make_uint2(src, y);
+    }
+}
+// slot[v] = rank of v among the vertices of degree >= thr (-1 for the others);
+// hubs = those vertices in id order.
+__global__ void hub_flags_kernel(const uint32_t *off, uint32_t n, uint32_t thr, uint32_t *flag) {
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < n) flag[v] = off[v + 1] - off[v] >= thr ? 1u : 0u;
+}
+__global__ void hub_slots_kernel(const uint32_t *off, uint32_t n, uint32_t thr, const uint32_t *at, int32_t *slot,
+                                 uint32_t *hubs) {
+    const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const bool hub = off[v + 1] - off[v] >= thr;
+    slot[v] = hub ? (int32_t)at[v] : -1;
+    if (hub) hubs[at[v]] = v;
+}
+
+// Exclusive prefix cum[0..n] of the vertices' wedges d(d-1)/2: tiles of 1,024
+// vertices, one block over the tiles, the tiles again.
+__device__ __forceinline__ unsigned long long wedges(const uint32_t *off, uint32_t n, unsigned long long v) {
+    if (v >= n) return 0;
+    const unsigned long long d = off[v + 1] - off[v];
+    return d ? d * (d - 1) / 2 : 0ull;
+}
+__device__ __forceinline__ unsigned long long block_prefix_u64(unsigned long long v, unsigned long long *ws,
+                                                               unsigned long long &total) {
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    unsigned long long incl = v;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(FULL_MASK, incl, o);
+        if (lane >= o) incl += t;
+    }
+    __syncthreads();
+    if (lane == 31) ws[w] = incl;
+    __syncthreads();
+    unsigned long long before = 0;
+    total = 0;
+    for (uint32_t q = 0; q < (blockDim.x >> 5); ++q) {
+        if (q < w) before += ws[q];
+        total += ws[q];
+    }
+    return before + incl - v;
+}
+__global__ void __launch_bounds__(1024) wedge_tiles_kernel(const uint32_t *off, uint32_t n, unsigned long long *tiles) {
+    __shared__ unsigned long long ws[32];
+    unsigned long long total;
+    block_prefix_u64(wedges(off, n, blockIdx.x * 1024ull + threadIdx.x), ws, total);
+    if (threadIdx.x == 0) tiles[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(1024) wedge_scan_kernel(unsigned long long *tiles, uint32_t nt) {
+    __shared__ unsigned long long ws[32];
+    unsigned long long run = 0;
+    for (uint32_t b = 0; b < nt; b += 1024) {
+        const uint32_t i = b + threadIdx.x;
+        unsigned long long total;
+        const unsigned long long at = block_prefix_u64(i < nt ? tiles[i] : 0ull, ws, total);
+        if (i < nt) tiles[i] = run + at;
+        run += total;
+    }
+}
+__global__ void __launch_bounds__(1024) wedge_cum_kernel(const uint32_t *off, uint32_t n,
+                                                         const unsigned long long *tiles, unsigned long long *cum) {
+    __shared__ unsigned long long ws[32];
+    unsigned long long total;
+    const unsigned long long v = blockIdx.x * 1024ull + threadIdx.x, w = wedges(off, n, v);
+    const unsigned long long at = tiles[blockIdx.x] + block_prefix_u64(w, ws, total);
+    if (v < n) cum[v] = at;
+    if (v + 1 == n) cum[n] = at + w;
+}
+// sample_clustering's samples, one per thread: sample s takes draws 3s, 3s+1
+// and 3s+2 of the generator (splitmix64's n-th draw is a mix of its start + n
+// steps), which is the host loop's order as long as no sample is drawn again.
+// res[0] = closed wedges, res[1] = samples the host loop would draw again.
+__global__ void clustering_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, const unsigned long long *cum,
+                                  unsigned long long state, uint32_t samples, uint32_t *res) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= samples) return;
+    auto draw = [&](uint32_t i) {
+        unsigned long long z = state + (3ull * s + i + 1ull) * 0x9E3779B97F4A7C15ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        return z ^ (z >> 31);
+    };
+    const double total = (double)cum[n];
+    const double r = __dmul_rn(__dmul_rn((double)(draw(0) >> 11), 1.0 / 9007199254740992.0), total);
+    uint32_t lo = 0, len = n + 1;   // first index with cum > r
+    while (len > 0) {
+        const uint32_t half = len >> 1;
+        if ((double)cum[lo + half] <= r) { lo += half + 1; len -= half + 1; }
+        else len = half;
+    }
+    const uint32_t v = lo - 1;
+    const uint32_t d = v < n ? off[v + 1] - off[v] : 0u;
+    if (d < 2) { atomicAdd(res + 1, 1u); return; }
+    const uint32_t a = (uint32_t)__umul64hi(draw(1), d);
+    uint32_t b = (uint32_t)__umul64hi(draw(2), d - 1);
+    if (b >= a) ++b;
+    const uint32_t x = adj[off[v] + a], y = adj[off[v] + b];
+    if (contains(adj + off[x], off[x + 1] - off[x], y)) atomicAdd(res, 1u);
+}
+}  // namespace
+
+namespace {
+// The sampled clustering coefficient on the device: the host function's draws
+// and its result.  *done = false where they could differ (a sample that the
+// host would draw again, or wedge sums that doubles do not hold exactly).
+sge_status clustering_device(const sge_graph *g, double *out, bool *done) {
+    constexpr uint32_t SAMPLES = 1u << 16;
+    *done = false;
+    *out = 0.0;
+    const uint32_t nt = (uint32_t)(((uint64_t)g->n + 1023) / 1024);
+    unsigned char *buf = nullptr;
+    const size_t cum_bytes = 8 * ((size_t)g->n + 1), bytes = cum_bytes + 8 * (size_t)nt + 16;
+    if (cudaMalloc(&buf, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return SGE_OK;
+    }
+    unsigned long long *cum = reinterpret_cast<unsigned long long *>(buf), *tiles = cum + g->n + 1, total = 0;
+    uint32_t *res = reinterpret_cast<uint32_t *>(tiles + nt), h[2] = {0, 0};
+    cudaMemsetAsync(res, 0, 8, g->stream);
+    wedge_tiles_kernel<<<nt, 1024, 0, g->stream>>>(g->d_off, g->n, tiles);
+    wedge_scan_kernel<<<1, 1024, 0, g->stream>>>(tiles, nt);
+    wedge_cum_kernel<<<nt, 1024, 0, g->stream>>>(g->d_off, g->n, tiles, cum);
+    clustering_kernel<<<SAMPLES / 256, 256, 0, g->stream>>>(g->d_off, g->d_adj, g->n, cum, Rng(0xC1A5u).s, SAMPLES, res);
+    cudaMemcpyAsync(h, res, 8, cudaMemcpyDeviceToHost, g->stream);
+    cudaMemcpyAsync(&total, cum + g->n, 8, cudaMemcpyDeviceToHost, g->stream);
+    const cudaError_t e = cudaStreamSynchronize(g->stream);
+    cudaFree(buf);
+    if (e != cudaSuccess) return fail(SGE_CUDA_ERROR, "clustering sample: %s", cudaGetErrorString(e));
+    if (total >= (1ull << 53) || (total && h[1])) return SGE_OK;
+    *out = total ? (double)h[0] / SAMPLES : 0.0;
+    *done = true;
+    return SGE_OK;
 }
 }  // namespace
 
 sge_status sge::graph_adopt(uint32_t *d_off, uint32_t *d_adj, uint32_t n, uint64_t nnz, int device,
-                            sge_graph **out, const uint32_t *h_off, const uint32_t *h_adj) {
+                            sge_graph **out, const uint32_t *h_off, const uint32_t *h_adj, bool planner_stats) {
     sge_graph *g = new sge_graph();
     g->device = device;
     g->d_off = d_off;
@@ -2807,46 +2966,67 @@ sge_status sge::graph_adopt(uint32_t *d_off, uint32_t *d_adj, uint32_t n, uint64
     if ((e = cudaMalloc(&g->d_edges, sizeof(uint2) * std::max<uint64_t>(g->m, 1))) != cudaSuccess)
         return cleanup(fail(SGE_OOM, "device allocation of the root edges failed: %s", cudaGetErrorString(e)));
     if (nnz) {
-        uint32_t *flags = nullptr, *pos = nullptr;
-        if ((e = cudaMalloc(&flags, 4 * nnz)) != cudaSuccess || (e = cudaMalloc(&pos, 4 * nnz)) != cudaSuccess) {
-            cudaFree(flags);
+        uint32_t *up = nullptr;   // up[n] | its prefix[n] | two sums
+        const size_t words = ((size_t)2 * n + 1) & ~(size_t)1;
+        if ((e = cudaMalloc(&up, 4 * words + 16)) != cudaSuccess)
             return cleanup(fail(SGE_OOM, "root edge scratch: %s", cudaGetErrorString(e)));
-        }
-        const unsigned grid = (unsigned)((nnz + 255) / 256);
-        root_flags_kernel<<<grid, 256, 0, g->stream>>>(d_off, d_adj, n, nnz, flags);
-        sge_status st = device_exclusive_scan(flags, pos, nnz, g->stream);
+        unsigned long long *d_sums = reinterpret_cast<unsigned long long *>(up + words), sums[2] = {0, 0};
+        cudaMemsetAsync(d_sums, 0, 16, g->stream);
+        upper_parts_kernel<<<std::min<unsigned>((n + 255) / 256, 8u * g->num_sms), 256, 0, g->stream>>>(d_off, d_adj, n,
+                                                                                                    up, d_sums);
+        sge_status st = device_exclusive_scan(up, up + n, n, g->stream);
         if (st == SGE_OK) {
-            root_scatter_kernel<<<grid, 256, 0, g->stream>>>(d_off, d_adj, n, nnz, flags, pos, g->d_edges);
-            // (flags is free once the scatter has read it: the two sums go there)
-            unsigned long long *d_sums = reinterpret_cast<unsigned long long *>(flags), sums[2] = {0, 0};
-            if (nnz >= 4) {
-                cudaMemsetAsync(d_sums, 0, 16, g->stream);
-                side_sums_kernel<<<std::min<unsigned>((n + 255) / 256, 8u * g->num_sms), 256, 0, g->stream>>>(
-                    d_off, pos, n, nnz, g->m, d_sums);
-                cudaMemcpyAsync(sums, d_sums, 16, cudaMemcpyDeviceToHost, g->stream);
-            }
+            root_edges_kernel<<<(unsigned)((nnz + EDGE_TILE - 1) / EDGE_TILE), 256, 0, g->stream>>>(
+                d_off, d_adj, n, nnz, up, up + n, g->d_edges);
+            cudaMemcpyAsync(sums, d_sums, 16, cudaMemcpyDeviceToHost, g->stream);
             e = cudaStreamSynchronize(g->stream);
             g->mirror = (double)sums[0] > 1.1 * (double)sums[1];
             if (e != cudaSuccess) st = fail(SGE_CUDA_ERROR, "root edges: %s", cudaGetErrorString(e));
         }
-        cudaFree(flags);
-        cudaFree(pos);
+        cudaFree(up);
         if (st != SGE_OK) return cleanup(st);
     }
-    // planner statistics from the host arrays (a copy of the device CSR when
-    // it was built on the device: the same numbers as a host-built graph)
+    // degrees on the host (the offsets alone are copied when the CSR was
+    // built on the device): histogram, planner statistics
     std::vector<uint32_t> off, adj;
     if (!h_off) {
         off.resize((size_t)n + 1);
-        adj.resize(std::max<uint64_t>(nnz, 1));
-        if ((e = cudaMemcpy(off.data(), d_off, 4 * ((size_t)n + 1), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-            (nnz && (e = cudaMemcpy(adj.data(), d_adj, 4 * nnz, cudaMemcpyDeviceToHost)) != cudaSuccess))
+        if ((e = cudaMemcpy(off.data(), d_off, 4 * ((size_t)n + 1), cudaMemcpyDeviceToHost)) != cudaSuccess)
             return cleanup(fail(SGE_CUDA_ERROR, "graph read-back: %s", cudaGetErrorString(e)));
         h_off = off.data();
-        h_adj = adj.data();
     }
     for (uint32_t v = 0; v < n; ++v) g->max_deg = std::max(g->max_deg, h_off[v + 1] - h_off[v]);
-    sge_graph_stats_compute(h_off, h_adj, n, &g->stats);
+    if (planner_stats) {
+        // the wedge sample runs on the device; the host function is kept for
+        // the graphs where its draws would differ
+        bool done = n == 0;
+        double clustering = 0.0;
+        if (n) {
+            const sge_status st = clustering_device(g, &clustering, &done);
+            if (st != SGE_OK) return cleanup(st);
+        }
+        if (!done && !h_adj) {
+            adj.resize(std::max<uint64_t>(nnz, 1));
+            if (nnz && (e = cudaMemcpy(adj.data(), d_adj, 4 * nnz, cudaMemcpyDeviceToHost)) != cudaSuccess)
+                return cleanup(fail(SGE_CUDA_ERROR, "graph read-back: %s", cudaGetErrorString(e)));
+            h_adj = adj.data();
+        }
+        degree_stats(h_off, n, &g->stats);
+        g->stats.clustering = done ? clustering : sample_clustering(h_off, h_adj, n);
+    } else {
+        // what a counting launch reads: the first moments
+        g->stats.num_vertices = n;
+        g->stats.num_directed_edges = (double)nnz;
+        g->stats.max_degree = g->max_deg;
+        double m2 = 0;
+        for (uint32_t v = 0; v < n; ++v) {
+            const double d = h_off[v + 1] - h_off[v];
+            m2 += d * d;
+        }
+        g->stats.moments[0] = n;
+        g->stats.moments[1] = (double)nnz;
+        g->stats.moments[2] = m2;
+    }
     sge_status hst = build_hub_index(g, h_off);
     if (hst != SGE_OK) return cleanup(hst);
     *out = g;
@@ -3208,7 +3388,7 @@ sge_status sge_count_host(const uint32_t *offsets, const uint32_t *nbrs, uint32_
     for (uint32_t i = 0; i < nplans; ++i)
         if (blobs[i].labeled) return fail(SGE_UNSUPPORTED, "sge_count_host takes unlabeled plans");
     sge_graph *g = nullptr;
-    sge_status st = sge_graph_create(offsets, nbrs, n, nnz, 0, &g);
+    sge_status st = graph_create(offsets, nbrs, n, nnz, 0, false, &g);
     if (st != SGE_OK) return st;
     std::vector<sge_plan *> ps(nplans, nullptr);
     for (uint32_t i = 0; i < nplans && st == SGE_OK; ++i) st = sge_plan_create(&blobs[i], &ps[i]);

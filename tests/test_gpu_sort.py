@@ -65,3 +65,29 @@ def test_ingest_drops_repeats_and_self_loops(sge, n, m):
     with sge.Engine.from_device_edges(d.data_ptr(), m, n) as eng:
         off, nb = eng.csr()
     assert np.array_equal(off, want.offsets) and np.array_equal(nb, want.nbrs)
+
+
+@pytest.mark.parametrize("kind", ["rmat", "chung_lu", "star", "path", "isolated"])
+def test_graph_handle_facts_match_the_host(sge, kind):
+    """Root edges (through counts), planner statistics and hub index of a
+    device graph, against the host's own: degree moments and wedge sample give
+    the same plan costs bit for bit."""
+    g = {"rmat": lambda: sge.gen_rmat(12, 30_001, seed=2), "chung_lu": lambda: sge.gen_chung_lu(5000, 30_000, 2.1, 0, 4),
+         "star": lambda: sge.DataGraph.from_edges(np.array([(0, i) for i in range(1, 3000)]), 3000),
+         "path": lambda: sge.DataGraph.from_edges(np.array([(i, i + 1) for i in range(2047)]), 2048),
+         "isolated": lambda: sge.DataGraph.from_edges(np.array([(5, 900), (5, 1023), (900, 1023)]), 4100)}[kind]()
+    pats = [sge.PatternGraph.random(k, m, 40 + k) for k, m in ((3, 3), (4, 4), (5, 7), (6, 11), (7, 16))]
+    stats = g.stats()
+    with sge.Engine(g) as eng:
+        info = eng.info()
+        for p in pats:
+            a, b = sge.plan(p, eng), sge.plan(p, stats)
+            assert a.to_bytes() == b.to_bytes()
+        deg = np.diff(g.offsets)
+        if info["hub_count"]:
+            assert info["hub_count"] == int((deg >= info["hub_min_degree"]).sum())
+        hubs, _, _ = eng.count([sge.plan(pats[0], eng)])
+        lists, _, _ = eng.count([sge.plan(pats[0], eng)], hub_bitmaps=False)
+    assert hubs == lists
+    if kind == "isolated":
+        assert hubs == [6]
