@@ -2631,13 +2631,13 @@ sge_status finish_counts(const LaunchCfg &L, const unsigned long long *hc, uint3
 constexpr uint64_t SGE_HOST_VALIDATE_MAX = 1ull << 22;
 
 namespace {
-__global__ void csr_check_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, uint32_t *res,
-                                 unsigned long long *cnt);
+__global__ void csr_check_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, unsigned long long nnz,
+                                 uint32_t *res, unsigned long long *cnt);
 }  // namespace
 
 namespace sge_csr_check {
 // validate_csr's list checks for a CSR already on the device (same messages).
-sge_status validate_csr_device(const uint32_t *d_off, const uint32_t *d_adj, uint32_t n, int device) {
+sge_status validate_csr_device(const uint32_t *d_off, const uint32_t *d_adj, uint32_t n, uint64_t nnz) {
     uint32_t *res = nullptr;
     unsigned long long *cnt = nullptr;
     CUDA_TRY(cudaMalloc(&res, 16));
@@ -2646,12 +2646,10 @@ sge_status validate_csr_device(const uint32_t *d_off, const uint32_t *d_adj, uin
     const uint32_t init[4] = {0u, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u};
     uint32_t h[4] = {0, 0, 0, 0};
     unsigned long long hc[2] = {0, 0};
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     e = cudaMemcpy(res, init, 16, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(cnt, 0, 16);
     if (e == cudaSuccess) {
-        csr_check_kernel<<<(unsigned)std::max(sms, 1) * 8u, 256>>>(d_off, d_adj, n, res, cnt);
+        csr_check_kernel<<<(unsigned)((nnz + 1023) / 1024), 256>>>(d_off, d_adj, n, nnz, res, cnt);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(h, res, 16, cudaMemcpyDeviceToHost);
@@ -2710,7 +2708,7 @@ static sge_status graph_create(const uint32_t *offsets, const uint32_t *nbrs, ui
         return fail(SGE_CUDA_ERROR, "graph upload failed: %s", cudaGetErrorString(e));
     }
     if (on_device) {
-        st = validate_csr_device(d_off, d_adj, n, device);
+        st = validate_csr_device(d_off, d_adj, n, nnz);
         if (st != SGE_OK) {
             cudaFree(d_off);
             cudaFree(d_adj);
@@ -2728,43 +2726,52 @@ sge_status sge_graph_create(const uint32_t *offsets, const uint32_t *nbrs, uint3
 }  // extern "C"
 
 namespace {
-// The checks of validate_csr on the device, one warp per vertex: res[0] |= 2
-// (a list not strictly increasing, out of range or with a self-loop; res[1] =
-// the smallest such vertex) or 4 (an entry above the diagonal without its
-// reverse; res[2] = the smallest such vertex); cnt[0/1] = entries above/below
-// the diagonal.  Offsets were checked on the host, so every list is in bounds.
-__global__ void csr_check_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, uint32_t *res,
-                                 unsigned long long *cnt) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long up = 0, lo = 0;
-    for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
-        const uint32_t a = off[v], b = off[v + 1];
-        for (uint32_t e = a + lane; e < b; e += 32) {
-            const uint32_t w = adj[e];
-            if (w >= n || w == v || (e > a && adj[e - 1] >= w)) {
-                atomicOr(res, 2u);
-                atomicMin(res + 1, v);
-                continue;
-            }
-            if (w < v) { ++lo; continue; }
-            ++up;
-            const uint32_t wa = off[w];
-            if (!contains(adj + wa, off[w + 1] - wa, v)) {
-                atomicOr(res, 4u);
-                atomicMin(res + 2, v);
-            }
+// The checks of validate_csr on the device, one thread per entry (a list as
+// long as a hub's is not one warp's work: 12M entries of R-MAT 2^19, one warp
+// per vertex 4.0 ms, so 0.21 ms): res[0] |= 2 (a list not strictly
+// increasing, out of range or with a self-loop; res[1] = the smallest such
+// vertex) or 4 (an entry above the diagonal without its reverse; res[2] = the
+// smallest such vertex); cnt[0/1] = entries above/below the diagonal.
+// Offsets were checked on the host, so every list is in bounds.
+constexpr uint32_t EDGE_TILE = 1024;   // entries per block
+__global__ void __launch_bounds__(256) csr_check_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n,
+                                                        unsigned long long nnz, uint32_t *res,
+                                                        unsigned long long *cnt) {
+    __shared__ uint32_t span[2];
+    const unsigned long long e0 = blockIdx.x * (unsigned long long)EDGE_TILE;
+    if (threadIdx.x < 2) {
+        const unsigned long long e = threadIdx.x ? min(e0 + EDGE_TILE, nnz) - 1 : e0;
+        span[threadIdx.x] = ub(off, n + 1, (uint32_t)e) - 1;
+    }
+    __syncthreads();
+    const uint32_t s0 = span[0], len = span[1] - s0 + 1;
+    uint32_t up = 0, lo = 0;
+    for (uint32_t r = 0; r < EDGE_TILE / 256; ++r) {
+        const unsigned long long e = e0 + r * 256 + threadIdx.x;
+        if (e >= nnz) break;
+        const uint32_t v = s0 + ub(off + s0, len, (uint32_t)e) - 1, w = adj[e];
+        if (w >= n || w == v || (e > off[v] && adj[e - 1] >= w)) {
+            atomicOr(res, 2u);
+            atomicMin(res + 1, v);
+            continue;
+        }
+        if (w < v) { ++lo; continue; }
+        ++up;
+        const uint32_t wa = off[w];
+        if (!contains(adj + wa, off[w + 1] - wa, v)) {
+            atomicOr(res, 4u);
+            atomicMin(res + 2, v);
         }
     }
-    up = warp_sum_u64(up);
-    lo = warp_sum_u64(lo);
-    if (lane == 0) {
-        atomicAdd(cnt, up);
-        atomicAdd(cnt + 1, lo);
+    __syncwarp();
+    up = __reduce_add_sync(FULL_MASK, up);
+    lo = __reduce_add_sync(FULL_MASK, lo);
+    if ((threadIdx.x & 31u) == 0) {
+        if (up) atomicAdd(cnt, (unsigned long long)up);
+        if (lo) atomicAdd(cnt + 1, (unsigned long long)lo);
     }
 }
 
-constexpr uint32_t EDGE_TILE = 1024;   // entries per block
 // Neighbours above each vertex (a list is sorted: its upper part), and the
 // sums over the vertices of their squares and of those below: the lengths of
 // the lists that lower and upper bounds leave, weighted by use.
