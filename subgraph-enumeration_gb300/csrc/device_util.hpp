@@ -33,6 +33,11 @@ sge_status device_exclusive_scan(const uint32_t *in, uint32_t *out, uint64_t n, 
 sge_status device_sort_keys(unsigned long long *&keys, unsigned long long *&tmp, uint64_t n, uint32_t bits,
                             cudaStream_t s);
 
+// sge_enumerate; any_representative = true may write another member of each
+// automorphism class than the plan's restrictions keep.
+sge_status enumerate_rows(sge_graph *g, const sge_plan *p, uint32_t *d_out, uint64_t capacity, uint64_t *n_matches,
+                          bool any_representative);
+
 // Wraps a CSR already in device memory on `device` (d_off: n+1 offsets,
 // d_adj: nnz neighbours; symmetric, lists strictly increasing, no
 // self-loops) as a graph, which takes ownership of both arrays (also on

@@ -1839,13 +1839,200 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
 // Writes every match of a plan (all k levels enumerated, no counting tail)
 // as k vertex ids in pattern-vertex order: the tuples of nodeJoin /
 // globalJoin before buildTrie (matching/join.cpp:309-421,1202-1420) and, for
-// the whole pattern, the embedding set -r writes.  A warp owns one root edge;
-// the last level's candidates are emitted 32 at a time with one atomicAdd of
-// the output cursor per chunk.
+// the whole pattern, the embedding set -r writes.  A warp owns one root edge
+// (32 of them for three-vertex patterns); the last two levels are generated
+// 32 candidates x at a time by one scan flattened over (x, element), as the
+// counting pair step does, and the survivors leave 32 at a time.  (Entering the last level once per x kept
+// most lanes idle on short lists: the 3.4M K4 tuples of a 7,100-vertex
+// Chung-Lu graph took 1.6 ms, now 0.8 ms; a cursor update per 32 scanned elements,
+// however few are kept, was a third of that.)
+struct EnumOut {
+    uint32_t *rows;
+    unsigned long long cap;
+    unsigned long long *n;
+};
+// The kept (x, y) of a scan wait in S.qx / S.qy; whole groups of 32 leave with
+// one atomicAdd of the cursor (one per 32 scanned elements makes the cursor
+// the bound where few are kept), the rest with `last`.  write(row, x, y)
+// stores one row.
+template <class F>
+__device__ __forceinline__ void enum_put(PairState &S, const EnumOut &o, uint32_t &qn, bool keep, uint32_t x, uint32_t y,
+                                         bool last, F write) {
+    const uint32_t lane = lane_id(), kb = __ballot_sync(FULL_MASK, keep);
+    if (keep) {
+        const uint32_t p = qn + __popc(kb & ((1u << lane) - 1u));
+        S.qx[p] = x;
+        S.qy[p] = y;
+    }
+    qn += __popc(kb);
+    if (qn < 32 && !(last && qn)) return;
+    __syncwarp();
+    const uint32_t take = min(qn, 32u);
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(o.n, (unsigned long long)take);
+    base = __shfl_sync(FULL_MASK, base, 0);
+    if (lane < take && base + lane < o.cap) write(base + lane, S.qx[lane], S.qy[lane]);
+    const uint32_t rx = S.qx[32 + lane], ry = S.qy[32 + lane];
+    __syncwarp();
+    qn -= take;
+    if (lane < qn) { S.qx[lane] = rx; S.qy[lane] = ry; }
+    __syncwarp();
+}
+// Inclusive prefix of the lanes' lengths in S.pref, the scanned lists in S.bp.
+__device__ __forceinline__ uint32_t enum_flatten(PairState &S, const uint32_t *bp, uint32_t blen) {
+    const uint32_t lane = lane_id();
+    S.bp[lane] = bp;
+    uint32_t incl = blen;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL_MASK, incl, o);
+        if (lane >= o) incl += v;
+    }
+    S.pref[lane] = incl;
+    const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
+    __syncwarp();
+    return total;
+}
+
+// Levels a = k-2 and k-1 under the matched prefix.
+__device__ __forceinline__ void enum_pairs(const DevPlan &P, WarpState &W, Ctx<false> &c, uint32_t a, const EnumOut &out) {
+    PairState &S = *c.PS;
+    const uint32_t lane = lane_id(), i = a + 1, k = P.k, n = W.cnt[a];
+    const uint32_t *lst = W.list[a];
+    pair_sources(P, W, c, a);
+    const uint32_t ns = S.ns, xpar = S.xpar, nex = S.nex;
+    const bool ex_x = (P.check[i] >> a) & 1u;
+    uint32_t qn = 0;
+    auto write = [&](unsigned long long row, uint32_t x, uint32_t y) {
+        uint32_t *o = out.rows + row * k;
+        for (uint32_t lv = 0; lv < a; ++lv) o[P.order_[lv]] = W.m[lv];
+        o[P.order_[a]] = x;
+        o[P.order_[i]] = y;
+    };
+    for (uint32_t b0 = 0; b0 < n; b0 += 32) {
+        const uint32_t idx = b0 + lane;
+        const uint32_t x = idx < n ? lst[idx] : 0u;
+        const bool valid = idx < n && !excluded(P, W, a, x);
+        const uint32_t *xp = nullptr, *bp = nullptr;
+        uint32_t xl = 0, blen = 0;
+        if (valid) nbr(c.g, x, xp, xl);
+        S.x[lane] = x;
+        S.xo[lane] = valid ? (uint32_t)(xp - c.g.adj) : 0u;
+        S.xl[lane] = xl;
+        // one list to scan for the batch: the least scan length x probes of the others
+        int32_t bsrc = -1;
+        {
+            unsigned long long allp = 0, best = ~0ull;
+            for (uint32_t q = 0; q < ns; ++q) allp += S.shub[q] >= 0 ? 1u : search_cost(S.slen[q]);
+            const unsigned long long xcost = xl >= c.g.hub_min ? 1u : search_cost(xl);
+            if (xpar) allp += xcost;
+            for (uint32_t q = 0; q < ns; ++q) {
+                const unsigned long long own = S.shub[q] >= 0 ? 1u : search_cost(S.slen[q]);
+                const unsigned long long cost = warp_sum_u64(valid ? (unsigned long long)S.slen[q] * (allp - own + 1) : 0ull);
+                if (cost < best) { best = cost; bsrc = (int32_t)q; }
+            }
+            if (xpar) {
+                const unsigned long long cost = warp_sum_u64(valid ? (unsigned long long)xl * (allp - xcost + 1) : 0ull);
+                if (cost < best) bsrc = -1;
+            }
+        }
+        if (valid) {
+            bp = bsrc < 0 ? xp : S.sptr[bsrc];
+            blen = bsrc < 0 ? xl : S.slen[bsrc];
+            Bounds b{0u, 0xFFFFFFFFu, P.lower[i] != 0, P.upper[i] != 0};
+            for (uint32_t msk = P.lower[i]; msk; msk &= msk - 1) {
+                const uint32_t p = __ffs(msk) - 1;
+                b.lo = max(b.lo, p == a ? x : W.m[p]);
+            }
+            for (uint32_t msk = P.upper[i]; msk; msk &= msk - 1) {
+                const uint32_t p = __ffs(msk) - 1;
+                b.hi = min(b.hi, p == a ? x : W.m[p]);
+            }
+            trim(bp, blen, b);
+        }
+        const uint32_t total = enum_flatten(S, bp, blen);
+        uint32_t l = 0;
+        for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+            const uint32_t j = j0 + lane;
+            bool keep = j < total;
+            uint32_t y = 0;
+            if (keep) {
+                while (S.pref[l] <= j) ++l;
+                y = S.bp[l][j - (l ? S.pref[l - 1] : 0u)];
+                for (uint32_t q = 0; q < ns && keep; ++q)
+                    if ((int32_t)q != bsrc) keep = pair_in(W, c, S, (int)q, l, y);
+                if (keep && xpar && bsrc != -1) keep = pair_in(W, c, S, -1, l, y);
+                for (uint32_t e = 0; e < nex && keep; ++e) keep = y != S.exv[e];
+                if (keep && ex_x) keep = y != S.x[l];
+            }
+            enum_put(S, out, qn, keep, keep ? S.x[l] : 0u, y, false, write);
+        }
+        __syncwarp();
+    }
+    enum_put(S, out, qn, false, 0u, 0u, true, write);
+}
+
+// Three-vertex patterns: up to 32 roots (u, v) at once, level 2 from the
+// shorter of its lists, the other one probed.
+__device__ __forceinline__ void enum_roots(const DevPlan &P, Ctx<false> &c, bool valid, uint2 e, const EnumOut &out) {
+    PairState &S = *c.PS;
+    const uint32_t lane = lane_id();
+    const bool p0 = P.parents[2] & 1u, p1 = P.parents[2] & 2u;
+    const uint32_t *bp = nullptr;
+    uint32_t blen = 0;
+    int32_t hub = -1;
+    if (valid) {
+        uint32_t ou, ov, du, dv;
+        nbr_off(c.g, e.x, ou, du);
+        nbr_off(c.g, e.y, ov, dv);
+        const bool scan_u = p0 && (!p1 || du <= dv);
+        bp = c.g.adj + (scan_u ? ou : ov);
+        blen = scan_u ? du : dv;
+        S.xo[lane] = scan_u ? ov : ou;
+        S.xl[lane] = scan_u ? dv : du;
+        if (p0 && p1) hub = hub_slot_of(c.g, scan_u ? e.y : e.x, S.xl[lane]);
+        Bounds b{0u, 0xFFFFFFFFu, P.lower[2] != 0, P.upper[2] != 0};
+        if (P.lower[2] & 1u) b.lo = max(b.lo, e.x);
+        if (P.lower[2] & 2u) b.lo = max(b.lo, e.y);
+        if (P.upper[2] & 1u) b.hi = min(b.hi, e.x);
+        if (P.upper[2] & 2u) b.hi = min(b.hi, e.y);
+        trim(bp, blen, b);
+    }
+    LeafState &L = *c.L;
+    L.cm[lane][0] = e.x;
+    L.cm[lane][1] = e.y;
+    S.tr[lane] = (uint32_t)hub;
+    const uint32_t total = enum_flatten(S, bp, blen);
+    uint32_t l = 0, qn = 0;
+    auto write = [&](unsigned long long row, uint32_t r, uint32_t y) {   // (r: the root's lane)
+        uint32_t *o = out.rows + row * 3;
+        o[P.order_[0]] = L.cm[r][0];
+        o[P.order_[1]] = L.cm[r][1];
+        o[P.order_[2]] = y;
+    };
+    for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        bool keep = j < total;
+        uint32_t y = 0;
+        if (keep) {
+            while (S.pref[l] <= j) ++l;
+            y = S.bp[l][j - (l ? S.pref[l - 1] : 0u)];
+            if (p0 && p1) {
+                const int32_t h = (int32_t)S.tr[l];
+                keep = h >= 0 ? hub_has(c.g, h, y) : contains(c.g.adj + S.xo[l], S.xl[l], y);
+            }
+            if ((P.check[2] & 1u) && y == L.cm[l][0]) keep = false;
+            if ((P.check[2] & 2u) && y == L.cm[l][1]) keep = false;
+        }
+        enum_put(S, out, qn, keep, l, y, false, write);
+    }
+    enum_put(S, out, qn, false, 0u, 0u, true, write);
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(256) enum_kernel(DevGraph g, const DevPlan *__restrict__ plan,
                                                    unsigned long long *queue, uint32_t *scratch, uint32_t cap,
-                                                   uint32_t bufs_per_warp, uint32_t *flags, uint32_t *out,
-                                                   unsigned long long out_cap, unsigned long long *out_n) {
+                                                   uint32_t bufs_per_warp, uint32_t *flags, EnumOut out) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t lane = lane_id();
     const uint32_t wib = threadIdx.x >> 5;
@@ -1860,13 +2047,18 @@ __global__ void __launch_bounds__(256) enum_kernel(DevGraph g, const DevPlan *__
     c.tstart = 0;
     c.deadline = 0;
     WarpState &W = setup_warp(smem_raw, wib, 0u, 0u, 1u, 1u, SGE_MAX_VSLOTS, c);
-    const uint32_t k = P.k, last = k - 1;
+    const uint32_t k = P.k, a = k - 2, grab = k == 3 ? 32u : 1u;
     while (true) {
         unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(queue, 1ull);
+        if (lane == 0) t = atomicAdd(queue, (unsigned long long)grab);
         t = __shfl_sync(FULL_MASK, t, 0);
         if (t >= P.ntasks) break;
         if (*(volatile uint32_t *)flags & FLAG_OVERFLOW) break;
+        if (k == 3) {
+            const bool valid = t + lane < P.ntasks;
+            enum_roots(P, c, valid, valid ? root_edge(g, P, t + lane) : make_uint2(0, 0), out);
+            continue;
+        }
         const uint2 e = root_edge(g, P, t);
         set_match(g, W, 0, e.x);
         set_match(g, W, 1, e.y);
@@ -1874,27 +2066,8 @@ __global__ void __launch_bounds__(256) enum_kernel(DevGraph g, const DevPlan *__
         bool ok = build_level_wcoj(P, W, c, lv);
         if (ok) { __syncwarp(); if (lane == 0) W.pos[lv] = 0; __syncwarp(); }
         while (ok) {
-            if (lv == last) {
-                const uint32_t n = W.cnt[lv];
-                const uint32_t *lst = W.list[lv];
-                for (uint32_t b0 = 0; b0 < n; b0 += 32) {
-                    const uint32_t idx = b0 + lane;
-                    bool valid = idx < n;
-                    const uint32_t x = valid ? lst[idx] : 0u;
-                    if (valid) valid = !excluded(P, W, lv, x);
-                    const uint32_t bal = __ballot_sync(FULL_MASK, valid);
-                    unsigned long long base = 0;
-                    if (lane == 0 && bal) base = atomicAdd(out_n, (unsigned long long)__popc(bal));
-                    base = __shfl_sync(FULL_MASK, base, 0);
-                    if (valid) {
-                        const unsigned long long row = base + __popc(bal & ((1u << lane) - 1u));
-                        if (row < out_cap) {
-                            uint32_t *o = out + row * k;
-                            for (uint32_t l = 0; l < last; ++l) o[P.order_[l]] = W.m[l];
-                            o[P.order_[last]] = x;
-                        }
-                    }
-                }
+            if (lv == a) {
+                enum_pairs(P, W, c, a, out);
                 if (lv == 2) break;
                 --lv;
                 continue;
@@ -3336,6 +3509,13 @@ sge_status sge_batch_run(sge_batch *b, uint64_t *counts, uint64_t *instances, sg
 }
 
 sge_status sge_enumerate(sge_graph *g, const sge_plan *p, uint32_t *d_out, uint64_t capacity, uint64_t *n_matches) {
+    return sge::enumerate_rows(g, p, d_out, capacity, n_matches, false);
+}
+
+}  // extern "C"
+
+sge_status sge::enumerate_rows(sge_graph *g, const sge_plan *p, uint32_t *d_out, uint64_t capacity,
+                               uint64_t *n_matches, bool any_representative) {
     if (!g || !p || !n_matches || (!d_out && capacity)) return fail(SGE_BAD_INPUT, "sge_enumerate: null argument");
     if (p->blob.tail_len != 1)
         return fail(SGE_BAD_INPUT, "sge_enumerate needs a plan with a one-level tail (plan it without IEP)");
@@ -3343,7 +3523,9 @@ sge_status sge_enumerate(sge_graph *g, const sge_plan *p, uint32_t *d_out, uint6
     DeviceGuard restore_device;
     CUDA_TRY(cudaSetDevice(g->device));
     DevPlan d = p->dp;
+    if (any_representative && g->mirror) mirror_plan(d);
     d.ne = d.k;  // every level is enumerated
+    d.join_style = SGE_JOIN_WCOJ;  // (the same tuples; running lists are not kept here)
     d.ntrie = 0;
     d.hoist_mask = 0;
     d.root_stride = 1;
@@ -3375,7 +3557,8 @@ sge_status sge_enumerate(sge_graph *g, const sge_plan *p, uint32_t *d_out, uint6
     CUDA_TRY(cudaMemcpyAsync(B, &d, sizeof(DevPlan), cudaMemcpyHostToDevice, g->stream));
     DevGraph dg = dev_graph(g, true);
     enum_kernel<<<(unsigned)blocks, threads, smem, g->stream>>>(dg, reinterpret_cast<const DevPlan *>(B), dq,
-                                                                g->d_scratch, cap, d.nbufs, dflags, d_out, capacity, dn);
+                                                                g->d_scratch, cap, d.nbufs, dflags,
+                                                                EnumOut{d_out, capacity, dn});
     CUDA_TRY(cudaGetLastError());
     unsigned long long n = 0;
     uint32_t flags = 0;
@@ -3387,6 +3570,8 @@ sge_status sge_enumerate(sge_graph *g, const sge_plan *p, uint32_t *d_out, uint6
     if (n > capacity) return fail(SGE_OOM, "%llu matches exceed the output capacity %llu", n, (unsigned long long)capacity);
     return SGE_OK;
 }
+
+extern "C" {
 
 sge_status sge_count_host(const uint32_t *offsets, const uint32_t *nbrs, uint32_t n, uint64_t nnz,
                           const sge_plan_blob *blobs, uint32_t nplans, const sge_count_opts *opts, uint64_t *counts,
@@ -3608,15 +3793,23 @@ void strip_restrictions(sge_plan_blob &b) {
 // One relation: count its tuples, enumerate them, sort, build the trie and
 // its dense first level.  *skipped is set (and nothing built) when the
 // relation holds more than max_rows tuples.
-sge_status build_rel(sge_graph *g, const sge_plan_blob &blob, uint32_t arity, uint64_t max_rows, size_t bag,
+sge_status build_rel(sge_graph *g, sge_plan_blob blob, uint32_t arity, uint64_t max_rows, size_t bag,
                      BagRel &r, bool *skipped) {
     *skipped = false;
+    // the embeddings are the instances times the automorphisms: counted under
+    // the restrictions, enumerated without them
     sge_plan *sp = nullptr;
     sge_status st = sge_plan_create(&blob, &sp);
     if (st != SGE_OK) return st;
     uint64_t cnt = 0, rows = 0;
     const sge_plan *cp = sp;
     st = sge_count(g, &cp, 1, nullptr, &cnt, &rows, nullptr);
+    sge_plan_destroy(sp);
+    sp = nullptr;
+    if (st != SGE_OK) return st;
+    rows *= blob.aut_size;
+    strip_restrictions(blob);
+    if ((st = sge_plan_create(&blob, &sp)) != SGE_OK) return st;
     if (st == SGE_OK && rows > max_rows) {
         sge_plan_destroy(sp);
         *skipped = true;
@@ -3714,7 +3907,6 @@ sge_status sge_bags_create(sge_graph *g, uint32_t k, uint32_t m, const uint32_t 
         // a bag whose sub-pattern is not connected is not planned (its tail
         // level keeps intersecting adjacency lists)
         if (sge_plan_pattern_stats(size, (uint32_t)sub.size() / 2, sub.data(), &g->stats, &o, &blob) != SGE_OK) continue;
-        strip_restrictions(blob);
         // (the sort and the trie index rows with 32 bits)
         const uint64_t cap = std::min<uint64_t>(max_rows ? max_rows : ~0ull, 0xFFFFFFFFull);
         bool skipped = false;

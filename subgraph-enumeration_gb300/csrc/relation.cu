@@ -636,26 +636,42 @@ sge_status sge_trie_free(sge_trie *t) {
 }
 
 // The sorted instance set of a pattern (the embedding set -r writes; the
-// reference never produces one): count, enumerate into an exactly sized
-// device buffer, canonicalise under the automorphisms, sort, copy to host.
+// reference never produces one): enumerate into a device buffer, canonicalise
+// under the automorphisms, sort, copy to host.
 sge_status sge_match_set(sge_graph *g, const sge_plan *p, uint32_t k, uint32_t m, const uint32_t *edges,
                          uint32_t *host_out, uint64_t cap_rows, uint64_t *n_rows) {
     if (!g || !p || !n_rows || (!host_out && cap_rows)) return fail(SGE_BAD_INPUT, "sge_match_set: null argument");
-    uint64_t counts = 0, inst = 0;
-    const sge_plan *pp = p;
-    sge_status st = sge_count(g, &pp, 1, nullptr, &counts, &inst, nullptr);
-    if (st != SGE_OK) return st;
-    *n_rows = inst;
-    if (inst > cap_rows) return fail(SGE_OOM, "%llu instances exceed the %llu-row output", (unsigned long long)inst,
-                                     (unsigned long long)cap_rows);
-    if (inst == 0) return SGE_OK;
+    // a buffer of the caller's own size is filled directly, unless it would
+    // take much of the device: then the instances are counted first
+    uint64_t inst = cap_rows, n2 = 0;
+    size_t free_b = 0, tot_b = 0;
+    CUDA_TRY(cudaMemGetInfo(&free_b, &tot_b));
+    const bool counted = cap_rows > std::min<uint64_t>(1ull << 30, free_b / 8) / (4ull * std::max<uint32_t>(k, 1));
+    if (counted) {
+        uint64_t counts = 0;
+        const sge_plan *pp = p;
+        const sge_status cst = sge_count(g, &pp, 1, nullptr, &counts, &inst, nullptr);
+        if (cst != SGE_OK) return cst;
+        *n_rows = inst;
+        if (inst > cap_rows) return fail(SGE_OOM, "%llu instances exceed the %llu-row output", (unsigned long long)inst,
+                                         (unsigned long long)cap_rows);
+        if (inst == 0) return SGE_OK;
+    }
     uint32_t *d = nullptr;
-    CUDA_TRY(cudaMalloc(&d, inst * k * 4ull));
-    uint64_t n2 = 0;
-    st = sge_enumerate(g, p, d, inst, &n2);
-    if (st == SGE_OK && n2 != inst)
+    if (inst) CUDA_TRY(cudaMalloc(&d, inst * k * 4ull));
+    sge_status st = enumerate_rows(g, p, d, inst, &n2, true);
+    if (counted && st == SGE_OK && n2 != inst)
         st = fail(SGE_CUDA_ERROR, "enumeration produced %llu rows but the count is %llu", (unsigned long long)n2,
                   (unsigned long long)inst);
+    if (!counted && (st == SGE_OK || st == SGE_OOM)) {
+        *n_rows = inst = n2;
+        if (n2 > cap_rows) st = fail(SGE_OOM, "%llu instances exceed the %llu-row output", (unsigned long long)n2,
+                                     (unsigned long long)cap_rows);
+    }
+    if (st != SGE_OK || inst == 0) {
+        cudaFree(d);
+        return st;
+    }
     std::vector<uint8_t> perms((size_t)4096 * k);
     uint32_t naut = 0;
     if (st == SGE_OK) st = sge_pattern_automorphisms(k, m, edges, perms.data(), 4096, &naut);
