@@ -125,6 +125,8 @@ struct DevPlan {
     uint32_t split_H;                             // roots whose level-2 bound exceeds this are deferred
     uint32_t split_S;                             // level-2 candidates per deferred task (0 = never defer)
     uint32_t split_P3;                            // parts of each level-3 list per deferred task (1 = none)
+    uint32_t split_par3;                          // level 3's parents among levels 0/1
+    uint32_t split_W;                             // level-2 candidates x level-3 bound per task (0 = not used)
     uint32_t pair;                                // 1: the last two enumerated levels run as one flattened step
     uint32_t pair_direct;                         // pair step may count a single-list tail per pair inline
     uint32_t epin;                                // exploration: tail level whose root-level running list is pinned
@@ -170,6 +172,8 @@ struct WarpState {
     uint32_t pmode[3];                    // pinned N(m[0]), N(m[1]), level-2 list: 0 none, 1 bitmap, 2 hash
     uint32_t hcnt[SGE_MAX_K];             // hoisted tail lists (buffer slot = level)
     uint32_t hpin;                        // tail level whose hoisted list is pinned in table 2 (0 = none)
+    uint32_t troot, tpin;                 // trie slots keyed by levels 0 and 1 alone; 1 + the one pinned in table 2
+    uint32_t toff[2], tlen[2];            // their ranges
     unsigned long long t_root;            // globaltimer at the start of the current root (per-plan busy time)
 };
 
@@ -421,7 +425,7 @@ __device__ __forceinline__ uint32_t probe_cost(const WarpState &W, uint32_t j, u
 // Pins a sorted list into table ti (a bitmap over all vertices, or an
 // open-addressing hash when it is at most half full); records the mode.
 template <bool STATS>
-__device__ void pin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
+__device__ __forceinline__ void pin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
     const uint32_t lane = lane_id();
     uint32_t mode = c.tmode;
     if (mode == 2 && len * 2u > c.tw) mode = 0;
@@ -445,7 +449,7 @@ __device__ void pin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_
 }
 
 template <bool STATS>
-__device__ void unpin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
+__device__ __forceinline__ void unpin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
     const uint32_t lane = lane_id();
     const uint32_t mode = W.pmode[ti];
     uint32_t *t = c.tab + ti * c.tw;
@@ -465,7 +469,7 @@ __device__ void unpin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint3
 
 // Pins N(m[0]) and N(m[1]) (levels probed inside the DFS).
 template <bool STATS>
-__device__ void pin_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
+__device__ __forceinline__ void pin_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
     for (uint32_t j = 0; j < 2; ++j)
         if ((P.pin_mask >> j) & 1u) pin_list(W, c, j, W.lptr[j], W.llen[j]);
 }
@@ -488,17 +492,20 @@ __device__ __forceinline__ const uint32_t *version_ptr(const DevPlan &P, const W
 }
 
 template <bool STATS>
-__device__ void unpin_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
+__device__ __forceinline__ void unpin_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
     for (uint32_t j = 0; j < 2; ++j)
         if (W.pmode[j]) unpin_list(W, c, j, W.lptr[j], W.llen[j]);
     if (W.pmode[2]) {
-        if (W.hpin && P.join_style == SGE_JOIN_EXPLORATION)
+        if (W.tpin) {
+            const DevTrie &T = P.tries[P.trel[W.tpin - 1]];
+            unpin_list(W, c, 2, T.val[T.nkeys] + W.toff[W.tpin - 1], W.tlen[W.tpin - 1]);
+        } else if (W.hpin && P.join_style == SGE_JOIN_EXPLORATION)
             unpin_list(W, c, 2, version_ptr(P, W, c, 1, W.hpin), version_len(P, W, c, 1, W.hpin));
         else if (W.hpin) unpin_list(W, c, 2, c.buf + (size_t)W.hpin * c.cap, W.hcnt[W.hpin]);
         else unpin_list(W, c, 2, W.flist[2], W.fcnt[2]);
     }
     __syncwarp();
-    if (lane_id() == 0) W.hpin = 0;
+    if (lane_id() == 0) { W.hpin = 0; W.tpin = 0; }
     __syncwarp();
 }
 
@@ -820,6 +827,7 @@ __device__ __forceinline__ unsigned long long trie_lookups(const DevPlan &P, con
                                                         uint32_t L0, uint32_t l) {
     unsigned long long bytes = 0;
     for (uint32_t j = 0; j < P.ntrie; ++j) {
+        if ((W.troot >> j) & 1u) continue;   // the same range for every candidate
         const DevTrie &Tr = P.tries[P.trel[j]];
         uint32_t key[3];
         for (uint32_t q = 0; q < Tr.nkeys; ++q) {
@@ -891,7 +899,7 @@ __device__ __forceinline__ bool td_member(const TailDesc &D, const LeafState &L,
 
 // Fills D for tail level i from the lists for_tail_lists visits.
 template <bool STATS>
-__device__ void tail_desc(const DevPlan &P, const WarpState &W, const LeafState &L, const Ctx<STATS> &c,
+__device__ __forceinline__ void tail_desc(const DevPlan &P, const WarpState &W, const LeafState &L, const Ctx<STATS> &c,
                           const LeafCtx &lc, uint32_t i, TailDesc &D) {
     uint32_t n = 0;
     if (P.ntrie && P.tri[i] >= 0) {
@@ -903,6 +911,11 @@ __device__ void tail_desc(const DevPlan &P, const WarpState &W, const LeafState 
         D.lvl[0] = -1;
         D.ptr[0] = T.val[T.nkeys];
         D.len[0] = 0;
+        if ((W.troot >> j) & 1u) {   // one list for all candidates, pinned in table 2 or sorted
+            D.kind[0] = W.tpin == j + 1u ? 2u : 3u;
+            D.ptr[0] += W.toff[j];
+            D.len[0] = W.tlen[j];
+        }
         n = 1;
     } else
     for_tail_lists(P, W, L, c, lc, 0, i, [&](const uint32_t *p, uint32_t len, int src, bool pinned) {
@@ -946,7 +959,7 @@ __device__ void tail_desc(const DevPlan &P, const WarpState &W, const LeafState 
 }
 
 template <bool STATS>
-__device__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t L0,
+__device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t L0,
                                          uint32_t ncand) {
     LeafState &L = *c.L;
     const uint32_t lane = lane_id();
@@ -1130,7 +1143,7 @@ __device__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<STA
 // Leaf over up to 32 root edges (plans with only two enumerated levels):
 // lane l < n holds root (u, v).
 template <bool STATS>
-__device__ unsigned long long leaf_roots(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t n, uint32_t u,
+__device__ __forceinline__ unsigned long long leaf_roots(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t n, uint32_t u,
                                          uint32_t v) {
     LeafState &L = *c.L;
     const uint32_t lane = lane_id();
@@ -1248,7 +1261,8 @@ __device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<STAT
 // without one warp-wide set operation and one short leaf call per x.
 // Returns false on timeout.
 template <bool STATS>
-__device__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t a, unsigned long long &acc) {
+__device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t a,
+                                           unsigned long long &acc, uint32_t part, uint32_t parts) {
     PairState &S = *c.PS;
     const uint32_t lane = lane_id();
     const uint32_t i = a + 1;
@@ -1373,11 +1387,19 @@ __device__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32
             if (lane >= o) incl += v;
         }
         S.pref[lane] = incl;
-        const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
+        uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
         __syncwarp();
+        uint32_t begin = 0;   // this task's part of the scan (the pair step's level is level 2)
+        if (parts > 1) {
+            begin = (uint32_t)((unsigned long long)total * part / parts);
+            total = (uint32_t)((unsigned long long)total * (part + 1) / parts);
+        }
         // 3. flattened scan; survivors are appended to the pair queue
         uint32_t l = 0;
-        for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+        // (one step past the last batch's scan drains the queue: the leaf is
+        // inlined once)
+        const bool last = b0 + 32 >= n;
+        for (uint32_t j0 = begin; j0 < total || (last && qn); j0 += 32) {
             if (j0 && (j0 & 0x1FFFu) == 0 && out_of_time(c)) { ok = false; break; }
             const uint32_t j = j0 + lane;
             bool keep = j < total;
@@ -1421,18 +1443,18 @@ __device__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32
             qn += __popc(kb);
             if (STATS) c.partial += __popc(kb);
             __syncwarp();
-            if (qn >= 32) {
-                acc += pair_flush(P, W, c, a, 32u);
+            if (qn >= 32 || j0 >= total) {
+                const uint32_t take = min(qn, 32u);
+                acc += pair_flush(P, W, c, a, take);
                 // move the remainder (< 32 pairs) to the front of the queue
                 const uint32_t rx = S.qx[32 + lane], ry = S.qy[32 + lane];
                 __syncwarp();
-                if (lane < qn - 32) { S.qx[lane] = rx; S.qy[lane] = ry; }
-                qn -= 32;
+                qn -= take;
+                if (lane < qn) { S.qx[lane] = rx; S.qy[lane] = ry; }
                 __syncwarp();
             }
         }
     }
-    if (ok && qn) acc += pair_flush(P, W, c, a, qn);
     if (inl) acc += warp_sum_u64(isum);
     return ok;
 }
@@ -1451,16 +1473,47 @@ __device__ __forceinline__ bool out_of_time(Ctx<STATS> &c) {
     return true;
 }
 
+// Bag relations keyed by levels 0 and 1 alone: their ranges are looked up once
+// per root, and the first one is pinned in table 2 when that is free, so that
+// the leaf's passes test it with one shared-memory load instead of a bisection
+// of the trie (two triangles joined by a 4-cycle, 1,500 roots of R-MAT 2^14:
+// some 4,400 such tests per 32 candidates; 54 -> 30 ms).
+template <bool STATS>
+__device__ __forceinline__ void root_tries(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
+    for (uint32_t j = 0; j < P.ntrie; ++j) {
+        const DevTrie &T = P.tries[P.trel[j]];
+        uint32_t key[3];
+        bool at_root = true;
+        for (uint32_t q = 0; q < T.nkeys; ++q) {
+            at_root &= P.tkey[j][q] < 2;
+            key[q] = W.m[P.tkey[j][q] & 1u];
+        }
+        if (!at_root) continue;
+        uint32_t off, len;
+        trie_range(T, key, off, len);
+        __syncwarp();
+        if (lane_id() == 0) { W.troot |= 1u << j; W.toff[j] = off; W.tlen[j] = len; }
+        __syncwarp();
+        if (c.tmode && !W.tpin && !((P.pin_mask >> 2) & 1u) && W.hpin == 0u && W.pmode[2] == 0u) {
+            pin_list(W, c, 2, T.val[T.nkeys] + off, len);
+            if (lane_id() == 0 && W.pmode[2]) W.tpin = j + 1;
+            __syncwarp();
+        }
+    }
+}
+
 // r2b/r2e restrict the level-2 candidates processed, and p3 of np3 the part
 // of each level-3 list (a heavy root is split into tasks over ranges of its
 // level-2 list and equal parts of the level-3 lists below them).
-template <bool STATS>
-__device__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t u, uint32_t v,
+// TWO: plans with two enumerated levels come here too (count_kernel takes
+// their roots 32 at a time itself).
+template <bool STATS, bool TWO = false>
+__device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t u, uint32_t v,
                                        uint32_t r2b = 0u, uint32_t r2e = 0xFFFFFFFFu, uint32_t p3 = 0u,
                                        uint32_t np3 = 1u) {
     const uint32_t lane = lane_id();
     const uint32_t ne = P.ne;
-    if (ne == 2) return leaf_roots(P, W, c, 1u, u, v);
+    if (TWO && ne == 2) return leaf_roots(P, W, c, 1u, u, v);
     const bool explore = P.join_style == SGE_JOIN_EXPLORATION;
     const uint32_t L0 = ne - 1;
     const uint32_t Lt = P.pair ? ne - 2 : L0;  // level whose candidates end the DFS
@@ -1481,6 +1534,7 @@ __device__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<STATS
     } else if (P.hoist_mask) {
         ok = hoist_after(P, W, c, 1);
     }
+    if (!STATS && ok && P.ntrie) root_tries(P, W, c);
     uint32_t lv = 2;
     if (ok) {
         if (explore) explore_level(P, W, c, lv);
@@ -1498,7 +1552,7 @@ __device__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<STATS
     }
     while (ok) {
         if (lv == Lt && P.pair) {
-            ok = pair_level(P, W, c, lv, acc);
+            ok = pair_level(P, W, c, lv, acc, p3, lv == 2 ? np3 : 1u);
             if (lv == 2) break;
             --lv;
             continue;
@@ -1557,7 +1611,12 @@ __device__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<STATS
         }
         __syncwarp();
     }
-    if (P.pin_mask || W.hpin) unpin_root(P, W, c);
+    if (P.pin_mask || W.hpin || W.tpin) unpin_root(P, W, c);
+    if (P.ntrie) {
+        __syncwarp();
+        if (lane == 0) W.troot = 0;
+        __syncwarp();
+    }
     return ok ? acc : 0ull;
 }
 
@@ -1596,7 +1655,7 @@ __device__ __forceinline__ WarpState &setup_warp(unsigned char *smem, uint32_t w
     c.tmode = tmode;
     const uint32_t fill = tmode == 2 ? PIN_EMPTY : 0u;
     for (uint32_t w = lane_id(); w < 3 * tw; w += 32) c.tab[w] = fill;
-    if (lane_id() == 0) { W.pmode[0] = 0; W.pmode[1] = 0; W.pmode[2] = 0; W.hpin = 0; }
+    if (lane_id() == 0) { W.pmode[0] = 0; W.pmode[1] = 0; W.pmode[2] = 0; W.hpin = 0; W.troot = 0; W.tpin = 0; }
     __syncwarp();
     return W;
 }
@@ -1643,6 +1702,27 @@ __device__ __forceinline__ uint32_t level2_bound(const DevGraph &g, const DevPla
     return ub;
 }
 
+// Level-2 candidates per deferred task of a root, and whether the root is
+// deferred at all: by its level-2 bound, or, where the level below is scanned
+// once per candidate (split_W), by the two bounds' product.
+struct RootSplit {
+    uint32_t S, P3;   // level-2 candidates per task; parts of what is below one of them
+    bool heavy;
+};
+__device__ __forceinline__ RootSplit root_split(const DevGraph &g, const DevPlan &P, uint2 e, uint32_t b2) {
+    RootSplit r{P.split_S, P.split_P3, b2 > P.split_H};
+    if (P.split_W) {
+        uint32_t w = 0xFFFFFFFFu;
+        if (P.split_par3 & 1u) w = min(w, __ldg(g.off + e.x + 1) - __ldg(g.off + e.x));
+        if (P.split_par3 & 2u) w = min(w, __ldg(g.off + e.y + 1) - __ldg(g.off + e.y));
+        w = max(w, 1u);
+        r.S = max(1u, min(r.S, P.split_W / w));
+        r.P3 = min(64u, (w + P.split_W - 1) / P.split_W);
+        r.heavy |= (unsigned long long)b2 * w > 2ull * P.split_W;
+    }
+    return r;
+}
+
 // Heavy roots deferred by phase 0: their ids, per-plan counts, and the
 // exclusive prefix of their task counts (phase 1 numbers tasks densely).
 struct HeavyBuf {
@@ -1668,7 +1748,8 @@ __global__ void heavy_prefix_kernel(DevGraph g, const DevPlan *__restrict__ plan
         if (h < n && P.split_S) {
             const uint2 e = root_edge(g, P, H.ids[(size_t)p * H.cap + h]);
             const uint32_t b2 = level2_bound(g, P, e);
-            tasks = (unsigned long long)((b2 + P.split_S - 1) / P.split_S) * P.split_P3;
+            const RootSplit sp = root_split(g, P, e, b2);
+            tasks = (unsigned long long)((b2 + sp.S - 1) / sp.S) * sp.P3;
         }
         unsigned long long incl = tasks;
 #pragma unroll
@@ -1757,26 +1838,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
             continue;
         }
         const unsigned long long t1 = min(t0 + chunk, ntasks);
-        if (phase == 1) {
-            // the heavy root holding task t0: the last with pre[h] <= t0
-            const uint32_t hn = min(H.cnt[cur], H.cap);
-            const unsigned long long *pre = H.pre + (size_t)cur * H.cap;
-            uint32_t lo = 0, len = hn;
-            while (len > 0) {
-                const uint32_t half = len >> 1;
-                if (pre[lo + half] <= t0) { lo += half + 1; len -= half + 1; }
-                else len = half;
-            }
-            const uint32_t h = lo - 1;
-            const unsigned long long local = t0 - pre[h];
-            const uint2 e = root_edge(g, P, H.ids[(size_t)cur * H.cap + h]);
-            const uint32_t c2 = (uint32_t)(local / P.split_P3), q3 = (uint32_t)(local % P.split_P3);
-            if (lane == 0) W.t_root = globaltimer_ns();
-            acc += run_root<STATS>(P, W, c, e.x, e.y, c2 * P.split_S, (c2 + 1) * P.split_S, q3, P.split_P3);
-            if (lane == 0) atomicAdd(H.ptime + cur, globaltimer_ns() - W.t_root);
-            continue;
-        }
-        if (P.ne == 2) {
+        if (P.ne == 2 && phase == 0) {
             // lane l takes task t0 + l; roots the degree cap drops are compacted out
             const uint32_t n = (uint32_t)(t1 - t0);
             uint32_t u = 0, v = 0;
@@ -1806,21 +1868,43 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
             continue;
         }
         for (unsigned long long t = t0; t < t1; ++t) {
-            if (dskip && P.dcls && dense_counts_root(P, dskip, t)) continue;
-            const uint2 e = root_edge(g, P, t);
-            if (!root_kept(g, P, e)) continue;
-            ++roots;
-            if (P.split_S && level2_bound(g, P, e) > P.split_H) {
-                uint32_t slot = 0;
-                if (lane == 0) slot = atomicAdd(H.cnt + cur, 1u);
-                slot = __shfl_sync(FULL_MASK, slot, 0);
-                if (slot < H.cap) {
-                    if (lane == 0) H.ids[(size_t)cur * H.cap + slot] = (uint32_t)t;
-                    continue;
+            uint2 e;
+            uint32_t r2b = 0, r2e = 0xFFFFFFFFu, q3 = 0, np3 = 1;
+            if (phase == 1) {
+                // the heavy root holding task t: the last with pre[h] <= t
+                const uint32_t hn = min(H.cnt[cur], H.cap);
+                const unsigned long long *pre = H.pre + (size_t)cur * H.cap;
+                uint32_t lo = 0, len = hn;
+                while (len > 0) {
+                    const uint32_t half = len >> 1;
+                    if (pre[lo + half] <= t) { lo += half + 1; len -= half + 1; }
+                    else len = half;
+                }
+                const uint32_t h = lo - 1;
+                const unsigned long long local = t - pre[h];
+                e = root_edge(g, P, H.ids[(size_t)cur * H.cap + h]);
+                const RootSplit sp = root_split(g, P, e, level2_bound(g, P, e));
+                np3 = sp.P3;
+                q3 = (uint32_t)(local % np3);
+                r2b = (uint32_t)(local / np3) * sp.S;
+                r2e = r2b + sp.S;
+            } else {
+                if (dskip && P.dcls && dense_counts_root(P, dskip, t)) continue;
+                e = root_edge(g, P, t);
+                if (!root_kept(g, P, e)) continue;
+                ++roots;
+                if (P.split_S && root_split(g, P, e, level2_bound(g, P, e)).heavy) {
+                    uint32_t slot = 0;
+                    if (lane == 0) slot = atomicAdd(H.cnt + cur, 1u);
+                    slot = __shfl_sync(FULL_MASK, slot, 0);
+                    if (slot < H.cap) {
+                        if (lane == 0) H.ids[(size_t)cur * H.cap + slot] = (uint32_t)t;
+                        continue;
+                    }
                 }
             }
             if (lane == 0) W.t_root = globaltimer_ns();
-            acc += run_root<STATS>(P, W, c, e.x, e.y);
+            acc += run_root<STATS>(P, W, c, e.x, e.y, r2b, r2e, q3, np3);
             if (lane == 0) atomicAdd(H.ptime + cur, globaltimer_ns() - W.t_root);
         }
     }
@@ -2668,7 +2752,9 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // 3.5, 8 -> 3.2 ms; on all 2M of them 35.6, 42.7, 79.7 ms)
         const uint32_t split_S = split3 ? 1u
             : (uint32_t)std::min<unsigned long long>(128, std::max<unsigned long long>(8, 2ull * d.ntasks / warps));
-        const double share = (double)d.ntasks * mean_deg / (double)std::max<unsigned long long>(warps, 1);
+        // (labels leave few of the roots: one in 256 is taken for granted)
+        const double share = (double)d.ntasks * mean_deg / (double)std::max<unsigned long long>(warps, 1) /
+                             (d.vlab ? 256.0 : 1.0);
         const uint32_t thr = tu.heavy_threshold ? tu.heavy_threshold : o.heavy_threshold;
         uint32_t split_H = thr ? std::max(thr, 4u * split_S)
                                : (uint32_t)std::min(1e9, std::max(32.0, share / 4.0));
@@ -2679,7 +2765,19 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // setup would count in the instrumented kernel's totals.)
         if (!thr && !L.want_stats && d.ne == 3 && (d.parents[2] & 3u) == 3u && (d.tail_par & 4u))
             split_H = std::min(split_H, std::max(8u * split_S, 256u));
-        if (d.ne >= 3 && g->max_deg > split_H) {
+        // four enumerated levels and a leaf for every pair: under each level-2
+        // candidate the pair step scans up to level 3's root list, so roots
+        // and tasks are weighed by both bounds (two triangles joined by a
+        // 4-cycle on 1,500 roots of R-MAT 2^14: a root with 53 candidates
+        // under a list of 8,000 ran 18 ms alone; by level 2 only 31 ms, W at a
+        // half of a warp's share 30, at a 50th 16.5 ms).  A tail counted
+        // inline costs a 30th per element, and the finer tasks' set-up more
+        // than they level (house, 7,100-vertex Chung-Lu graph: 4.9 -> 5.7 ms).
+        if (!thr && !L.want_stats && d.ne == 4 && d.pair && !d.pair_direct && (d.parents[3] & 3u)) {
+            d.split_par3 = d.parents[3] & 3u;
+            d.split_W = (uint32_t)std::min(1e9, std::max(1024.0, share * mean_deg / 50.0));
+        }
+        if (d.ne >= 3 && (g->max_deg > split_H || d.split_W)) {
             d.split_S = split_S;
             d.split_H = split_H;
             d.split_P3 = split_P3;
@@ -3656,7 +3754,7 @@ __global__ void __launch_bounds__(256) count_kernel_noalloc(DevGraph g, const De
             const uint32_t v = g.adj[e];
             if (P.root_kind == SGE_ROOT_ASC && !(u < v)) continue;
             if (P.root_kind == SGE_ROOT_DESC && !(u > v)) continue;
-            acc += run_root<false>(P, W, c, u, v);
+            acc += run_root<false, true>(P, W, c, u, v);
         }
     }
     if (cur >= 0 && lane == 0 && acc) atomicAdd(counts + cur, acc * plans[cur].mult);
