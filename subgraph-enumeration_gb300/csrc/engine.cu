@@ -224,10 +224,11 @@ struct PairState {
     uint32_t x[32];                   // this batch's level-a candidates
     uint32_t xo[32];                  // N(x): CSR offset
     uint32_t xl[32];
-    const uint32_t *bp[32];           // list scanned for candidate x (trimmed by bounds)
+    int32_t xhub[32];                 // N(x)'s hub bitmap, -1 = none
+    const uint32_t *bp[32];           // list scanned for candidate x (trimmed by bounds), less the scan index it starts at
     uint32_t pref[32];
-    uint32_t qx[64], qy[64];          // (x, y) pairs waiting for the leaf
-    uint32_t tr[32];                  // inline tail: x's count before y's own exclusion
+    uint32_t qx[64], qy[64];          // (x, y) pairs waiting for the leaf; inline tail: qx = x's count before y's
+                                      // own exclusion
     TailDesc ptd;                     // inline tail: the tail level as seen from level a
 };
 
@@ -354,8 +355,9 @@ __device__ __forceinline__ bool excluded(const DevPlan &P, const WarpState &W, u
 // x may not be level i's match: an earlier match (injectivity) or, for a
 // labeled plan, a vertex of another label.  (Stored lists are filtered by
 // excluded() alone: a later level with another label may reuse them.)
-__device__ __forceinline__ bool rejected(const DevPlan &P, const WarpState &W, uint32_t i, uint32_t x) {
-    if (P.vlab && __ldg(P.vlab + x) != P.lab[i]) return true;
+__device__ __forceinline__ bool rejected(const DevPlan &P, const WarpState &W, uint32_t i, uint32_t x,
+                                         const uint32_t *vlab) {
+    if (vlab && __ldg(vlab + x) != P.lab[i]) return true;
     return excluded(P, W, i, x);
 }
 
@@ -377,7 +379,23 @@ __device__ __forceinline__ void trim(const uint32_t *&p, uint32_t &len, const Bo
     if (b.has_hi) { len = lb(p, len, b.hi); }
 }
 
-template <bool STATS>
+// What a build of the counting code holds: the instrumented counters, and
+// labeled plans and bag relations.  Most launches have neither; compiled in,
+// their branches cost the pair step registers (the 12 plans of a 7,100-vertex
+// Chung-Lu graph: 30.9 ms with them, PLAINMS ms without).
+enum { MODE_FULL = 0, MODE_STATS = 1, MODE_PLAIN = 2 };
+template <int M>
+constexpr bool stats_of = (M & MODE_STATS) != 0;
+template <int M>
+__device__ __forceinline__ const uint32_t *labels_of(const DevPlan &P) {
+    return (M & MODE_PLAIN) ? nullptr : P.vlab;
+}
+template <int M>
+__device__ __forceinline__ uint32_t ntrie_of(const DevPlan &P) {
+    return (M & MODE_PLAIN) ? 0u : P.ntrie;
+}
+
+template <int M>
 struct Ctx {
     DevGraph g;
     uint32_t *buf;    // this warp's scratch: nbufs × cap
@@ -409,8 +427,8 @@ __device__ __forceinline__ bool pin_has(const uint32_t *t, uint32_t mode, uint32
 }
 
 // y ∈ N(m[j]) for a shared level j (pinned table when present).
-template <bool STATS>
-__device__ __forceinline__ bool in_level_list(const WarpState &W, const Ctx<STATS> &c, uint32_t j, uint32_t y) {
+template <int M>
+__device__ __forceinline__ bool in_level_list(const WarpState &W, const Ctx<M> &c, uint32_t j, uint32_t y) {
     if (j < 2 && W.pmode[j]) return pin_has(c.tab + j * c.tw, W.pmode[j], c.tw, y);
     if (W.hs[j] >= 0) return hub_has(c.g, W.hs[j], y);
     return contains(W.lptr[j], W.llen[j], y);
@@ -424,8 +442,8 @@ __device__ __forceinline__ uint32_t probe_cost(const WarpState &W, uint32_t j, u
 
 // Pins a sorted list into table ti (a bitmap over all vertices, or an
 // open-addressing hash when it is at most half full); records the mode.
-template <bool STATS>
-__device__ __forceinline__ void pin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
+template <int M>
+__device__ __forceinline__ void pin_list(WarpState &W, Ctx<M> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
     const uint32_t lane = lane_id();
     uint32_t mode = c.tmode;
     if (mode == 2 && len * 2u > c.tw) mode = 0;
@@ -442,14 +460,14 @@ __device__ __forceinline__ void pin_list(WarpState &W, Ctx<STATS> &c, uint32_t t
             }
         }
     }
-    if (STATS && mode) c.alg_bytes += 4ull * len;
+    if (stats_of<M> && mode) c.alg_bytes += 4ull * len;
     __syncwarp();
     if (lane == 0) W.pmode[ti] = mode;
     __syncwarp();
 }
 
-template <bool STATS>
-__device__ __forceinline__ void unpin_list(WarpState &W, Ctx<STATS> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
+template <int M>
+__device__ __forceinline__ void unpin_list(WarpState &W, Ctx<M> &c, uint32_t ti, const uint32_t *p, uint32_t len) {
     const uint32_t lane = lane_id();
     const uint32_t mode = W.pmode[ti];
     uint32_t *t = c.tab + ti * c.tw;
@@ -468,35 +486,35 @@ __device__ __forceinline__ void unpin_list(WarpState &W, Ctx<STATS> &c, uint32_t
 }
 
 // Pins N(m[0]) and N(m[1]) (levels probed inside the DFS).
-template <bool STATS>
-__device__ __forceinline__ void pin_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
+template <int M>
+__device__ __forceinline__ void pin_root(const DevPlan &P, WarpState &W, Ctx<M> &c) {
     for (uint32_t j = 0; j < 2; ++j)
         if ((P.pin_mask >> j) & 1u) pin_list(W, c, j, W.lptr[j], W.llen[j]);
 }
 
 // Exploration: version (j, i) list length and pointer.  The first parent's
 // version is N(m[j]) itself; the others live in buffer slot[j][i].
-template <bool STATS>
-__device__ __forceinline__ uint32_t version_len(const DevPlan &P, const WarpState &W, const Ctx<STATS> &c, uint32_t j,
+template <int M>
+__device__ __forceinline__ uint32_t version_len(const DevPlan &P, const WarpState &W, const Ctx<M> &c, uint32_t j,
                                                 uint32_t i) {
     const int s = P.slot[j][i];
     return s < 0 ? W.llen[j] : c.vs[s];
 }
 
-template <bool STATS>
-__device__ __forceinline__ const uint32_t *version_ptr(const DevPlan &P, const WarpState &W, const Ctx<STATS> &c,
+template <int M>
+__device__ __forceinline__ const uint32_t *version_ptr(const DevPlan &P, const WarpState &W, const Ctx<M> &c,
                                                        uint32_t j, uint32_t i) {
     int s = P.slot[j][i];
     if (s < 0) return W.lptr[j];
     return c.buf + (size_t)s * c.cap;
 }
 
-template <bool STATS>
-__device__ __forceinline__ void unpin_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
+template <int M>
+__device__ __forceinline__ void unpin_root(const DevPlan &P, WarpState &W, Ctx<M> &c) {
     for (uint32_t j = 0; j < 2; ++j)
         if (W.pmode[j]) unpin_list(W, c, j, W.lptr[j], W.llen[j]);
     if (W.pmode[2]) {
-        if (W.tpin) {
+        if (!(M & MODE_PLAIN) && W.tpin) {
             const DevTrie &T = P.tries[P.trel[W.tpin - 1]];
             unpin_list(W, c, 2, T.val[T.nkeys] + W.toff[W.tpin - 1], W.tlen[W.tpin - 1]);
         } else if (W.hpin && P.join_style == SGE_JOIN_EXPLORATION)
@@ -522,8 +540,8 @@ __device__ __forceinline__ void set_match(const DevGraph &g, WarpState &W, uint3
 // Base list of level i for WCOJ: a reused stored list, or the parent list that
 // is cheapest to scan while probing the others; `rest` returns the parents
 // still to test.
-template <bool STATS>
-__device__ __forceinline__ void wcoj_base(const DevPlan &P, const WarpState &W, Ctx<STATS> &c, uint32_t i,
+template <int M>
+__device__ __forceinline__ void wcoj_base(const DevPlan &P, const WarpState &W, Ctx<M> &c, uint32_t i,
                                           const uint32_t *&bp, uint32_t &blen, uint32_t &rest) {
     if (P.base[i] >= 0) {
         uint32_t l = (uint32_t)P.base[i];
@@ -553,12 +571,12 @@ __device__ __forceinline__ void wcoj_base(const DevPlan &P, const WarpState &W, 
 // of `rest`, by the exclusion set of level i and (vlab: labeled plans whose
 // list no other level reuses) by its label; stores the survivors (in order)
 // to out when STORE.  Returns the survivor count (warp-uniform).
-template <bool STATS, bool STORE, bool EXCLUDE = true>
-__device__ __forceinline__ uint32_t setop(const DevPlan &P, const WarpState &W, Ctx<STATS> &c, uint32_t i,
+template <int M, bool STORE, bool EXCLUDE = true>
+__device__ __forceinline__ uint32_t setop(const DevPlan &P, const WarpState &W, Ctx<M> &c, uint32_t i,
                                           const uint32_t *bp, uint32_t blen, uint32_t rest, uint32_t *out,
                                           const uint32_t *vlab = nullptr) {
     const uint32_t lane = lane_id();
-    if (STATS) {
+    if (stats_of<M>) {
         c.set_ops += 1;
         c.alg_bytes += 4ull * blen;
         for (uint32_t msk = rest; msk; msk &= msk - 1) {
@@ -587,8 +605,8 @@ __device__ __forceinline__ uint32_t setop(const DevPlan &P, const WarpState &W, 
 // Builds level i's candidate list (WCOJ).  Returns false on overflow.
 // A level that later levels reuse keeps its full intersection (bounds not
 // applied); its own iteration range is that list trimmed by its bounds.
-template <bool STATS>
-__device__ __forceinline__ bool build_level_wcoj(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t i) {
+template <int M>
+__device__ __forceinline__ bool build_level_wcoj(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t i) {
     const uint32_t *bp;
     uint32_t blen, rest;
     wcoj_base(P, W, c, i, bp, blen, rest);
@@ -600,10 +618,10 @@ __device__ __forceinline__ bool build_level_wcoj(const DevPlan &P, WarpState &W,
     // a labeled plan stores the level's own list filtered by its label (also
     // where nothing is intersected), so that the levels below it run over the
     // few candidates that remain, 32 at a time
-    const uint32_t *vlab = keep ? nullptr : P.vlab;
+    const uint32_t *vlab = keep ? nullptr : labels_of<M>(P);
     if (rest != 0 || (vlab && blen <= c.cap)) {
         uint32_t *out = c.buf + (size_t)i * c.cap;
-        uint32_t n = setop<STATS, true>(P, W, c, i, bp, blen, rest, out, vlab);
+        uint32_t n = setop<M, true>(P, W, c, i, bp, blen, rest, out, vlab);
         if (n > c.cap) {
             if (lane_id() == 0) atomicOr(c.flags, FLAG_OVERFLOW);
             return false;
@@ -625,8 +643,8 @@ __device__ __forceinline__ bool build_level_wcoj(const DevPlan &P, WarpState &W,
 // enumerated level gets its full intersection computed once, right after its
 // last parent is matched (bounds and exclusions are applied at the leaf; a
 // labeled plan's label here, so that the leaf may count the list by its length).
-template <bool STATS>
-__device__ __forceinline__ bool hoist_after(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t j) {
+template <int M>
+__device__ __forceinline__ bool hoist_after(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t j) {
     for (uint32_t msk = P.hoist_mask; msk; msk &= msk - 1) {
         const uint32_t i = __ffs(msk) - 1;
         if (P.hoist_at[i] != j) continue;
@@ -653,7 +671,7 @@ __device__ __forceinline__ bool hoist_after(const DevPlan &P, WarpState &W, Ctx<
             rest = P.parents[i] & ~(1u << best);
         }
         uint32_t *out = c.buf + (size_t)i * c.cap;
-        const uint32_t n = setop<STATS, true, false>(P, W, c, i, bp, blen, rest, out, P.vlab);
+        const uint32_t n = setop<M, true, false>(P, W, c, i, bp, blen, rest, out, labels_of<M>(P));
         __syncwarp();
         if (lane_id() == 0) W.hcnt[i] = n;
         __syncwarp();
@@ -677,8 +695,8 @@ __device__ __forceinline__ bool hoist_after(const DevPlan &P, WarpState &W, Ctx<
 // Exploration: after level j is matched, intersect N(m[j]) into the running
 // list of every later level that has j as a parent.  false = prune (empty) or
 // overflow.  Levels past `upto` are left to the leaf.
-template <bool STATS>
-__device__ __forceinline__ bool explore_update(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t j) {
+template <int M>
+__device__ __forceinline__ bool explore_update(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t j) {
     const uint32_t lane = lane_id();
     for (uint32_t msk = P.after[j]; msk; msk &= msk - 1) {
         uint32_t i = __ffs(msk) - 1;
@@ -697,7 +715,7 @@ __device__ __forceinline__ bool explore_update(const DevPlan &P, WarpState &W, C
         // scan the running list, probe N(m[j]) (pinned table when present)
         const bool pinned = j < 2 && W.pmode[j];
         const bool scan_prev = pinned || plen <= W.llen[j];
-        if (STATS) {
+        if (stats_of<M>) {
             c.set_ops += 1;
             c.alg_bytes += scan_prev ? 4ull * plen + probe_bytes(plen, W.llen[j], pinned || W.hs[j] >= 0)
                                      : 8ull + 4ull * (plen + W.llen[j]);
@@ -727,8 +745,8 @@ __device__ __forceinline__ bool explore_update(const DevPlan &P, WarpState &W, C
 }
 
 // Exploration: level i's candidates = its running list (last parent's version), trimmed.
-template <bool STATS>
-__device__ __forceinline__ void explore_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t i) {
+template <int M>
+__device__ __forceinline__ void explore_level(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t i) {
     uint32_t lastp = 31 - __clz(P.parents[i]);
     const uint32_t *bp = version_ptr(P, W, c, lastp, i);
     uint32_t blen = version_len(P, W, c, lastp, i);
@@ -760,9 +778,9 @@ struct LeafCtx {
 // Visits the lists whose intersection is tail level i's candidate set for
 // candidate l: f(ptr, len, src, pinned) with src = level of the list, or -1 for
 // the shared running list (exploration).  f returns false to stop.
-template <bool STATS, class F>
+template <int M, class F>
 __device__ __forceinline__ void for_tail_lists(const DevPlan &P, const WarpState &W, const LeafState &L,
-                                               const Ctx<STATS> &c, const LeafCtx &lc, uint32_t l, uint32_t i, F f) {
+                                               const Ctx<M> &c, const LeafCtx &lc, uint32_t l, uint32_t i, F f) {
     const uint32_t below = (1u << lc.L0) - 1u;
     uint32_t shared = P.parents[i] & below, cand = P.parents[i] & ~below;
     if (!lc.explore && ((P.hoist_mask >> i) & 1u)) {
@@ -852,9 +870,9 @@ __device__ __forceinline__ uint32_t td_len(const TailDesc &D, const LeafState &L
 }
 
 // y ∈ list q of the level for candidate l.
-template <bool STATS>
+template <int M>
 __device__ __forceinline__ bool td_has(const TailDesc &D, const LeafState &L, const WarpState &W,
-                                       const Ctx<STATS> &c, uint32_t q, uint32_t l, uint32_t y) {
+                                       const Ctx<M> &c, uint32_t q, uint32_t l, uint32_t y) {
     const uint32_t k = D.kind[q];
     if (k < 3) return pin_has(c.tab + k * c.tw, W.pmode[k], c.tw, y);
     if (k == 3) {
@@ -886,23 +904,23 @@ __device__ __forceinline__ bool td_excluded(const TailDesc &D, const LeafState &
 }
 
 // y ∈ the level's candidate set for candidate l (bounds, every list, exclusions).
-template <bool STATS>
+template <int M>
 __device__ __forceinline__ bool td_member(const TailDesc &D, const LeafState &L, const WarpState &W,
-                                          const Ctx<STATS> &c, uint32_t l, uint32_t y) {
+                                          const Ctx<M> &c, uint32_t l, uint32_t y) {
     const Bounds b = td_bounds(D, L, l);
     if ((b.has_lo && y <= b.lo) || (b.has_hi && y >= b.hi)) return false;
     for (uint32_t q = 0; q < D.nsrc; ++q)
         if (!td_has(D, L, W, c, q, l, y)) return false;
-    if (D.vlab && __ldg(D.vlab + y) != D.lab) return false;  // labeled plans
+    if (!(M & MODE_PLAIN) && D.vlab && __ldg(D.vlab + y) != D.lab) return false;  // labeled plans
     return !td_excluded(D, L, l, y);
 }
 
 // Fills D for tail level i from the lists for_tail_lists visits.
-template <bool STATS>
-__device__ __forceinline__ void tail_desc(const DevPlan &P, const WarpState &W, const LeafState &L, const Ctx<STATS> &c,
+template <int M>
+__device__ __forceinline__ void tail_desc(const DevPlan &P, const WarpState &W, const LeafState &L, const Ctx<M> &c,
                           const LeafCtx &lc, uint32_t i, TailDesc &D) {
     uint32_t n = 0;
-    if (P.ntrie && P.tri[i] >= 0) {
+    if (ntrie_of<M>(P) && P.tri[i] >= 0) {
         // the bag relation's trie: each candidate's child range (looked up at
         // the start of the leaf) is the whole candidate list
         const uint32_t j = (uint32_t)P.tri[i];
@@ -930,7 +948,7 @@ __device__ __forceinline__ void tail_desc(const DevPlan &P, const WarpState &W, 
         return true;
     });
     D.nsrc = (uint8_t)n;
-    D.vlab = P.vlab;
+    D.vlab = labels_of<M>(P);
     D.lab = P.lab[i];
     D.has_lo = P.lower[i] != 0;
     D.has_hi = P.upper[i] != 0;
@@ -958,8 +976,8 @@ __device__ __forceinline__ void tail_desc(const DevPlan &P, const WarpState &W, 
     D.nex = (uint8_t)nex;
 }
 
-template <bool STATS>
-__device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t L0,
+template <int M>
+__device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t L0,
                                          uint32_t ncand) {
     LeafState &L = *c.L;
     const uint32_t lane = lane_id();
@@ -970,7 +988,7 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
     __syncwarp();
     if (lane < passes) tail_desc(P, W, L, c, lc, ne + lane, c.td[lane]);
     unsigned long long tbytes = 0;
-    if (P.ntrie && lane < ncand) tbytes = trie_lookups(P, W, L, L0, lane);
+    if (ntrie_of<M>(P) && lane < ncand) tbytes = trie_lookups(P, W, L, L0, lane);
     if (P.tail_mode != SGE_TAIL_SINGLE) {
         for (uint32_t q = 0; q < c.cs; ++q) c.cnt[lane * c.cs + q] = 0;
     }
@@ -998,7 +1016,7 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
         // is a plain count too)
         // (a labeled plan's only where the list holds that label alone)
         const bool direct = (P.tail_mode != SGE_TAIL_IEP || t + 1 == T) && D.nsrc == 1 &&
-                            (!P.vlab || ((P.hoist_mask >> (ne + tp)) & 1u));
+                            (!labels_of<M>(P) || ((P.hoist_mask >> (ne + tp)) & 1u));
         if (direct) {
             if (lane < ncand) {
                 const uint32_t *fp = td_ptr(D, L, 0, lane);
@@ -1017,7 +1035,7 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
                 if (P.tail_mode == SGE_TAIL_SINGLE) single += cnt;
                 else if (P.tail_mode == SGE_TAIL_CHOOSE) c.cnt[(lane) * c.cs + (1)] = cnt;
                 else c.cnt[(lane) * c.cs + (1u << tp)] = cnt;
-                if (STATS) bytes += 4ull * (2u + __popc(P.check[ne + tp])) * (31u - __clz(blen + 1u));
+                if (stats_of<M>) bytes += 4ull * (2u + __popc(P.check[ne + tp])) * (31u - __clz(blen + 1u));
             }
             __syncwarp();
             continue;
@@ -1047,13 +1065,12 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
             bp = td_ptr(D, L, bq, lane);
             blen = td_len(D, L, bq, lane);
             trim(bp, blen, td_bounds(D, L, lane));
-            if (STATS) {  // the scanned range, and each other list probed once per element of it
+            if (stats_of<M>) {  // the scanned range, and each other list probed once per element of it
                 bytes += 4ull * blen;
                 for (uint32_t q = 0; q < D.nsrc; ++q)
                     if (q != bq) bytes += probe_bytes(blen, td_len(D, L, q, lane), td_probe_cost(D, L, W, c.g, q, lane) == 1);
             }
         }
-        L.bptr[lane] = bp;
         uint32_t incl = blen;
 #pragma unroll
         for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -1061,6 +1078,7 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
             if (lane >= o) incl += v;
         }
         L.pref[lane] = incl;
+        L.bptr[lane] = bp - (incl - blen);   // (indexed by the scan's element)
         const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
         __syncwarp();
         const uint32_t ns = D.nsrc;
@@ -1085,13 +1103,12 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
             const uint32_t j = j0 + lane;
             if (j >= total) break;
             while (L.pref[l] <= j) ++l;
-            const uint32_t start = l ? L.pref[l - 1] : 0u;
-            const uint32_t y = L.bptr[l][j - start];
+            const uint32_t y = L.bptr[l][j];
             bool ok = true;
             for (uint32_t q = 0; q < ns && ok; ++q)
                 if (q != bq) ok = td_has(D, L, W, c, q, l, y);
             if (ok) ok = !td_excluded(D, L, l, y);
-            if (ok && P.vlab) ok = __ldg(P.vlab + y) == D.lab;
+            if (labels_of<M>(P) && ok) ok = __ldg(labels_of<M>(P) + y) == D.lab;
             if (!ok) continue;
             if (P.tail_mode == SGE_TAIL_SINGLE) {
                 ++single;
@@ -1132,7 +1149,7 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
             }
         }
     }
-    if (STATS) {
+    if (stats_of<M>) {
         c.alg_bytes += warp_sum_u64(bytes);
         c.set_ops += (unsigned long long)ncand * passes;
     }
@@ -1142,8 +1159,8 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
 
 // Leaf over up to 32 root edges (plans with only two enumerated levels):
 // lane l < n holds root (u, v).
-template <bool STATS>
-__device__ __forceinline__ unsigned long long leaf_roots(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t n, uint32_t u,
+template <int M>
+__device__ __forceinline__ unsigned long long leaf_roots(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t n, uint32_t u,
                                          uint32_t v) {
     LeafState &L = *c.L;
     const uint32_t lane = lane_id();
@@ -1159,8 +1176,8 @@ __device__ __forceinline__ unsigned long long leaf_roots(const DevPlan &P, WarpS
 
 // Pair step helpers.  The leaf takes up to 32 queued (x, y) pairs as its
 // candidates with L0 = a: cm[l][0] = x (level a), cm[l][1] = y (level a+1).
-template <bool STATS>
-__device__ __forceinline__ unsigned long long pair_flush(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t a,
+template <int M>
+__device__ __forceinline__ unsigned long long pair_flush(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t a,
                                                          uint32_t nq) {
     LeafState &L = *c.L;
     PairState &S = *c.PS;
@@ -1179,8 +1196,8 @@ __device__ __forceinline__ unsigned long long pair_flush(const DevPlan &P, WarpS
 // Level a+1's lists that are the same for every candidate x of level a
 // (matched levels below a only), its exclusion values, and whether N(x) is
 // one of its lists.  Mirrors build_level_wcoj / explore_level for level a+1.
-template <bool STATS>
-__device__ __forceinline__ void pair_sources(const DevPlan &P, const WarpState &W, const Ctx<STATS> &c,
+template <int M>
+__device__ __forceinline__ void pair_sources(const DevPlan &P, const WarpState &W, const Ctx<M> &c,
                                              uint32_t a) {
     PairState &S = *c.PS;
     const uint32_t i = a + 1;
@@ -1230,18 +1247,21 @@ __device__ __forceinline__ void pair_sources(const DevPlan &P, const WarpState &
 }
 
 // y ∈ list q of level a+1 (shared list q, or N(x) for q = -1).
-template <bool STATS>
-__device__ __forceinline__ bool pair_in(const WarpState &W, const Ctx<STATS> &c, const PairState &S, int q,
+template <int M>
+__device__ __forceinline__ bool pair_in(const WarpState &W, const Ctx<M> &c, const PairState &S, int q,
                                         uint32_t l, uint32_t y) {
-    if (q < 0) return csr_has(c.g, S.x[l], c.g.adj + S.xo[l], S.xl[l], y);
+    if (q < 0) {
+        const int32_t h = S.xhub[l];
+        return h >= 0 ? hub_has(c.g, h, y) : contains(c.g.adj + S.xo[l], S.xl[l], y);
+    }
     if (S.stab[q] >= 0) return pin_has(c.tab + S.stab[q] * c.tw, W.pmode[S.stab[q]], c.tw, y);
     if (S.shub[q] >= 0) return hub_has(c.g, S.shub[q], y);
     return contains(S.sptr[q], S.slen[q], y);
 }
 
 // v ∈ the inline tail's single list for batch candidate l.
-template <bool STATS>
-__device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<STATS> &c, const PairState &S,
+template <int M>
+__device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<M> &c, const PairState &S,
                                               uint32_t l, uint32_t v) {
     const TailDesc &D = S.ptd;
     const uint32_t k = D.kind[0];
@@ -1260,8 +1280,8 @@ __device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<STAT
 // level a+1 once per x (build_level_wcoj / explore_update + explore_level),
 // without one warp-wide set operation and one short leaf call per x.
 // Returns false on timeout.
-template <bool STATS>
-__device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t a,
+template <int M>
+__device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t a,
                                            unsigned long long &acc, uint32_t part, uint32_t parts) {
     PairState &S = *c.PS;
     const uint32_t lane = lane_id();
@@ -1278,7 +1298,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
             tail_desc(P, W, *c.L, c, lc, P.ne, S.ptd);
         }
         __syncwarp();
-        inl = S.ptd.nsrc == 1 && (!P.vlab || ((P.hoist_mask >> P.ne) & 1u));
+        inl = S.ptd.nsrc == 1 && (!labels_of<M>(P) || ((P.hoist_mask >> P.ne) & 1u));
     }
     const TailDesc &D = S.ptd;
     const uint32_t ns = S.ns, xpar = S.xpar, nex = S.nex;
@@ -1292,12 +1312,12 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
         const uint32_t idx = b0 + lane;
         bool valid = idx < n;
         const uint32_t xv = valid ? lst[idx] : 0u;
-        if (valid) valid = !rejected(P, W, a, xv);
+        if (valid) valid = !rejected(P, W, a, xv, labels_of<M>(P));
         const uint32_t bal = __ballot_sync(FULL_MASK, valid);
         const uint32_t nc = __popc(bal);
         if (valid) S.x[__popc(bal & ((1u << lane) - 1u))] = xv;
         __syncwarp();
-        if (STATS) { c.partial += nc; c.set_ops += nc; }
+        if (stats_of<M>) { c.partial += nc; c.set_ops += nc; }
         // 2. per candidate: N(x); the warp scans one source for every
         // candidate (the least cost summed over the batch: scan length ×
         // probes of the others), trimmed by level a+1's bounds
@@ -1312,6 +1332,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
             nbr(c.g, x, xp, xl);
             S.xo[lane] = (uint32_t)(xp - c.g.adj);
             S.xl[lane] = xl;
+            S.xhub[lane] = hub_slot_of(c.g, x, xl);
         }
         {
             unsigned long long allp = 0;
@@ -1333,7 +1354,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
         if (lane < nc) {
             bp = bsrc < 0 ? xp : S.sptr[bsrc];
             blen = bsrc < 0 ? xl : S.slen[bsrc];
-            if (STATS) {
+            if (stats_of<M>) {
                 unsigned long long by = 4ull * blen;
                 for (uint32_t q = 0; q < ns; ++q)
                     if ((int32_t)q != bsrc) by += probe_bytes(blen, S.slen[q], S.stab[q] >= 0 || S.shub[q] >= 0);
@@ -1374,12 +1395,11 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
                     if ((!tb.has_lo || v > tb.lo) && (!tb.has_hi || v < tb.hi) && pair_tail_has(W, c, S, lane, v))
                         --cnt;
                 }
-                S.tr[lane] = cnt;
-                if (STATS) pbytes += 4ull * (2u + D.nex) * (31u - __clz(fl + 1u));
+                S.qx[lane] = cnt;
+                if (stats_of<M>) pbytes += 4ull * (2u + D.nex) * (31u - __clz(fl + 1u));
             }
         }
-        S.bp[lane] = bp;
-        if (STATS) c.alg_bytes += warp_sum_u64(pbytes);  // all lanes, after the per-candidate branch
+        if (stats_of<M>) c.alg_bytes += warp_sum_u64(pbytes);  // all lanes, after the per-candidate branch
         uint32_t incl = blen;
 #pragma unroll
         for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -1387,6 +1407,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
             if (lane >= o) incl += v;
         }
         S.pref[lane] = incl;
+        S.bp[lane] = bp - (incl - blen);
         uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
         __syncwarp();
         uint32_t begin = 0;   // this task's part of the scan (the pair step's level is level 2)
@@ -1394,46 +1415,54 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
             begin = (uint32_t)((unsigned long long)total * part / parts);
             total = (uint32_t)((unsigned long long)total * (part + 1) / parts);
         }
-        // 3. flattened scan; survivors are appended to the pair queue
+        // y of scan element j under candidate l, and whether level a+1 keeps it
         uint32_t l = 0;
-        // (one step past the last batch's scan drains the queue: the leaf is
-        // inlined once)
-        const bool last = b0 + 32 >= n;
-        for (uint32_t j0 = begin; j0 < total || (last && qn); j0 += 32) {
-            if (j0 && (j0 & 0x1FFFu) == 0 && out_of_time(c)) { ok = false; break; }
-            const uint32_t j = j0 + lane;
-            bool keep = j < total;
-            uint32_t y = 0;
-            if (keep) {
-                while (S.pref[l] <= j) ++l;
-                const uint32_t start = l ? S.pref[l - 1] : 0u;
-                y = S.bp[l][j - start];
-                for (uint32_t q = 0; q < ns && keep; ++q)
-                    if ((int32_t)q != bsrc) keep = pair_in(W, c, S, (int)q, l, y);
-                if (keep && xpar && bsrc != -1) keep = pair_in(W, c, S, -1, l, y);
-                for (uint32_t e = 0; e < nex && keep; ++e) keep = y != S.exv[e];
-                if (keep && ex_x) keep = y != S.x[l];
-                if (P.vlab && keep) keep = __ldg(P.vlab + y) == P.lab[i];
-            }
-            if (inl) {
+        auto element = [&](uint32_t j, uint32_t &y) {
+            while (S.pref[l] <= j) ++l;
+            y = S.bp[l][j];
+            bool keep = true;
+            for (uint32_t q = 0; q < ns && keep; ++q)
+                if ((int32_t)q != bsrc) keep = pair_in(W, c, S, (int)q, l, y);
+            if (keep && xpar && bsrc != -1) keep = pair_in(W, c, S, -1, l, y);
+            for (uint32_t e = 0; e < nex && keep; ++e) keep = y != S.exv[e];
+            if (keep && ex_x) keep = y != S.x[l];
+            if (labels_of<M>(P) && keep) keep = __ldg(labels_of<M>(P) + y) == P.lab[i];
+            return keep;
+        };
+        // 3. flattened scan; an inline tail is summed on the spot ...
+        if (inl) {
+            for (uint32_t j0 = begin; j0 < total; j0 += 32) {
+                if (j0 && (j0 & 0x1FFFu) == 0 && out_of_time(c)) { ok = false; break; }
+                const uint32_t j = j0 + lane;
+                uint32_t y;
+                const bool keep = j < total && element(j, y);
                 if (keep) {
-                    uint32_t r = S.tr[l];
-                    // y itself, when the tail excludes it and it lies in x's range and list
-                    const uint32_t xl0 = S.x[l];
-                    const uint32_t tlo = (D.lo_slots & 1u) ? max(D.lo, xl0) : D.lo;
-                    const uint32_t thi = (D.hi_slots & 1u) ? min(D.hi, xl0) : D.hi;
-                    if ((D.ex_slots & 2u) && (!D.has_lo || y > tlo) && (!D.has_hi || y < thi) &&
-                        pair_tail_has(W, c, S, l, y))
-                        --r;
+                    uint32_t r = S.qx[l];
+                    if (D.ex_slots & 2u) {
+                        // y itself, when it lies in x's range and list of the tail
+                        const uint32_t xl0 = S.x[l];
+                        const uint32_t tlo = (D.lo_slots & 1u) ? max(D.lo, xl0) : D.lo;
+                        const uint32_t thi = (D.hi_slots & 1u) ? min(D.hi, xl0) : D.hi;
+                        if ((!D.has_lo || y > tlo) && (!D.has_hi || y < thi) && pair_tail_has(W, c, S, l, y)) --r;
+                    }
                     isum += r;
                 }
-                if (STATS) {
+                if (stats_of<M>) {
                     const uint32_t kb = __ballot_sync(FULL_MASK, keep);
                     c.partial += __popc(kb);
                     c.set_ops += __popc(kb);
                 }
-                continue;
             }
+            continue;
+        }
+        // ... otherwise survivors are appended to the pair queue (one step
+        // past the last batch's scan drains it: the leaf is inlined once)
+        const bool last = b0 + 32 >= n;
+        for (uint32_t j0 = begin; j0 < total || (last && qn); j0 += 32) {
+            if (j0 && (j0 & 0x1FFFu) == 0 && out_of_time(c)) { ok = false; break; }
+            const uint32_t j = j0 + lane;
+            uint32_t y = 0;
+            const bool keep = j < total && element(j, y);
             const uint32_t kb = __ballot_sync(FULL_MASK, keep);
             if (keep) {
                 const uint32_t p = qn + __popc(kb & ((1u << lane) - 1u));
@@ -1441,7 +1470,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
                 S.qy[p] = y;
             }
             qn += __popc(kb);
-            if (STATS) c.partial += __popc(kb);
+            if (stats_of<M>) c.partial += __popc(kb);
             __syncwarp();
             if (qn >= 32 || j0 >= total) {
                 const uint32_t take = min(qn, 32u);
@@ -1462,8 +1491,8 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<S
 // One root edge: DFS over levels 2..ne-2; the candidates of level ne-1 go to
 // the leaf 32 at a time.
 // Past the time budget?  (all lanes agree: lane 0 reads the clock)
-template <bool STATS>
-__device__ __forceinline__ bool out_of_time(Ctx<STATS> &c) {
+template <int M>
+__device__ __forceinline__ bool out_of_time(Ctx<M> &c) {
     if (!c.deadline) return false;
     unsigned long long now = 0;
     if (lane_id() == 0) now = globaltimer_ns();
@@ -1478,8 +1507,8 @@ __device__ __forceinline__ bool out_of_time(Ctx<STATS> &c) {
 // the leaf's passes test it with one shared-memory load instead of a bisection
 // of the trie (two triangles joined by a 4-cycle, 1,500 roots of R-MAT 2^14:
 // some 4,400 such tests per 32 candidates; 54 -> 30 ms).
-template <bool STATS>
-__device__ __forceinline__ void root_tries(const DevPlan &P, WarpState &W, Ctx<STATS> &c) {
+template <int M>
+__device__ __forceinline__ void root_tries(const DevPlan &P, WarpState &W, Ctx<M> &c) {
     for (uint32_t j = 0; j < P.ntrie; ++j) {
         const DevTrie &T = P.tries[P.trel[j]];
         uint32_t key[3];
@@ -1507,8 +1536,8 @@ __device__ __forceinline__ void root_tries(const DevPlan &P, WarpState &W, Ctx<S
 // level-2 list and equal parts of the level-3 lists below them).
 // TWO: plans with two enumerated levels come here too (count_kernel takes
 // their roots 32 at a time itself).
-template <bool STATS, bool TWO = false>
-__device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<STATS> &c, uint32_t u, uint32_t v,
+template <int M, bool TWO = false>
+__device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t u, uint32_t v,
                                        uint32_t r2b = 0u, uint32_t r2e = 0xFFFFFFFFu, uint32_t p3 = 0u,
                                        uint32_t np3 = 1u) {
     const uint32_t lane = lane_id();
@@ -1534,7 +1563,7 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
     } else if (P.hoist_mask) {
         ok = hoist_after(P, W, c, 1);
     }
-    if (!STATS && ok && P.ntrie) root_tries(P, W, c);
+    if (!stats_of<M> && ok && ntrie_of<M>(P)) root_tries(P, W, c);
     uint32_t lv = 2;
     if (ok) {
         if (explore) explore_level(P, W, c, lv);
@@ -1565,7 +1594,7 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
                 const uint32_t idx = b0 + lane;
                 bool valid = idx < n;
                 const uint32_t x = valid ? lst[idx] : 0u;
-                if (valid) valid = !rejected(P, W, lv, x);
+                if (valid) valid = !rejected(P, W, lv, x, labels_of<M>(P));
                 const uint32_t bal = __ballot_sync(FULL_MASK, valid);
                 const uint32_t nc = __popc(bal);
                 if (valid) {
@@ -1575,7 +1604,7 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
                 }
                 __syncwarp();
                 if (nc) acc += leaf_chunk(P, W, c, L0, nc);
-                if (STATS) c.partial += nc;
+                if (stats_of<M>) c.partial += nc;
             }
             if (lv == 2) break;
             --lv;
@@ -1592,9 +1621,9 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
         __syncwarp();
         if (lane == 0) W.pos[lv] = pos + 1;
         __syncwarp();
-        if (rejected(P, W, lv, x)) continue;
+        if (rejected(P, W, lv, x, labels_of<M>(P))) continue;
         set_match(c.g, W, lv, x);
-        if (STATS) c.partial += 1;
+        if (stats_of<M>) c.partial += 1;
         if (explore && !explore_update(P, W, c, lv)) continue;
         if (!explore && P.hoist_mask && !hoist_after(P, W, c, lv)) { ok = false; break; }
         ++lv;
@@ -1611,8 +1640,8 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
         }
         __syncwarp();
     }
-    if (P.pin_mask || W.hpin || W.tpin) unpin_root(P, W, c);
-    if (P.ntrie) {
+    if (P.pin_mask || W.hpin || (!(M & MODE_PLAIN) && W.tpin)) unpin_root(P, W, c);
+    if (ntrie_of<M>(P)) {
         __syncwarp();
         if (lane == 0) W.troot = 0;
         __syncwarp();
@@ -1632,9 +1661,9 @@ __host__ __device__ inline size_t warp_smem_bytes(uint32_t tw, uint32_t ntd, uin
            align128(nvs * sizeof(uint32_t)) + align128(3ull * tw * sizeof(uint32_t));
 }
 
-template <bool STATS>
+template <int M>
 __device__ __forceinline__ WarpState &setup_warp(unsigned char *smem, uint32_t wib, uint32_t tw, uint32_t tmode,
-                                                 uint32_t ntd, uint32_t cs, uint32_t nvs, Ctx<STATS> &c,
+                                                 uint32_t ntd, uint32_t cs, uint32_t nvs, Ctx<M> &c,
                                                  uint32_t ntr = 0) {
     unsigned char *base = smem + (size_t)wib * warp_smem_bytes(tw, ntd, cs, nvs, ntr);
     WarpState &W = *reinterpret_cast<WarpState *>(base);
@@ -1686,8 +1715,8 @@ __device__ __forceinline__ uint2 root_edge(const DevGraph &g, const DevPlan &P, 
 }
 
 // A root kept by the degree cap: both endpoints of degree <= root_maxdeg.
-__device__ __forceinline__ bool root_kept(const DevGraph &g, const DevPlan &P, uint2 e) {
-    if (P.vlab && (__ldg(P.vlab + e.x) != P.lab[0] || __ldg(P.vlab + e.y) != P.lab[1])) return false;
+__device__ __forceinline__ bool root_kept(const DevGraph &g, const DevPlan &P, uint2 e, const uint32_t *vlab) {
+    if (vlab && (__ldg(vlab + e.x) != P.lab[0] || __ldg(vlab + e.y) != P.lab[1])) return false;
     if (!P.root_maxdeg) return true;
     return __ldg(g.off + e.x + 1) - __ldg(g.off + e.x) <= P.root_maxdeg &&
            __ldg(g.off + e.y + 1) - __ldg(g.off + e.y) <= P.root_maxdeg;
@@ -1781,7 +1810,7 @@ __device__ __forceinline__ bool dense_counts_root(const DevPlan &P, const uint8_
 // memory per warp fit 28 resident warps (the DFS is latency-bound, so
 // resident warps set the speed)
 constexpr uint32_t COUNT_MAX_WARPS = 4;
-template <bool STATS>
+template <int M>
 __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph g, const DevPlan *__restrict__ plans, uint32_t nplans,
                                                     unsigned long long *queues, unsigned long long *counts,
                                                     uint32_t *scratch, uint32_t cap, uint32_t bufs_per_warp,
@@ -1793,7 +1822,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
     const uint32_t lane = lane_id();
     const uint32_t wib = threadIdx.x >> 5;
     const size_t gwarp = (size_t)blockIdx.x * (blockDim.x >> 5) + wib;
-    Ctx<STATS> c;
+    Ctx<M> c;
     c.g = g;
     c.buf = scratch + gwarp * (size_t)bufs_per_warp * cap;
     c.cap = cap;
@@ -1847,7 +1876,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
                 const uint2 e = root_edge(g, P, t0 + lane);
                 u = e.x;
                 v = e.y;
-                keep = root_kept(g, P, e);
+                keep = root_kept(g, P, e, labels_of<M>(P));
             }
             const uint32_t kb = __ballot_sync(FULL_MASK, keep);
             const uint32_t nk = __popc(kb);
@@ -1891,7 +1920,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
             } else {
                 if (dskip && P.dcls && dense_counts_root(P, dskip, t)) continue;
                 e = root_edge(g, P, t);
-                if (!root_kept(g, P, e)) continue;
+                if (!root_kept(g, P, e, labels_of<M>(P))) continue;
                 ++roots;
                 if (P.split_S && root_split(g, P, e, level2_bound(g, P, e)).heavy) {
                     uint32_t slot = 0;
@@ -1904,12 +1933,12 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
                 }
             }
             if (lane == 0) W.t_root = globaltimer_ns();
-            acc += run_root<STATS>(P, W, c, e.x, e.y, r2b, r2e, q3, np3);
+            acc += run_root<M>(P, W, c, e.x, e.y, r2b, r2e, q3, np3);
             if (lane == 0) atomicAdd(H.ptime + cur, globaltimer_ns() - W.t_root);
         }
     }
     if (cur < nplans && lane == 0 && acc) atomicAdd(counts + cur, acc);
-    if (STATS && lane == 0) {
+    if (stats_of<M> && lane == 0) {
         atomicAdd(&stats->set_ops, c.set_ops);
         atomicAdd(&stats->alg_bytes, c.alg_bytes);
         atomicAdd(&stats->partial, c.partial);
@@ -1962,10 +1991,10 @@ __device__ __forceinline__ void enum_put(PairState &S, const EnumOut &o, uint32_
     if (lane < qn) { S.qx[lane] = rx; S.qy[lane] = ry; }
     __syncwarp();
 }
-// Inclusive prefix of the lanes' lengths in S.pref, the scanned lists in S.bp.
+// Inclusive prefix of the lanes' lengths in S.pref, the scanned lists in S.bp
+// (less the scan index each starts at).
 __device__ __forceinline__ uint32_t enum_flatten(PairState &S, const uint32_t *bp, uint32_t blen) {
     const uint32_t lane = lane_id();
-    S.bp[lane] = bp;
     uint32_t incl = blen;
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -1973,13 +2002,14 @@ __device__ __forceinline__ uint32_t enum_flatten(PairState &S, const uint32_t *b
         if (lane >= o) incl += v;
     }
     S.pref[lane] = incl;
+    S.bp[lane] = bp - (incl - blen);
     const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
     __syncwarp();
     return total;
 }
 
 // Levels a = k-2 and k-1 under the matched prefix.
-__device__ __forceinline__ void enum_pairs(const DevPlan &P, WarpState &W, Ctx<false> &c, uint32_t a, const EnumOut &out) {
+__device__ __forceinline__ void enum_pairs(const DevPlan &P, WarpState &W, Ctx<MODE_PLAIN> &c, uint32_t a, const EnumOut &out) {
     PairState &S = *c.PS;
     const uint32_t lane = lane_id(), i = a + 1, k = P.k, n = W.cnt[a];
     const uint32_t *lst = W.list[a];
@@ -2003,6 +2033,7 @@ __device__ __forceinline__ void enum_pairs(const DevPlan &P, WarpState &W, Ctx<f
         S.x[lane] = x;
         S.xo[lane] = valid ? (uint32_t)(xp - c.g.adj) : 0u;
         S.xl[lane] = xl;
+        S.xhub[lane] = valid ? hub_slot_of(c.g, x, xl) : -1;
         // one list to scan for the batch: the least scan length x probes of the others
         int32_t bsrc = -1;
         {
@@ -2042,7 +2073,7 @@ __device__ __forceinline__ void enum_pairs(const DevPlan &P, WarpState &W, Ctx<f
             uint32_t y = 0;
             if (keep) {
                 while (S.pref[l] <= j) ++l;
-                y = S.bp[l][j - (l ? S.pref[l - 1] : 0u)];
+                y = S.bp[l][j];
                 for (uint32_t q = 0; q < ns && keep; ++q)
                     if ((int32_t)q != bsrc) keep = pair_in(W, c, S, (int)q, l, y);
                 if (keep && xpar && bsrc != -1) keep = pair_in(W, c, S, -1, l, y);
@@ -2058,7 +2089,7 @@ __device__ __forceinline__ void enum_pairs(const DevPlan &P, WarpState &W, Ctx<f
 
 // Three-vertex patterns: up to 32 roots (u, v) at once, level 2 from the
 // shorter of its lists, the other one probed.
-__device__ __forceinline__ void enum_roots(const DevPlan &P, Ctx<false> &c, bool valid, uint2 e, const EnumOut &out) {
+__device__ __forceinline__ void enum_roots(const DevPlan &P, Ctx<MODE_PLAIN> &c, bool valid, uint2 e, const EnumOut &out) {
     PairState &S = *c.PS;
     const uint32_t lane = lane_id();
     const bool p0 = P.parents[2] & 1u, p1 = P.parents[2] & 2u;
@@ -2085,7 +2116,7 @@ __device__ __forceinline__ void enum_roots(const DevPlan &P, Ctx<false> &c, bool
     LeafState &L = *c.L;
     L.cm[lane][0] = e.x;
     L.cm[lane][1] = e.y;
-    S.tr[lane] = (uint32_t)hub;
+    S.xhub[lane] = hub;
     const uint32_t total = enum_flatten(S, bp, blen);
     uint32_t l = 0, qn = 0;
     auto write = [&](unsigned long long row, uint32_t r, uint32_t y) {   // (r: the root's lane)
@@ -2100,9 +2131,9 @@ __device__ __forceinline__ void enum_roots(const DevPlan &P, Ctx<false> &c, bool
         uint32_t y = 0;
         if (keep) {
             while (S.pref[l] <= j) ++l;
-            y = S.bp[l][j - (l ? S.pref[l - 1] : 0u)];
+            y = S.bp[l][j];
             if (p0 && p1) {
-                const int32_t h = (int32_t)S.tr[l];
+                const int32_t h = S.xhub[l];
                 keep = h >= 0 ? hub_has(c.g, h, y) : contains(c.g.adj + S.xo[l], S.xl[l], y);
             }
             if ((P.check[2] & 1u) && y == L.cm[l][0]) keep = false;
@@ -2122,7 +2153,7 @@ __global__ void __launch_bounds__(256) enum_kernel(DevGraph g, const DevPlan *__
     const uint32_t wib = threadIdx.x >> 5;
     const DevPlan &P = *plan;
     const size_t gwarp = (size_t)blockIdx.x * (blockDim.x >> 5) + wib;
-    Ctx<false> c;
+    Ctx<MODE_PLAIN> c;
     c.g = g;
     c.buf = scratch + gwarp * (size_t)bufs_per_warp * cap;
     c.cap = cap;
@@ -2541,6 +2572,7 @@ struct LaunchCfg {
     uint32_t ntr = 0;                   // per-warp trie ranges (bag relations of the plans)
     size_t smem = 0, blocks = 1, scratch_bytes = 0;
     bool want_stats = false, any_split = false, use_hubs = true;
+    decltype(&count_kernel<MODE_FULL>) kern = count_kernel<MODE_FULL>;
     unsigned long long deadline = 0;
     size_t off_plans = 0, off_counts = 0, off_queue = 0, off_flags = 0, off_stats = 0, off_hcnt = 0, off_htot = 0,
            off_hids = 0, off_hpre = 0, off_ptime = 0, bytes_zeroed = 0, bytes = 0;
@@ -2681,7 +2713,12 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
     else if (o.pin_tables == 2 || !g->d_hub_bits || o.no_hub_bitmaps) { L.tmode = 2; L.tw = 512; }
     else { L.tmode = 0; L.tw = 0; }
     L.want_stats = o.collect_counters != 0;
-    for (auto &d : L.dps) d.root_maxdeg = o.root_max_degree;
+    bool plain = true;
+    for (auto &d : L.dps) {
+        d.root_maxdeg = o.root_max_degree;
+        plain &= !d.vlab && !d.ntrie;
+    }
+    L.kern = L.want_stats ? count_kernel<MODE_STATS> : plain ? count_kernel<MODE_PLAIN> : count_kernel<MODE_FULL>;
     L.use_hubs = o.no_hub_bitmaps == 0;
     // warps per block: 4 or 2, whichever keeps more warps resident per SM
     // (shared memory per warp is several KB, so smaller blocks pack better)
@@ -2693,11 +2730,9 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
             if (o.warps_per_block && wpb != std::min<uint32_t>(o.warps_per_block, COUNT_MAX_WARPS)) continue;
             const size_t smem = warp_smem_bytes(L.tw, L.ntd, L.cs, L.nvs, L.ntr) * wpb;
             int b = 0;
-            // static (plan copies) + dynamic shared memory exceed the 48 KB default: opt in
-            CUDA_TRY(cudaFuncSetAttribute(count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CUDA_TRY(cudaFuncSetAttribute(count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            if (L.want_stats) CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, count_kernel<true>, wpb * 32, smem));
-            else CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, count_kernel<false>, wpb * 32, smem));
+            // dynamic shared memory exceeds the 48 KB default: opt in
+            CUDA_TRY(cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, L.kern, wpb * 32, smem));
             if (b * (int)wpb > best_warps) { best_warps = b * (int)wpb; bps = b; L.wpb = wpb; L.smem = smem; }
         }
         if (o.warps_per_block && best_warps < 0) {
@@ -2705,8 +2740,7 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
             L.smem = warp_smem_bytes(L.tw, L.ntd, L.cs, L.nvs, L.ntr) * L.wpb;
         }
         L.threads = L.wpb * 32;
-        CUDA_TRY(cudaFuncSetAttribute(count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
-        CUDA_TRY(cudaFuncSetAttribute(count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
+        CUDA_TRY(cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
     }
     if (o.blocks_per_sm) bps = std::min<int>(bps, (int)o.blocks_per_sm);
     bps = std::max(bps, 1);
@@ -2857,14 +2891,9 @@ sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, ui
             CUDA_TRY(cudaGetLastError());
             ++launches;
         }
-        if (L.want_stats)
-            count_kernel<true><<<(unsigned)L.blocks, L.threads, L.smem, s>>>(
-                dg, dplans, L.nplans, dqueue, dcounts, scratch, L.cap, L.nbufs, L.tw, L.tmode, L.deadline, dflags,
-                dstats, phase, H, L.ntd, L.cs, L.nvs, L.ntr, dskip);
-        else
-            count_kernel<false><<<(unsigned)L.blocks, L.threads, L.smem, s>>>(
-                dg, dplans, L.nplans, dqueue, dcounts, scratch, L.cap, L.nbufs, L.tw, L.tmode, L.deadline, dflags,
-                dstats, phase, H, L.ntd, L.cs, L.nvs, L.ntr, dskip);
+        L.kern<<<(unsigned)L.blocks, L.threads, L.smem, s>>>(
+            dg, dplans, L.nplans, dqueue, dcounts, scratch, L.cap, L.nbufs, L.tw, L.tmode, L.deadline, dflags, dstats,
+            phase, H, L.ntd, L.cs, L.nvs, L.ntr, dskip);
         CUDA_TRY(cudaGetLastError());
         ++launches;
     }
@@ -3722,7 +3751,7 @@ __global__ void __launch_bounds__(256) count_kernel_noalloc(DevGraph g, const De
     const uint32_t lane = lane_id();
     const uint32_t wib = threadIdx.x >> 5;
     const size_t gwarp = (size_t)blockIdx.x * (blockDim.x >> 5) + wib;
-    Ctx<false> c;
+    Ctx<MODE_PLAIN> c;
     c.g = g;
     c.buf = lists + gwarp * (size_t)bufs_per_warp * cap;
     c.cap = cap;
@@ -3754,7 +3783,7 @@ __global__ void __launch_bounds__(256) count_kernel_noalloc(DevGraph g, const De
             const uint32_t v = g.adj[e];
             if (P.root_kind == SGE_ROOT_ASC && !(u < v)) continue;
             if (P.root_kind == SGE_ROOT_DESC && !(u > v)) continue;
-            acc += run_root<false, true>(P, W, c, u, v);
+            acc += run_root<MODE_PLAIN, true>(P, W, c, u, v);
         }
     }
     if (cur >= 0 && lane == 0 && acc) atomicAdd(counts + cur, acc * plans[cur].mult);
