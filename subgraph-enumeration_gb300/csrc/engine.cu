@@ -382,7 +382,7 @@ __device__ __forceinline__ void trim(const uint32_t *&p, uint32_t &len, const Bo
 // What a build of the counting code holds: the instrumented counters, and
 // labeled plans and bag relations.  Most launches have neither; compiled in,
 // their branches cost the pair step registers (the 12 plans of a 7,100-vertex
-// Chung-Lu graph: 30.9 ms with them, PLAINMS ms without).
+// Chung-Lu graph: 30.9 ms with them, 30.1 ms without).
 enum { MODE_FULL = 0, MODE_STATS = 1, MODE_PLAIN = 2 };
 template <int M>
 constexpr bool stats_of = (M & MODE_STATS) != 0;
@@ -1259,10 +1259,10 @@ __device__ __forceinline__ bool pair_in(const WarpState &W, const Ctx<M> &c, con
     return contains(S.sptr[q], S.slen[q], y);
 }
 
-// v ∈ the inline tail's single list for batch candidate l.
+// v ∈ the inline tail's single list for candidate x with list (xp, xl).
 template <int M>
-__device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<M> &c, const PairState &S,
-                                              uint32_t l, uint32_t v) {
+__device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<M> &c, const PairState &S, uint32_t x,
+                                              const uint32_t *xp, uint32_t xl, uint32_t v) {
     const TailDesc &D = S.ptd;
     const uint32_t k = D.kind[0];
     if (k < 3) return pin_has(c.tab + k * c.tw, W.pmode[k], c.tw, v);
@@ -1270,7 +1270,289 @@ __device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<M> &
         const int32_t hs = D.lvl[0] >= 0 ? W.hs[D.lvl[0]] : -1;
         return hs >= 0 ? hub_has(c.g, hs, v) : contains(D.ptr[0], D.len[0], v);
     }
-    return csr_has(c.g, S.x[l], c.g.adj + S.xo[l], S.xl[l], v);
+    return csr_has(c.g, x, xp, xl, v);
+}
+
+template <int M>
+__device__ __forceinline__ bool out_of_time(Ctx<M> &c);
+
+// A list as the pair step probes it: a bitmap (a pinned table or a hub's), a
+// hash table, or a sorted list.
+struct PairProbe {
+    const uint32_t *p;
+    uint32_t len, mode;   // mode 0: bitmap, 1: hash table of len words, 2: sorted list
+};
+__device__ __forceinline__ bool probe_has(const PairProbe &q, uint32_t y) {
+    if (q.mode == 0) return (q.p[y >> 5] >> (y & 31u)) & 1u;
+    if (q.mode == 1) return pin_has(q.p, 2u, q.len, y);
+    return contains(q.p, q.len, y);
+}
+template <int M>
+__device__ __forceinline__ PairProbe probe_of(const WarpState &W, const Ctx<M> &c, const uint32_t *p, uint32_t len,
+                                              int32_t tab, int32_t hub) {
+    PairProbe q{p, len, 2u};
+    if (tab >= 0) { q.p = c.tab + tab * c.tw; q.len = c.tw; q.mode = W.pmode[tab] == 1 ? 0u : 1u; }
+    else if (hub >= 0) { q.p = c.g.hub_bits + (size_t)hub * c.g.hub_words; q.mode = 0; }
+    return q;
+}
+
+// pair_inline where the shared list and T are bitmaps in shared memory and
+// neither y nor z is bounded: |N(x) ∩ S| and |N(x) ∩ S ∩ T| together, by words
+// of x's hub bitmap (coalesced, no probe per element) or, for a list of less
+// than a quarter as many elements as a bitmap has words, by its elements.
+// Some 100 instructions per x, bound by issue; house as above 4.1 -> 1.5 ms.
+template <int M>
+__device__ __forceinline__ bool pair_rows(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t a,
+                                          unsigned long long &acc) {
+    PairState &S = *c.PS;
+    const TailDesc &D = S.ptd;
+    const uint32_t lane = lane_id(), n = W.cnt[a], nex = S.nex, words = c.g.hub_words;
+    const uint32_t *lst = W.list[a], *sb = c.tab + S.stab[0] * c.tw, *tb = c.tab + D.kind[0] * c.tw;
+    const bool not_y = D.ex_slots & 2u;
+    auto bit = [](const uint32_t *b, uint32_t y) { return (b[y >> 5] >> (y & 31u)) & 1u; };
+    // |T| less the matched vertices below level a in it
+    uint32_t t0 = D.len[0];
+    for (uint32_t e = 0; e < D.nex; ++e) t0 -= bit(tb, D.exv[e]);
+    unsigned long long isum = 0;
+    for (uint32_t b0 = W.pos[a]; b0 < n; b0 += 32) {
+        if (out_of_time(c)) return false;
+        const uint32_t idx = b0 + lane;
+        const uint32_t x = idx < n ? lst[idx] : 0u;
+        const bool valid = idx < n && !rejected(P, W, a, x, labels_of<M>(P));
+        uint32_t xo = 0, xl = 0, tr = 0;
+        int32_t hx = -1;
+        if (valid) {
+            nbr_off(c.g, x, xo, xl);
+            hx = hub_slot_of(c.g, x, xl);
+            if (hx >= 0 && xl < words / 4) hx = -1;
+            tr = t0 - ((D.ex_slots & 1u) ? bit(tb, x) : 0u);
+            // the matched vertices that the scan below counts
+            for (uint32_t e = 0; e < nex; ++e) {
+                const uint32_t v = S.exv[e];
+                if (!bit(sb, v) || !csr_has(c.g, x, c.g.adj + xo, xl, v)) continue;
+                isum -= tr;
+                if (not_y) isum += bit(tb, v);
+            }
+        }
+        uint32_t todo = __ballot_sync(FULL_MASK, valid && xl != 0);
+        while (todo) {
+            const uint32_t l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int32_t h = __shfl_sync(FULL_MASK, hx, l);
+            const uint32_t t = __shfl_sync(FULL_MASK, tr, l);
+            uint32_t k = 0, kt = 0;
+            if (h >= 0) {
+                const uint32_t *row = c.g.hub_bits + (size_t)h * words;
+                for (uint32_t w0 = lane; w0 < words; w0 += 128) {
+                    uint32_t v[4];
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) v[q] = w0 + 32 * q < words ? __ldg(row + w0 + 32 * q) : 0u;
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        if (w0 + 32 * q >= words) break;
+                        const uint32_t y = v[q] & sb[w0 + 32 * q];
+                        k += __popc(y);
+                        kt += __popc(y & tb[w0 + 32 * q]);
+                    }
+                }
+            } else {
+                const uint32_t *p = c.g.adj + __shfl_sync(FULL_MASK, xo, l);
+                const uint32_t len = __shfl_sync(FULL_MASK, xl, l);
+#pragma unroll 2
+                for (uint32_t e = lane; e < len; e += 32) {
+                    const uint32_t y = p[e];
+                    if (!bit(sb, y)) continue;
+                    ++k;
+                    kt += bit(tb, y);
+                }
+            }
+            isum += (unsigned long long)k * t - (not_y ? kt : 0u);
+        }
+    }
+    acc += warp_sum_u64(isum);
+    return true;
+}
+
+// The pair step where the tail level's single list T does not depend on y and
+// level a+1 has at most two lists: Σ over x of |Y_x|·tr(x) - |Y_x ∩ T|, with
+// Y_x level a+1's candidates under x and tr(x) = |T| less the matched vertices
+// in it.  A lane per x takes everything but |Y_x| (bounds, the matched vertices
+// to leave out, |Y_x ∩ T| from the short list T); |Y_x| is then one scan of
+// the cheaper list per x with one probe per element.  The general step's scan,
+// flattened over (x, element), spends some 80 instructions on 32 elements
+// where this one needs about 12: bound by the probes' L1 and shared-memory
+// latency.  House on a 7,100-vertex Chung-Lu graph: 4.7 -> 4.1 ms this way
+// alone, 1.5 ms with pair_rows where that fits.
+template <int M>
+__device__ __forceinline__ bool pair_inline(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t a,
+                                            unsigned long long &acc) {
+    PairState &S = *c.PS;
+    const TailDesc &D = S.ptd;
+    const uint32_t lane = lane_id(), i = a + 1, n = W.cnt[a];
+    const uint32_t *lst = W.list[a];
+    const uint32_t ns = S.ns, xpar = S.xpar, nex = S.nex;
+    const bool ex_x = (P.check[i] >> a) & 1u, two = ns + xpar == 2;
+    // the shared list that is scanned or probed beside N(x), or the two shared ones
+    const uint32_t s0 = ns == 2 && S.slen[1] < S.slen[0] ? 1u : 0u;
+    PairProbe sp{nullptr, 0, 2u};
+    if (ns == 2) sp = probe_of(W, c, S.sptr[1 - s0], S.slen[1 - s0], S.stab[1 - s0], S.shub[1 - s0]);
+    else if (ns == 1) sp = probe_of(W, c, S.sptr[0], S.slen[0], S.stab[0], S.shub[0]);
+    const uint32_t *tl = D.ptr[0];
+    const bool t_is_x = D.kind[0] == 4;
+    // T lies inside level a+1's shared lists (its parents hold theirs)
+    const bool t_in_s = !labels_of<M>(P) && !t_is_x && !(P.parents[i] & ((1u << a) - 1u) & ~P.parents[P.ne]);
+    unsigned long long isum = 0;
+    for (uint32_t b0 = W.pos[a]; b0 < n; b0 += 32) {
+        if (out_of_time(c)) return false;
+        const uint32_t idx = b0 + lane;
+        const uint32_t x = idx < n ? lst[idx] : 0u;
+        const bool valid = idx < n && !rejected(P, W, a, x, labels_of<M>(P));
+        // this lane's x: the list to scan, the list to probe, tr(x) and the correction
+        const uint32_t *bp = nullptr;
+        uint32_t blen = 0, tr = 0;
+        PairProbe q = sp;
+        bool probe_x = false, scan_t = false;
+        Bounds tb{D.lo, D.hi, D.has_lo != 0, D.has_hi != 0};
+        if (valid) {
+            const uint32_t *xp;
+            uint32_t xl;
+            nbr(c.g, x, xp, xl);
+            const int32_t hx = hub_slot_of(c.g, x, xl);
+            PairProbe px{xp, xl, 2u};
+            if (hx >= 0) { px.p = c.g.hub_bits + (size_t)hx * c.g.hub_words; px.mode = 0; }
+            if (!xpar) {
+                bp = S.sptr[s0];
+                blen = S.slen[s0];
+            } else {
+                const unsigned long long cs = sp.mode < 2 ? 1u : search_cost(sp.len),
+                                         cx = hx >= 0 ? 1u : search_cost(xl);
+                if (ns == 0 || xl * (cs + 1) <= S.slen[0] * (cx + 1)) {
+                    bp = xp;
+                    blen = xl;
+                } else {
+                    bp = S.sptr[0];
+                    blen = S.slen[0];
+                    q = px;
+                    probe_x = true;
+                }
+            }
+            Bounds b{0u, 0xFFFFFFFFu, P.lower[i] != 0, P.upper[i] != 0};
+            for (uint32_t msk = P.lower[i]; msk; msk &= msk - 1) {
+                const uint32_t p = __ffs(msk) - 1;
+                b.lo = max(b.lo, p == a ? x : W.m[p]);
+            }
+            for (uint32_t msk = P.upper[i]; msk; msk &= msk - 1) {
+                const uint32_t p = __ffs(msk) - 1;
+                b.hi = min(b.hi, p == a ? x : W.m[p]);
+            }
+            trim(bp, blen, b);
+            // T within the tail's bounds, less the matched vertices in it
+            const uint32_t *tp = t_is_x ? xp : tl;
+            const uint32_t tn = t_is_x ? xl : D.len[0];
+            if (D.lo_slots & 1u) tb.lo = max(tb.lo, x);
+            if (D.hi_slots & 1u) tb.hi = min(tb.hi, x);
+            uint32_t tlen = tn;
+            trim(tp, tlen, tb);
+            tr = tlen;
+            for (uint32_t e = 0; e < D.nex + ((D.ex_slots & 1u) ? 1u : 0u); ++e) {
+                const uint32_t v = e < D.nex ? D.exv[e] : x;
+                if ((!tb.has_lo || v > tb.lo) && (!tb.has_hi || v < tb.hi) && pair_tail_has(W, c, S, x, xp, xl, v)) --tr;
+            }
+            // y ∈ Y_x before the matched vertices are left out
+            auto in_y = [&](uint32_t y) {
+                if ((b.has_lo && y <= b.lo) || (b.has_hi && y >= b.hi)) return false;
+                if (labels_of<M>(P) && __ldg(labels_of<M>(P) + y) != P.lab[i]) return false;
+                if (xpar && !probe_has(px, y)) return false;
+                if (ns && !probe_has(sp, y)) return false;
+                return ns < 2 || pair_in(W, c, S, (int)s0, lane, y);
+            };
+            auto matched = [&](uint32_t y) {
+                bool m = ex_x && y == x;
+                for (uint32_t e = 0; e < nex; ++e) m |= y == S.exv[e];
+                return m;
+            };
+            uint32_t out = 0;   // matched vertices the scan will count
+            for (uint32_t e = 0; e < nex; ++e) out += in_y(S.exv[e]) ? 1u : 0u;
+            if (ex_x) out += in_y(x) ? 1u : 0u;
+            isum -= (unsigned long long)out * tr;
+            // z = y: T is searched for it when T is the shorter list, else each y in T
+            scan_t = (D.ex_slots & 2u) && tlen > 16u && tlen > blen / 8u;
+            if ((D.ex_slots & 2u) && !scan_t) {
+                const uint32_t *zp = tp;
+                uint32_t zl = tlen, hit = 0;
+                trim(zp, zl, b);
+                if (t_in_s && xpar && px.mode == 0) {
+                    for (uint32_t e = 0; e < zl; ++e) {
+                        const uint32_t y = zp[e];
+                        hit += (px.p[y >> 5] >> (y & 31u)) & 1u;
+                    }
+                    for (uint32_t e = 0; e < nex; ++e)
+                        if (probe_has(px, S.exv[e]) && contains(zp, zl, S.exv[e])) --hit;
+                } else if (t_in_s && xpar && xl < zl) {
+                    for (uint32_t e = 0; e < xl; ++e) {
+                        const uint32_t y = xp[e];
+                        hit += !matched(y) && contains(zp, zl, y) ? 1u : 0u;
+                    }
+                } else {
+                    for (uint32_t e = 0; e < zl; ++e) hit += !matched(zp[e]) && in_y(zp[e]) ? 1u : 0u;
+                }
+                isum -= hit;
+            }
+        }
+        uint32_t todo = __ballot_sync(FULL_MASK, blen != 0 && tr != 0);
+        const uint32_t in_t = __ballot_sync(FULL_MASK, scan_t);
+        const unsigned long long addr = reinterpret_cast<unsigned long long>(bp), qaddr = reinterpret_cast<unsigned long long>(q.p);
+        while (todo) {
+            const uint32_t l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t *y_of = reinterpret_cast<const uint32_t *>(__shfl_sync(FULL_MASK, addr, l));
+            const uint32_t len = __shfl_sync(FULL_MASK, blen, l), t = __shfl_sync(FULL_MASK, tr, l);
+            PairProbe u = sp;
+            if (__shfl_sync(FULL_MASK, (uint32_t)probe_x, l)) {
+                u.p = reinterpret_cast<const uint32_t *>(__shfl_sync(FULL_MASK, qaddr, l));
+                u.len = __shfl_sync(FULL_MASK, q.len, l);
+                u.mode = __shfl_sync(FULL_MASK, q.mode, l);
+            }
+            uint32_t k = 0;
+            if ((in_t >> l) & 1u) {
+                const uint32_t xx = __shfl_sync(FULL_MASK, x, l);
+                Bounds xb{__shfl_sync(FULL_MASK, tb.lo, l), __shfl_sync(FULL_MASK, tb.hi, l), tb.has_lo, tb.has_hi};
+                const uint32_t *xp;
+                uint32_t xl, sub = 0;
+                nbr(c.g, xx, xp, xl);
+                for (uint32_t e = lane; e < len; e += 32) {
+                    const uint32_t y = y_of[e];
+                    bool ok = !labels_of<M>(P) || __ldg(labels_of<M>(P) + y) == P.lab[i];
+                    if (two && ok) ok = probe_has(u, y);
+                    k += ok;
+                    if (!ok || (xb.has_lo && y <= xb.lo) || (xb.has_hi && y >= xb.hi) || (ex_x && y == xx)) continue;
+                    for (uint32_t z = 0; z < nex; ++z) ok &= y != S.exv[z];
+                    sub += ok && pair_tail_has(W, c, S, xx, xp, xl, y);
+                }
+                isum -= sub;
+            } else if (two && u.mode == 0 && !labels_of<M>(P)) {
+                // four elements in flight per lane: a list of 128 costs one trip to L2
+                for (uint32_t e = lane; e < len; e += 128) {
+                    uint32_t y[4];
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) y[q] = e + 32 * q < len ? y_of[e + 32 * q] : 0xFFFFFFFFu;
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q)
+                        if (y[q] != 0xFFFFFFFFu) k += (u.p[y[q] >> 5] >> (y[q] & 31u)) & 1u;
+                }
+            } else {
+                for (uint32_t e = lane; e < len; e += 32) {
+                    const uint32_t y = y_of[e];
+                    bool ok = !labels_of<M>(P) || __ldg(labels_of<M>(P) + y) == P.lab[i];
+                    if (two && ok) ok = probe_has(u, y);
+                    k += ok;
+                }
+            }
+            isum += (unsigned long long)k * t;
+        }
+    }
+    acc += warp_sum_u64(isum);
+    return true;
 }
 
 // The last two enumerated levels as one step: for 32 candidates x of level
@@ -1299,6 +1581,17 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
         }
         __syncwarp();
         inl = S.ptd.nsrc == 1 && (!labels_of<M>(P) || ((P.hoist_mask >> P.ne) & 1u));
+    }
+    // (a stored list, as N(m0) ∩ N(m1), is short: a scan per x would leave most
+    // lanes idle, so those plans stay with the flattened step; an 8-edge
+    // near-5-clique on a 7,100-vertex Chung-Lu graph: 1.0 ms, 1.3 per x)
+    if (!stats_of<M> && inl && parts == 1 && P.base[i] < 0 && S.ns + S.xpar <= 2 && (S.ns == 0 || S.slen[0] >= 64u))
+    {
+        if (S.ns == 1 && S.xpar && S.stab[0] >= 0 && S.ptd.kind[0] < 3 && c.tmode == 1 && W.pmode[S.stab[0]] == 1 &&
+            W.pmode[S.ptd.kind[0]] == 1 && c.g.hub_words <= c.tw && c.g.hub_min != 0xFFFFFFFFu && !labels_of<M>(P) &&
+            !((P.lower[i] | P.upper[i]) | S.ptd.has_lo | S.ptd.has_hi) && !((P.check[i] >> a) & 1u))
+            return pair_rows(P, W, c, a, acc);
+        return pair_inline(P, W, c, a, acc);
     }
     const TailDesc &D = S.ptd;
     const uint32_t ns = S.ns, xpar = S.xpar, nex = S.nex;
@@ -1392,7 +1685,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
                 uint32_t cnt = tl;
                 for (uint32_t e = 0; e < D.nex + ((D.ex_slots & 1u) ? 1u : 0u); ++e) {
                     const uint32_t v = e < D.nex ? D.exv[e] : x;
-                    if ((!tb.has_lo || v > tb.lo) && (!tb.has_hi || v < tb.hi) && pair_tail_has(W, c, S, lane, v))
+                    if ((!tb.has_lo || v > tb.lo) && (!tb.has_hi || v < tb.hi) && pair_tail_has(W, c, S, x, xp, xl, v))
                         --cnt;
                 }
                 S.qx[lane] = cnt;
@@ -1443,7 +1736,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
                         const uint32_t xl0 = S.x[l];
                         const uint32_t tlo = (D.lo_slots & 1u) ? max(D.lo, xl0) : D.lo;
                         const uint32_t thi = (D.hi_slots & 1u) ? min(D.hi, xl0) : D.hi;
-                        if ((!D.has_lo || y > tlo) && (!D.has_hi || y < thi) && pair_tail_has(W, c, S, l, y)) --r;
+                        if ((!D.has_lo || y > tlo) && (!D.has_hi || y < thi) && pair_tail_has(W, c, S, xl0, c.g.adj + S.xo[l], S.xl[l], y)) --r;
                     }
                     isum += r;
                 }

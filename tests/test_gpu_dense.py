@@ -71,3 +71,34 @@ def test_counts_do_not_depend_on_the_id_order(sge, oracle, reverse, exploration)
         split, _, _ = eng.count(plans, heavy_threshold=32)
     want = [oracle.count_plan(g.offsets, g.nbrs, b, threads=0)[0] * b.count_multiplier for b in plans]
     assert got == want and split == want
+
+
+INLINE_PATTERNS = {
+    "house": MIRROR_PATTERNS["house"],
+    "cycle4_tail": (5, [(0, 1), (1, 2), (2, 3), (0, 3), (0, 4)]),
+    "cycle4_far_tail": (5, [(0, 1), (1, 2), (2, 3), (0, 3), (2, 4)]),
+    "cycle5": (5, [(0, 1), (1, 2), (2, 3), (3, 4), (0, 4)]),
+    "path_triangle": (5, [(0, 1), (1, 2), (2, 3), (1, 3), (0, 4)]),
+    "near5clique_8e": (5, [(0, 1), (0, 2), (0, 3), (0, 4), (1, 2), (1, 3), (1, 4), (2, 3)]),
+}
+
+
+@pytest.mark.parametrize("exploration", [False, True])
+@pytest.mark.parametrize("n,m,maxd", [(300, 2500, 120), (3000, 9000, 900), (33_000, 40_000, 1500)])
+def test_inline_tails(sge, oracle, n, m, maxd, exploration):
+    """Tails that do not depend on the last enumerated level: by words of the
+    hub bitmaps (small n), by a scan per candidate (no shared-memory tables
+    beyond 32,768 vertices), hub and list candidates side by side."""
+    g = sge.gen_chung_lu(n, m, 2.1, maxd, seed=n)
+    plans = [sge.plan(sge.PatternGraph.from_edges(k, e), g, iep=iep, exploration=exploration)
+             for k, e in INLINE_PATTERNS.values() for iep in (False, True)]
+    opts = dict(root_stride=7, root_offset=2) if n > 300 else {}
+    with sge.Engine(g) as eng:
+        got, _, _ = eng.count(plans, **opts)
+        split, _, _ = eng.count(plans, heavy_threshold=32, **opts)
+        lists, _, _ = eng.count(plans, hub_bitmaps=False, **opts)
+    raw = b"".join(b.to_bytes() for b in plans)
+    want, _ = oracle.count_plans(g.offsets, g.nbrs, raw, len(plans), stride=opts.get("root_stride", 1),
+                                 offset=opts.get("root_offset", 0))
+    want = [w * b.count_multiplier for w, b in zip(want, plans)]
+    assert got == want and split == want and lists == want
