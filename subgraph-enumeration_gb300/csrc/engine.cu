@@ -976,6 +976,44 @@ __device__ __forceinline__ void tail_desc(const DevPlan &P, const WarpState &W, 
     D.nex = (uint8_t)nex;
 }
 
+// A list as the scans below probe it: a bitmap (a pinned table or a hub's), a
+// hash table, or a sorted list.
+struct PairProbe {
+    const uint32_t *p;
+    uint32_t len, mode;   // mode 0: bitmap, 1: hash table of len words, 2: sorted list
+};
+__device__ __forceinline__ bool probe_has(const PairProbe &q, uint32_t y) {
+    if (q.mode == 0) return (q.p[y >> 5] >> (y & 31u)) & 1u;
+    if (q.mode == 1) return pin_has(q.p, 2u, q.len, y);
+    return contains(q.p, q.len, y);
+}
+// How many elements of the sorted list [p, p + len) the probed list holds (and
+// carry the label, for labeled plans), a share per lane: four elements in
+// flight per lane, so a list of 128 costs one trip to L2, and some 12
+// instructions per 32 elements.
+__device__ __forceinline__ uint32_t scan_count(const uint32_t *p, uint32_t len, const PairProbe &q, bool probed,
+                                               const uint32_t *vlab, uint32_t lab) {
+    uint32_t k = 0;
+    if (probed && q.mode == 0 && !vlab) {
+        for (uint32_t e = lane_id(); e < len; e += 128) {
+            uint32_t y[4];
+#pragma unroll
+            for (uint32_t r = 0; r < 4; ++r) y[r] = e + 32 * r < len ? p[e + 32 * r] : 0xFFFFFFFFu;
+#pragma unroll
+            for (uint32_t r = 0; r < 4; ++r)
+                if (y[r] != 0xFFFFFFFFu) k += (q.p[y[r] >> 5] >> (y[r] & 31u)) & 1u;
+        }
+    } else {
+        for (uint32_t e = lane_id(); e < len; e += 32) {
+            const uint32_t y = p[e];
+            bool ok = !vlab || __ldg(vlab + y) == lab;
+            if (probed && ok) ok = probe_has(q, y);
+            k += ok;
+        }
+    }
+    return k;
+}
+
 template <int M>
 __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t L0,
                                          uint32_t ncand) {
@@ -1082,6 +1120,65 @@ __device__ __forceinline__ unsigned long long leaf_chunk(const DevPlan &P, WarpS
         const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
         __syncwarp();
         const uint32_t ns = D.nsrc;
+        // 2a. one tail list (SINGLE, CHOOSE) from two lists and enough to scan
+        // per candidate: one scan each (scan_count) instead of the flattened
+        // one, which spends some 80 instructions on 32 elements.  Over every
+        // root of R-MAT 2^18: triangle 1.03 -> 0.47 ms, diamond 3.4 -> 1.0
+        // ms, K4 23 -> 17 ms, 4-cycle 309 -> 83 ms; below some 48 elements
+        // per candidate most of a scan's lanes would be idle.
+        if (!stats_of<M> && P.tail_mode != SGE_TAIL_IEP && ns == 2 && total >= 48u * ncand) {
+            const uint32_t oq = 1u - bq, kind = D.kind[oq];
+            PairProbe pr{D.ptr[oq], D.len[oq], 2u};
+            if (kind < 3) {
+                pr.p = c.tab + kind * c.tw;
+                pr.len = c.tw;
+                pr.mode = W.pmode[kind] == 1 ? 0u : 1u;
+            } else if (kind == 3) {
+                const int32_t h = D.lvl[oq] >= 0 ? W.hs[D.lvl[oq]] : -1;
+                if (h >= 0) { pr.p = c.g.hub_bits + (size_t)h * c.g.hub_words; pr.mode = 0; }
+            } else if (lane < ncand) {
+                const uint2 r = L.ol[kind - 4][lane];
+                pr.p += r.x;
+                pr.len = r.y;
+                const int32_t h = kind < 6 ? hub_slot_of(c.g, L.cm[lane][kind - 4], r.y) : -1;
+                if (h >= 0) { pr.p = c.g.hub_bits + (size_t)h * c.g.hub_words; pr.mode = 0; }
+            }
+            // the excluded values that the scan will count
+            uint32_t out = 0, found = 0;
+            if (lane < ncand && blen) {
+                const Bounds b = td_bounds(D, L, lane);
+                auto counted = [&](uint32_t v) {
+                    return (!b.has_lo || v > b.lo) && (!b.has_hi || v < b.hi) && contains(bp, blen, v) &&
+                           probe_has(pr, v) && (!labels_of<M>(P) || __ldg(labels_of<M>(P) + v) == D.lab);
+                };
+                for (uint32_t e = 0; e < D.nex; ++e) out += counted(D.exv[e]) ? 1u : 0u;
+                if (D.ex_slots & 1u) out += counted(L.cm[lane][0]) ? 1u : 0u;
+                if (D.ex_slots & 2u) out += counted(L.cm[lane][1]) ? 1u : 0u;
+            }
+            const unsigned long long addr = reinterpret_cast<unsigned long long>(bp), qaddr = reinterpret_cast<unsigned long long>(pr.p);
+            uint32_t todo = __ballot_sync(FULL_MASK, blen != 0);
+            for (uint32_t turn = 0; todo; ++turn) {
+                if ((turn & 7u) == 7u && out_of_time(c)) break;
+                const uint32_t l = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const uint32_t *sp = reinterpret_cast<const uint32_t *>(__shfl_sync(FULL_MASK, addr, l));
+                PairProbe u;
+                u.p = reinterpret_cast<const uint32_t *>(__shfl_sync(FULL_MASK, qaddr, l));
+                u.len = __shfl_sync(FULL_MASK, pr.len, l);
+                u.mode = __shfl_sync(FULL_MASK, pr.mode, l);
+                const uint32_t k = scan_count(sp, __shfl_sync(FULL_MASK, blen, l), u, true, labels_of<M>(P), D.lab);
+                if (P.tail_mode == SGE_TAIL_SINGLE) {
+                    single += k;
+                } else {
+                    const uint32_t sum = __reduce_add_sync(FULL_MASK, k);
+                    if (lane == l) found = sum;
+                }
+            }
+            if (P.tail_mode == SGE_TAIL_SINGLE) single -= out;
+            else c.cnt[lane * c.cs + 1] = found - out;
+            __syncwarp();
+            continue;
+        }
         const uint32_t nu = (P.tail_mode == SGE_TAIL_IEP) ? (T - 1 - t) : 0u;
         // 2. flattened scan: element j belongs to the candidate l with
         // pref[l-1] <= j < pref[l].  A lane's elements of one candidate are
@@ -1276,17 +1373,6 @@ __device__ __forceinline__ bool pair_tail_has(const WarpState &W, const Ctx<M> &
 template <int M>
 __device__ __forceinline__ bool out_of_time(Ctx<M> &c);
 
-// A list as the pair step probes it: a bitmap (a pinned table or a hub's), a
-// hash table, or a sorted list.
-struct PairProbe {
-    const uint32_t *p;
-    uint32_t len, mode;   // mode 0: bitmap, 1: hash table of len words, 2: sorted list
-};
-__device__ __forceinline__ bool probe_has(const PairProbe &q, uint32_t y) {
-    if (q.mode == 0) return (q.p[y >> 5] >> (y & 31u)) & 1u;
-    if (q.mode == 1) return pin_has(q.p, 2u, q.len, y);
-    return contains(q.p, q.len, y);
-}
 template <int M>
 __device__ __forceinline__ PairProbe probe_of(const WarpState &W, const Ctx<M> &c, const uint32_t *p, uint32_t len,
                                               int32_t tab, int32_t hub) {
@@ -1530,23 +1616,8 @@ __device__ __forceinline__ bool pair_inline(const DevPlan &P, WarpState &W, Ctx<
                     sub += ok && pair_tail_has(W, c, S, xx, xp, xl, y);
                 }
                 isum -= sub;
-            } else if (two && u.mode == 0 && !labels_of<M>(P)) {
-                // four elements in flight per lane: a list of 128 costs one trip to L2
-                for (uint32_t e = lane; e < len; e += 128) {
-                    uint32_t y[4];
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) y[q] = e + 32 * q < len ? y_of[e + 32 * q] : 0xFFFFFFFFu;
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        if (y[q] != 0xFFFFFFFFu) k += (u.p[y[q] >> 5] >> (y[q] & 31u)) & 1u;
-                }
             } else {
-                for (uint32_t e = lane; e < len; e += 32) {
-                    const uint32_t y = y_of[e];
-                    bool ok = !labels_of<M>(P) || __ldg(labels_of<M>(P) + y) == P.lab[i];
-                    if (two && ok) ok = probe_has(u, y);
-                    k += ok;
-                }
+                k = scan_count(y_of, len, u, two, labels_of<M>(P), P.lab[i]);
             }
             isum += (unsigned long long)k * t;
         }
