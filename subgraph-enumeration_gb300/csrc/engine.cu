@@ -2985,7 +2985,7 @@ void mirror_plan(DevPlan &d) {
 // their buffer.  The instrumented kernel (its counters are defined on lists)
 // and runs with a caller's list capacity (which lists may overflow) keep to
 // the lists.
-void prepare_dense(const sge_graph *g, const sge_count_opts &o, size_t free_b, LaunchCfg &L) {
+void prepare_dense(const sge_graph *g, const sge_count_opts &o, LaunchCfg &L) {
     if (L.want_stats || o.max_level_capacity || g->max_deg < 2) return;
     L.drows_both = 15u;
     for (uint32_t i = 0; i < L.nplans; ++i) {
@@ -3012,6 +3012,13 @@ void prepare_dense(const sge_graph *g, const sge_count_opts &o, size_t free_b, L
     for (uint32_t c = 0; c < 4; ++c)
         if ((L.dneed >> c) & 1u)
             units += dense_units((uint32_t)std::min<unsigned long long>(DENSE_WORDS, (c == DENSE_UNION ? 2ull * deg : deg) / 32 + 3));
+    size_t free_b = 0, tot_b = 0;
+    if (cudaMemGetInfo(&free_b, &tot_b) != cudaSuccess) {
+        cudaGetLastError();
+        drop_dense(L);
+        return;
+    }
+    free_b += g->dense_bytes;   // (the held buffer is part of what is there)
     L.darena_units = std::min({L.dedges * units, DENSE_ARENA_MAX / 16, (unsigned long long)free_b / 16 / 16});
     L.drec_cap = (uint32_t)std::min<unsigned long long>(L.dedges, DENSE_REC_MAX);
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -3111,10 +3118,11 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
     L.cap = o.max_level_capacity ? o.max_level_capacity : std::max<uint32_t>(g->max_deg, 1);
     L.cap = (L.cap + 31) & ~31u;
     // fit the scratch into a quarter of free memory by trimming resident blocks
+    // (what is held already needs no look at the device's memory)
     size_t free_b = 0, tot_b = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_b, &tot_b));
     const size_t per_block = (size_t)L.wpb * L.nbufs * L.cap * sizeof(uint32_t);
     size_t blocks = (size_t)g->num_sms * bps;
+    if (blocks * per_block > scratch_held) CUDA_TRY(cudaMemGetInfo(&free_b, &tot_b));
     const size_t budget = free_b / 4 + scratch_held;
     while (blocks > (size_t)g->num_sms && blocks * per_block > budget) blocks -= g->num_sms;
     if (blocks * per_block > budget) blocks = std::max<size_t>(1, budget / std::max<size_t>(per_block, 1));
@@ -3182,9 +3190,18 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
             L.any_split = true;
         }
         max_tasks = std::max(max_tasks, d.ntasks);
-        if (d.ne == 2) d.chunk = 32;  // one leaf over 32 root edges
+        // two enumerated levels: one leaf over up to 32 root edges, fewer
+        // where that would leave warps without any (915 roots: 25 -> 13 us;
+        // the instrumented kernel's bytes are defined on full leaves)
+        if (d.ne == 2) d.chunk = L.want_stats ? 32u : (uint32_t)std::min<unsigned long long>(32, std::max<unsigned long long>(1, d.ntasks / (2 * warps)));
         else if (o.chunk) d.chunk = o.chunk;
         else d.chunk = (uint32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(8, d.ntasks / (warps * 64 + 1)));
+    }
+    if (!L.any_split) {   // no more blocks than there are root chunks
+        unsigned long long chunks = 0;
+        for (const DevPlan &d : L.dps) chunks += (d.ntasks + d.chunk - 1) / d.chunk;
+        L.blocks = (size_t)std::min<unsigned long long>(L.blocks, std::max<unsigned long long>(1, (chunks + L.wpb - 1) / L.wpb));
+        L.scratch_bytes = L.blocks * per_block;
     }
     L.heavy_cap = L.any_split ? (uint32_t)std::min<unsigned long long>(max_tasks, 1ull << 18) : 1u;
     // buffer: plans | counts | per-plan queues | flags | stats | heavy counts | heavy task totals |
@@ -3202,15 +3219,15 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
     L.off_hpre = L.off_hids + (((size_t)L.heavy_cap * nplans * 4 + 255) & ~(size_t)255);
     L.bytes = L.off_hpre + (((size_t)L.heavy_cap * nplans * 8 + 255) & ~(size_t)255);
     if (o.time_budget_s > 0) L.deadline = std::max<unsigned long long>(1, (unsigned long long)(o.time_budget_s * 1e9));
-    prepare_dense(g, o, free_b, L);
+    prepare_dense(g, o, L);
     return SGE_OK;
 }
 
 // Stream-ordered: clear the counters, run phase 0 and (when roots may be
 // split) phase 1.  Capturable (no host synchronisation).
 sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, uint32_t *scratch, unsigned char *dense,
-                          cudaStream_t s, uint32_t &launches) {
-    CUDA_TRY(cudaMemsetAsync(B + L.off_counts, 0, L.bytes_zeroed - L.off_counts, s));
+                          bool cleared, cudaStream_t s, uint32_t &launches) {
+    if (!cleared) CUDA_TRY(cudaMemsetAsync(B + L.off_counts, 0, L.bytes_zeroed - L.off_counts, s));
     DevGraph dg = dev_graph(g, L.use_hubs);
     const DevPlan *dplans = reinterpret_cast<const DevPlan *>(B + L.off_plans);
     unsigned long long *dcounts = reinterpret_cast<unsigned long long *>(B + L.off_counts);
@@ -3829,21 +3846,28 @@ static sge_status count_impl(sge_graph *g, const sge_plan *const *plans, uint32_
     if (!L.dpo.empty())
         CUDA_TRY(cudaMemcpyAsync(g->d_dense + L.off_dpo, L.dpo.data(), sizeof(DensePO) * L.dpo.size(),
                                  cudaMemcpyHostToDevice, g->stream));
-    CUDA_TRY(cudaMemcpyAsync(B + L.off_plans, L.dps.data(), sizeof(DevPlan) * nplans, cudaMemcpyHostToDevice, g->stream));
+    // plans and cleared counters go up in one copy (a few plans), counters,
+    // flags and statistics come back in one
+    std::vector<unsigned char> up(sizeof(DevPlan) * nplans <= (16u << 10) ? L.bytes_zeroed : sizeof(DevPlan) * nplans, 0);
+    memcpy(up.data(), L.dps.data(), sizeof(DevPlan) * nplans);
+    CUDA_TRY(cudaMemcpyAsync(B + L.off_plans, up.data(), up.size(), cudaMemcpyHostToDevice, g->stream));
     CUDA_TRY(cudaEventRecord(g->ev0, g->stream));
     uint32_t launches = 0;
-    if ((st = enqueue_launch(g, L, B, g->d_scratch, g->d_dense, g->stream, launches)) != SGE_OK) return st;
+    if ((st = enqueue_launch(g, L, B, g->d_scratch, g->d_dense, up.size() == L.bytes_zeroed, g->stream, launches)) != SGE_OK)
+        return st;
     g->launched = true;
     CUDA_TRY(cudaEventRecord(g->ev1, g->stream));
     std::vector<unsigned long long> hc(nplans);
     uint32_t hflags = 0;
     DevStats hs{};
-    CUDA_TRY(cudaMemcpyAsync(hc.data(), B + L.off_counts, 8 * nplans, cudaMemcpyDeviceToHost, g->stream));
-    CUDA_TRY(cudaMemcpyAsync(&hflags, B + L.off_flags, 4, cudaMemcpyDeviceToHost, g->stream));
-    if (L.want_stats) CUDA_TRY(cudaMemcpyAsync(&hs, B + L.off_stats, sizeof hs, cudaMemcpyDeviceToHost, g->stream));
+    std::vector<unsigned char> down(L.off_stats + sizeof hs - L.off_counts);
+    CUDA_TRY(cudaMemcpyAsync(down.data(), B + L.off_counts, down.size(), cudaMemcpyDeviceToHost, g->stream));
     std::vector<unsigned long long> hp(busy_ms ? nplans : 0);
     if (busy_ms) CUDA_TRY(cudaMemcpyAsync(hp.data(), B + L.off_ptime, 8 * (size_t)nplans, cudaMemcpyDeviceToHost, g->stream));
     CUDA_TRY(cudaStreamSynchronize(g->stream));
+    memcpy(hc.data(), down.data(), 8 * (size_t)nplans);
+    memcpy(&hflags, down.data() + (L.off_flags - L.off_counts), 4);
+    if (L.want_stats) memcpy(&hs, down.data() + (L.off_stats - L.off_counts), sizeof hs);
     for (uint32_t i = 0; busy_ms && i < nplans; ++i) busy_ms[i] = (double)hp[i] / 1e6;
     float ms = 0;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);
@@ -3962,7 +3986,7 @@ sge_status sge_batch_create(sge_graph *g, const sge_plan *const *plans, uint32_t
     // capture: clear counters, both launch phases, read back counts/flags/stats
     if ((e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return bail(fail(SGE_CUDA_ERROR, "stream capture: %s", cudaGetErrorString(e)));
-    st = enqueue_launch(g, b->L, b->d_buf, b->d_scratch, b->d_dense, g->stream, b->launches);
+    st = enqueue_launch(g, b->L, b->d_buf, b->d_scratch, b->d_dense, false, g->stream, b->launches);
     if (st == SGE_OK) {
         cudaMemcpyAsync(b->h_res, b->d_buf + b->L.off_counts, 8 * (size_t)nplans, cudaMemcpyDeviceToHost, g->stream);
         cudaMemcpyAsync(b->h_res + 8 * (size_t)nplans, b->d_buf + b->L.off_flags, 4, cudaMemcpyDeviceToHost, g->stream);
