@@ -649,7 +649,8 @@ __global__ void __launch_bounds__(128) dense_count_kernel(const DevPlan *__restr
         --r;
         const DenseRec &R = D.recs[D.order[r]];
         const uint32_t ps = dense_parts_log2(D, R), per = dense_tasks(R.n2, ps);
-        const uint32_t local = (uint32_t)(t - D.pre[r] * D.npo), task = local % per;
+        const unsigned long long local = t - D.pre[r] * D.npo;
+        const uint32_t task = (uint32_t)(local % per);
         const DensePO po = D.po[local / per];
         if (R.off[po.cls] == DENSE_NONE) continue;   // counted by the list path
         const uint32_t c0 = ps ? task >> ps : task * DENSE_CAND, c1 = ps ? c0 + 1 : min(R.n2, c0 + DENSE_CAND);

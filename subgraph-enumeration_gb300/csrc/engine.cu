@@ -2965,10 +2965,10 @@ void drop_dense(LaunchCfg &L) {
 // sides).  K4 over every root of R-MAT 2^18: 287 -> 36 ms, triangles 2.05 ->
 // 1.10 ms; house on a 7,100-vertex Chung-Lu graph: 8.1 -> 4.9 ms.  A sample
 // or a shard counts the instances its roots represent, so it keeps the plan's
-// own order, as do the instrumented kernel and wrapping CHOOSE leaves, whose
-// results are defined by the lists.
+// own order, as do the instrumented kernel, wrapping CHOOSE leaves and runs
+// with a caller's list capacity, whose results are defined by the lists.
 bool mirror_ok(const DevPlan &d, const sge_count_opts &o) {
-    return o.root_stride <= 1 && !o.root_max_degree && !o.collect_counters && !(d.tail_mode == SGE_TAIL_CHOOSE && d.T > 2);
+    return o.root_stride <= 1 && !o.root_max_degree && !o.collect_counters && !o.max_level_capacity && !(d.tail_mode == SGE_TAIL_CHOOSE && d.T > 2);
 }
 void mirror_plan(DevPlan &d) {
     uint32_t lo = 0, up = 0;

@@ -474,30 +474,6 @@ sge_status sge::device_sort_keys(unsigned long long *&keys, unsigned long long *
 }
 
 namespace {
-// Packs, sorts and unpacks rows whose columns fit one key.
-template <class K>
-sge_status sort_packed(uint32_t *d_tuples, uint64_t n, uint32_t arity, const Widths &w, uint32_t bits) {
-    K *a = nullptr, *b = nullptr;
-    uint32_t *hist = nullptr;
-    const uint64_t ntiles = (n + SORT_TILE<K> - 1) / SORT_TILE<K>;
-    cudaError_t e;
-    if ((e = cudaMalloc(&a, n * sizeof(K))) != cudaSuccess || (e = cudaMalloc(&b, n * sizeof(K))) != cudaSuccess ||
-        (e = cudaMalloc(&hist, (256 * ntiles + 256) * 4)) != cudaSuccess) {
-        cudaFree(a);
-        cudaFree(b);
-        return fail(SGE_OOM, "sge_sort_tuples: %s", cudaGetErrorString(e));
-    }
-    pack_kernel<K><<<grid_for(n), 256>>>(d_tuples, n, arity, w, a);
-    const sge_status st = sort_keys(a, b, n, 0u, bits, hist, 0);
-    if (st == SGE_OK) unpack_kernel<K><<<grid_for(n), 256>>>(a, n, arity, w, d_tuples);
-    e = cudaDeviceSynchronize();
-    cudaFree(a);
-    cudaFree(b);
-    cudaFree(hist);
-    if (st != SGE_OK) return st;
-    if (e != cudaSuccess) return fail(SGE_CUDA_ERROR, "sge_sort_tuples: %s", cudaGetErrorString(e));
-    return SGE_OK;
-}
 // Wider rows: one stable sort of (column value, row) keys per column, last column first.
 sge_status sort_wide(uint32_t *d_tuples, uint64_t n, uint32_t arity, const Widths &w) {
     Key64 *a = nullptr, *b = nullptr;
@@ -506,8 +482,7 @@ sge_status sort_wide(uint32_t *d_tuples, uint64_t n, uint32_t arity, const Width
     auto cleanup = [&]() { cudaFree(a); cudaFree(b); cudaFree(hist); cudaFree(rows); };
     cudaError_t e;
     if ((e = cudaMalloc(&a, n * 8)) != cudaSuccess || (e = cudaMalloc(&b, n * 8)) != cudaSuccess ||
-        (e = cudaMalloc(&hist, (256 * ntiles + 256) * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&rows, n * arity * 4ull)) != cudaSuccess) {
+        (e = cudaMalloc(&hist, (256 * ntiles + 256) * 4)) != cudaSuccess) {
         cleanup();
         return fail(SGE_OOM, "sge_sort_tuples: %s", cudaGetErrorString(e));
     }
@@ -523,12 +498,44 @@ sge_status sort_wide(uint32_t *d_tuples, uint64_t n, uint32_t arity, const Width
             return st;
         }
     }
+    cudaFree(b);   // (the rows' copy takes its place)
+    b = nullptr;
+    if ((e = cudaMalloc(&rows, n * arity * 4ull)) != cudaSuccess) {
+        cleanup();
+        return fail(SGE_OOM, "sge_sort_tuples: %s", cudaGetErrorString(e));
+    }
     gather_rows<<<grid_for(n), 256>>>(d_tuples, a, rows, n, arity);
     e = cudaMemcpy(d_tuples, rows, n * arity * 4ull, cudaMemcpyDeviceToDevice);
     cudaError_t e2 = cudaDeviceSynchronize();
     cleanup();
     if (e != cudaSuccess || e2 != cudaSuccess)
         return fail(SGE_CUDA_ERROR, "sge_sort_tuples: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
+    return SGE_OK;
+}
+// Packs, sorts and unpacks rows whose columns fit one key.
+template <class K>
+sge_status sort_packed(uint32_t *d_tuples, uint64_t n, uint32_t arity, const Widths &w, uint32_t bits) {
+    K *a = nullptr, *b = nullptr;
+    uint32_t *hist = nullptr;
+    const uint64_t ntiles = (n + SORT_TILE<K> - 1) / SORT_TILE<K>;
+    cudaError_t e;
+    if ((e = cudaMalloc(&a, n * sizeof(K))) != cudaSuccess || (e = cudaMalloc(&b, n * sizeof(K))) != cudaSuccess ||
+        (e = cudaMalloc(&hist, (256 * ntiles + 256) * 4)) != cudaSuccess) {
+        cudaFree(a);
+        cudaFree(b);
+        cudaGetLastError();
+        if (arity > 1) return sort_wide(d_tuples, n, arity, w);   // (needs less at once)
+        return fail(SGE_OOM, "sge_sort_tuples: %s", cudaGetErrorString(e));
+    }
+    pack_kernel<K><<<grid_for(n), 256>>>(d_tuples, n, arity, w, a);
+    const sge_status st = sort_keys(a, b, n, 0u, bits, hist, 0);
+    if (st == SGE_OK) unpack_kernel<K><<<grid_for(n), 256>>>(a, n, arity, w, d_tuples);
+    e = cudaDeviceSynchronize();
+    cudaFree(a);
+    cudaFree(b);
+    cudaFree(hist);
+    if (st != SGE_OK) return st;
+    if (e != cudaSuccess) return fail(SGE_CUDA_ERROR, "sge_sort_tuples: %s", cudaGetErrorString(e));
     return SGE_OK;
 }
 }  // namespace
