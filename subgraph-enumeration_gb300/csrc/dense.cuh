@@ -28,7 +28,7 @@
 constexpr uint32_t DENSE_MAX_U = 2048;   // vertices of a universe (padded segments): 64 words a row, two per lane
 constexpr uint32_t DENSE_WORDS = DENSE_MAX_U / 32;
 constexpr uint32_t DENSE_MAX_K = 8;      // levels the running masks in shared memory are sized for
-constexpr uint32_t DENSE_MAX_T = 3;      // inclusion–exclusion tail levels (counters per lane in shared memory)
+constexpr uint32_t DENSE_MAX_T = 3;      // inclusion–exclusion tail levels (2^T counters per lane)
 constexpr uint32_t DENSE_ROWS = 256;     // rows per build item
 constexpr uint32_t DENSE_MIN_N2 = 8, DENSE_MIN_DEG = 64, DENSE_MIN_WORDS = 3;   // see dense_worth
 constexpr int DENSE_SPLIT_LOG2 = 9;      // a level-2 candidate is split once |U|^2 n2 passes 2^19
@@ -406,19 +406,27 @@ __global__ void __launch_bounds__(256) dense_prefix_kernel(DenseBuf D) {
     if (threadIdx.x == 0) *reinterpret_cast<unsigned long long *>(D.hdr + 6) = run;
 }
 
-// Per-warp shared memory of the dense count.
+// Per-warp shared memory of the dense count; `run` has as many slots as the
+// launch's longest plan uses (dense_slots), which decides the resident warps:
+// 24 per SM with all 20 slots and counters per lane beside them, 32 for
+// seven-vertex plans with the counters in registers (78 such plans on 976 root
+// edges of R-MAT 2^22: the launch sequence 35.8 -> 33.5 ms).
 struct alignas(16) DenseWarp {
-    // run[s]: candidates of level i after matching level d (word w of lane w % 32),
-    // for d = 1..ne-2 and i = d+1..k-1; slot s = dense_slot(d, i)
-    uint32_t run[20][DENSE_WORDS];
-    uint32_t S[32][1u << DENSE_MAX_T];
     uint16_t ylist[DENSE_MAX_U / 2];
     uint16_t par[DENSE_MAX_K], lo[DENSE_MAX_K], up[DENSE_MAX_K];   // level i in entry i - 1
+    // run[s]: candidates of level i after matching level d (word w of lane w % 32),
+    // for d = 1..ne-2 and i = d+1..k-1; slot s = dense_slot(d, i)
+    uint32_t run[1][DENSE_WORDS];
 };
 // Slots for k = DENSE_MAX_K: six levels after the root, five after level 2, ...
-__device__ __forceinline__ uint32_t dense_slot(uint32_t d, uint32_t i) {
+__host__ __device__ constexpr uint32_t dense_slot(uint32_t d, uint32_t i) {
     const uint32_t r = d - 1;                        // rows d' < d hold 6, 5, 4, ... slots
     return r * (2u * (DENSE_MAX_K - 2u) - r + 1u) / 2u + (i - d - 1u);
+}
+// Slots a k-vertex plan uses: the prefix ends at level ne-2 <= k-3.
+__host__ __device__ constexpr uint32_t dense_slots(uint32_t k) { return dense_slot(k - 3, k - 1) + 1u; }
+__host__ __device__ constexpr size_t dense_warp_bytes(uint32_t slots) {
+    return sizeof(DenseWarp) + (slots - 1u) * DENSE_WORDS * sizeof(uint32_t);
 }
 
 // Word of a segment: its ranks from `c` on (t = c - the word's first rank).
@@ -607,11 +615,14 @@ __device__ __forceinline__ void dense_leaf(const DevPlan &P, DenseWarp &S, const
             if (P.tail_mode == SGE_TAIL_CHOOSE) {
                 acc += choose_leaf(cnt[1], P.T, P.choose_wrap, flags);
             } else {
-#pragma unroll
-                for (uint32_t A = 1; A < (1u << DENSE_MAX_T); ++A) S.S[lane][A] = cnt[A];
                 for (uint32_t q = 0; q < P.nparts; ++q) {
                     unsigned long long term = (unsigned long long)(long long)P.part_coef[q];
-                    for (uint32_t bk = 0; bk < P.part_nblocks[q]; ++bk) term *= S.S[lane][P.part_block[q][bk]];
+                    for (uint32_t bk = 0; bk < P.part_nblocks[q]; ++bk) {
+                        uint32_t v = 0;   // cnt[part_block], without an indexed array
+#pragma unroll
+                        for (uint32_t A = 1; A < (1u << DENSE_MAX_T); ++A) v = P.part_block[q][bk] == A ? cnt[A] : v;
+                        term *= v;
+                    }
                     acc += term;
                 }
             }
@@ -621,12 +632,13 @@ __device__ __forceinline__ void dense_leaf(const DevPlan &P, DenseWarp &S, const
 }
 
 // Counts every task, a warp at a time.
-__global__ void __launch_bounds__(128) dense_count_kernel(const DevPlan *__restrict__ plans, DenseBuf D,
-                                                          unsigned long long *counts, unsigned long long *ptime,
-                                                          unsigned long long deadline_ns, uint32_t *flags) {
+__global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__restrict__ plans, DenseBuf D,
+                                                             unsigned long long *counts, unsigned long long *ptime,
+                                                             unsigned long long deadline_ns, uint32_t *flags,
+                                                             uint32_t slots) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t lane = lane_id();
-    DenseWarp &S = reinterpret_cast<DenseWarp *>(smem_raw)[threadIdx.x >> 5];
+    DenseWarp &S = *reinterpret_cast<DenseWarp *>(smem_raw + (threadIdx.x >> 5) * dense_warp_bytes(slots));
     Ctx<false> c;
     c.flags = flags;
     c.deadline = deadline_ns;

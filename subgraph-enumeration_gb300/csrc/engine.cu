@@ -2943,7 +2943,7 @@ struct LaunchCfg {
     // dense roots (dense.cuh): the plans' universe classes and the layout of their buffer
     // (header | edge classes | records | order | prefix | (plan, orientation) table | rows)
     std::vector<DensePO> dpo;           // empty: every root is counted on lists
-    uint32_t dneed = 0, drows_both = 0, drec_cap = 0, dmaxdeg = 0;
+    uint32_t dslots = 1, dneed = 0, drows_both = 0, drec_cap = 0, dmaxdeg = 0;
     unsigned long long dedges = 0, darena_units = 0, droot_offset = 0, droot_stride = 1;
     size_t dense_blocks = 0, off_dskip = 256, off_drecs = 0, off_dorder = 0, off_dpre = 0, off_dpo = 0, off_darena = 0, dense_bytes = 0;
 };
@@ -3029,8 +3029,10 @@ void prepare_dense(const sge_graph *g, const sge_count_opts &o, LaunchCfg &L) {
     L.off_darena = up(L.off_dpo + sizeof(DensePO) * L.dpo.size());
     L.dense_bytes = L.off_darena + 16 * (size_t)L.darena_units;
     int b = 0;
-    const size_t smem = 4 * sizeof(DenseWarp);
-    if (cudaFuncSetAttribute(dense_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    for (const DensePO &po : L.dpo) L.dslots = std::max(L.dslots, dense_slots(L.dps[po.plan].k));
+    const size_t smem = 4 * dense_warp_bytes(L.dslots);
+    if (cudaFuncSetAttribute(dense_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(4 * dense_warp_bytes(dense_slots(DENSE_MAX_K)))) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, dense_count_kernel, 128, smem) != cudaSuccess || b < 1) {
         cudaGetLastError();
         drop_dense(L);
@@ -3260,8 +3262,8 @@ sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, ui
         dense_select_kernel<<<sel, 256, 0, s>>>(dg, L.droot_offset, L.droot_stride, L.dedges, L.dmaxdeg, D, dflags);
         dense_build_kernel<<<8u * g->num_sms, 256, 0, s>>>(dg, D);
         dense_prefix_kernel<<<1, 256, 0, s>>>(D);
-        dense_count_kernel<<<(unsigned)L.dense_blocks, 128, 4 * sizeof(DenseWarp), s>>>(dplans, D, dcounts, H.ptime,
-                                                                                       L.deadline, dflags);
+        dense_count_kernel<<<(unsigned)L.dense_blocks, 128, 4 * dense_warp_bytes(L.dslots), s>>>(
+            dplans, D, dcounts, H.ptime, L.deadline, dflags, L.dslots);
         CUDA_TRY(cudaGetLastError());
         launches += 4;
     }
