@@ -3181,9 +3181,16 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // half of a warp's share 30, at a 50th 16.5 ms).  A tail counted
         // inline costs a 30th per element, and the finer tasks' set-up more
         // than they level (house, 7,100-vertex Chung-Lu graph: 4.9 -> 5.7 ms).
-        if (!thr && !L.want_stats && d.ne == 4 && d.pair && !d.pair_direct && (d.parents[3] & 3u)) {
+        // A bag plan without a pair step has the same long level-3 lists: the
+        // 6-cycle with two chords on 16,384 roots of R-MAT 2^16 took 3,880 ms
+        // by level 2, 667 with W at a 50th, 533 at a 500th, 509 at a 2,000th
+        // (the two triangles: 1,013, 860 and 868; on R-MAT 2^14 17.9, 18.2 and
+        // 21.0).  On adjacency lists such a level is cut by intersections and
+        // ends far below its bound: 78 seven-vertex plans on 3,300 roots of
+        // R-MAT 2^22 15.3 -> 21.5 ms, K5 less an edge 1.7 -> 11.9.
+        if (!thr && !L.want_stats && d.ne == 4 && (d.pair ? !d.pair_direct : d.ntrie != 0) && (d.parents[3] & 3u)) {
             d.split_par3 = d.parents[3] & 3u;
-            d.split_W = (uint32_t)std::min(1e9, std::max(1024.0, share * mean_deg / 50.0));
+            d.split_W = (uint32_t)std::min(1e9, std::max(1024.0, share * mean_deg / 500.0));
         }
         if (d.ne >= 3 && (g->max_deg > split_H || d.split_W)) {
             d.split_S = split_S;
