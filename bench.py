@@ -471,9 +471,9 @@ def run_rmat22(args):
             launches += s["gpu_launches"]
             counts = c
     batch.close()
-    # untimed: algorithmic bytes of one step (instrumented kernel) and the
-    # same step without hub bitmaps
-    _, _, sst = eng.count(plans, stats=True, pin_tables=tuned.pin_tables, tuning=tuned.plans, **shard)
+    # untimed: the bytes that counting every root on lists would take (the
+    # instrumented kernel) and the same step without hub bitmaps
+    _, _, sst = eng.count(plans, stats=True, **shard)
     _, _, snh = eng.count(plans, hub_bitmaps=False, **shard)
     if dist:
         tc = torch.tensor([x % (1 << 63) for x in counts], dtype=torch.int64, device=f"cuda:{device}")
@@ -501,8 +501,8 @@ def run_rmat22(args):
     h2d = 4 * (info["num_vertices"] + 1) + 4 * info["num_directed_edges"] + len(plans[0].to_bytes()) * len(plans)
     d2h = 8 * len(plans) + 4
     peak, peak_kind = peaks()
-    achieved = sst["alg_bytes"] / avg_s / 1e9
     traffic = profile_traffic("count_kernel_rmat22-sample.md")  # DRAM bytes of one step, measured by ncu
+    achieved = traffic / avg_s / 1e9 if traffic else None
     line = {
         "metric": METRIC, "value": value, "unit": "embeddings/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": sum_k / len(kernel_ms), "higher_is_better": True,
@@ -526,17 +526,19 @@ def run_rmat22(args):
         "speedup_wall": pw / lw, "speedup_kernel": pk / lk,
         "kernel_ms_without_hub_bitmaps": snh["kernel_ms"],
         "total_count": total,
-        "roofline": {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_kind": peak_kind, "traffic": traffic,
+        "roofline": {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                     "frac": achieved / peak if traffic else None, "peak_kind": peak_kind, "traffic": traffic,
                      "dram_gbs": traffic / avg_s / 1e9 if traffic else None,
                      "dram_frac": traffic / avg_s / 1e9 / peak if traffic else None,
                      "alg_bytes_per_launch": sst["alg_bytes"],
-                     "note": "one step = the batched launch sequence (phase 0, task numbering, phase 1); "
-                             "algorithmic bytes = 4 B per scanned element + per probed list 4 B per probe through "
-                             "a hub bitmap or pinned table, else the list as a merge consumes it (+8 B offsets), "
-                             "summed by the instrumented kernel; traffic = ncu DRAM read+write of the same step "
-                             "(profiles/count_kernel_rmat22-sample.md). The working set stays in L1/L2, so the DFS "
-                             "is bound by dependent-load latency, not HBM bandwidth"},
+                     "note": "one step = the batched launch sequence (bit rows of the dense roots: select, build, "
+                             "prefix, count; the other roots on lists: phase 0, task numbering, phase 1); achieved = "
+                             "traffic = ncu DRAM read+write of the same step (profiles/count_kernel_rmat22-sample.md) "
+                             "over the step's time. alg_bytes_per_launch is what the same counts take on lists, summed "
+                             "by the instrumented kernel (4 B per scanned element + per probed list 4 B per probe "
+                             "through a hub bitmap or pinned table, else the list as a merge consumes it, + 8 B "
+                             "offsets): the bit rows replace most of it. Rows and running masks stay in L1/L2 and "
+                             "shared memory, so the step is bound by instruction issue and dependent loads, not HBM"},
         "e2e": {"value": e2e_value, "unit": "embeddings/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": statistics.median(e2e_ms)},
         "gpu_launches": launches,

@@ -23,6 +23,7 @@ import sge
 
 # candidate per-plan settings: (heavy threshold, level-3 parts, binary search only)
 CANDIDATES = [(0, 0, 0), (64, 0, 0), (256, 0, 0), (256, 32, 0), (256, 0, 1)]
+CLEAR = 0.9   # a setting is taken over the automatic one below this fraction of its time
 
 
 @dataclass
@@ -42,7 +43,9 @@ def tune(engine: "sge.Engine", plans, sample: dict, sub: int = 4) -> Tuning:
     opts["root_stride"] = sample.get("root_stride", 1) * sub
     spent, runs = 0.0, 0
     ref = None
-    # launch level: shared-memory tables or more resident warps
+    # launch level: shared-memory tables or more resident warps.  Another
+    # setting than the automatic one (0) has to be faster by more than runs
+    # differ
     best_pin, best_ms = 0, None
     for pin in (0, 1, 2):
         c, _, st = engine.count(plans, pin_tables=pin, **opts)
@@ -50,10 +53,13 @@ def tune(engine: "sge.Engine", plans, sample: dict, sub: int = 4) -> Tuning:
         runs += 1
         ref = ref if ref is not None else c
         assert c == ref, "counts changed with the shared-memory tables"
-        if best_ms is None or st["kernel_ms"] < best_ms:
+        if best_ms is None or st["kernel_ms"] < CLEAR * best_ms:
             best_pin, best_ms = pin, st["kernel_ms"]
     # per plan: every candidate setting once for the whole batch; each plan
-    # keeps the setting under which its own roots took the least warp time
+    # keeps the setting under which its own roots took the least warp time,
+    # the automatic one unless another is clearly below it (most roots of a
+    # plan may be counted on bit rows, which no setting changes: its settings
+    # then differ by noise, and the finer ones only add tasks)
     busy = []
     for thr, p3, nohub in CANDIDATES:
         tun = [sge.PlanTuning(thr, p3, nohub) for _ in plans]
@@ -62,6 +68,9 @@ def tune(engine: "sge.Engine", plans, sample: dict, sub: int = 4) -> Tuning:
         runs += 1
         assert c == ref, "counts changed with the plan tuning"
         busy.append(st["plan_busy_ms"])
-    choice = [min(range(len(CANDIDATES)), key=lambda k: busy[k][i]) for i in range(len(plans))]
+    choice = []
+    for i in range(len(plans)):
+        k = min(range(len(CANDIDATES)), key=lambda k: busy[k][i])
+        choice.append(k if busy[k][i] < CLEAR * busy[0][i] else 0)
     return Tuning(pin_tables=best_pin, plans=[sge.PlanTuning(*CANDIDATES[k]) for k in choice], choice=choice,
                   tuning_ms=spent, runs=runs)
