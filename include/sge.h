@@ -177,10 +177,13 @@ typedef struct sge_count_opts {
     uint64_t root_offset;       /* (root-range sharding across ranks, or sampled runs) */
     uint32_t collect_counters;  /* 1: run the instrumented kernel (set_ops, alg_bytes, partial matches) */
     uint32_t heavy_threshold;   /* 0 = auto (a quarter of a warp's share of the launch's level-2
-                                   candidates, at least 32); otherwise roots whose level-2 list may
-                                   exceed it are deferred to a second launch that splits each into tasks
-                                   of one level-2 candidate and a part of its level-3 list (or, where
-                                   level 3 is not enumerated, of up to 128 level-2 candidates) */
+                                   candidates, at least 32; less where a root's work grows with the
+                                   square of that list, and by the bounds of levels 2 and 3 together
+                                   where level 3 is scanned once per candidate); otherwise roots whose
+                                   level-2 list may exceed it are deferred to a second launch that
+                                   splits each into tasks of one level-2 candidate and a part of its
+                                   level-3 list (or, where level 3 is not enumerated, of 8 to 128 level-2
+                                   candidates).  Roots counted on bit rows are split by their own rule */
     uint32_t no_hub_bitmaps;    /* 1: probe every adjacency list by binary search, ignoring the graph's
                                    hub bitmaps (for comparison runs); 0 = use them */
     uint32_t root_max_degree;   /* 0 = every sampled root; d > 0: only roots whose two endpoints both have
@@ -388,16 +391,18 @@ sge_status sge_plan_destroy(sge_plan *p);
 typedef struct sge_plan_tuning {
     uint32_t heavy_threshold;   /* 0 = automatic; roots whose level-2 bound exceeds it are split */
     uint32_t level3_parts;      /* 0 = automatic; parts of each level-3 list per split task (1 = none) */
-    uint32_t no_hub_bitmaps;    /* 1: this plan probes adjacency lists by binary search only */
+    uint32_t no_hub_bitmaps;    /* 1: this plan probes adjacency lists by binary search only (its roots
+                                   that are counted on bit rows probe no list) */
 } sge_plan_tuning;
 sge_status sge_plan_set_tuning(sge_plan *p, const sge_plan_tuning *t);
 /* Labeled matching.  sge_graph_set_labels uploads one label per data vertex
  * (n values; NULL removes them); sge_plan_set_labels attaches k pattern
  * labels (pattern vertex order; NULL detaches) to a plan planned with the
  * same labels (blob.labeled).  A labeled plan then matches pattern vertex u
- * only to data vertices of label labels[u]: the root edge's ends and every
- * enumerated candidate are checked, and tail levels are counted by a scan
- * that checks labels (not by range size).  WCOJ plans only; bag relations,
+ * only to data vertices of label labels[u]: the root edge's ends, every
+ * enumerated candidate and the candidates of the tail levels are checked
+ * (a tail list that is filtered by label when it is stored is counted by
+ * range size as an unlabeled one is).  WCOJ plans only; bag relations,
  * sge_enumerate, sge_count_host and sge_count_noalloc take unlabeled plans. */
 sge_status sge_graph_set_labels(sge_graph *g, const uint32_t *labels);
 sge_status sge_plan_set_labels(sge_plan *p, const uint32_t *labels);

@@ -20,7 +20,9 @@
 //     (relation/relation.cpp:290-338), choosec (utils.cpp:80-94) and the
 //     inclusion–exclusion of numUniqueCombine (utils.cpp:290-350);
 //   - exploration style (-i) keeps running candidate lists per later level,
-//     updated as soon as a parent is matched (join.cpp:266-307).
+//     updated as soon as a parent is matched (join.cpp:266-307);
+//   - roots whose later levels all lie in their neighbourhood are counted on
+//     bit rows over it instead of lists (dense.cuh).
 // The DFS is latency-bound, so the per-warp state is kept small enough for 28
 // resident warps per SM.  Counts are exact uint64 (wrapping like the
 // reference's size_t).
