@@ -406,17 +406,19 @@ __global__ void __launch_bounds__(256) dense_prefix_kernel(DenseBuf D) {
     if (threadIdx.x == 0) *reinterpret_cast<unsigned long long *>(D.hdr + 6) = run;
 }
 
-// Per-warp shared memory of the dense count; `run` has as many slots as the
+// Per-warp shared memory of the dense count, with as many running rows as the
 // launch's longest plan uses (dense_slots), which decides the resident warps:
 // 24 per SM with all 20 slots and counters per lane beside them, 32 for
 // seven-vertex plans with the counters in registers (78 such plans on 976 root
 // edges of R-MAT 2^22: the launch sequence 35.8 -> 33.5 ms).
 struct alignas(16) DenseWarp {
     uint16_t ylist[DENSE_MAX_U / 2];
-    uint16_t par[DENSE_MAX_K], lo[DENSE_MAX_K], up[DENSE_MAX_K];   // level i in entry i - 1
-    // run[s]: candidates of level i after matching level d (word w of lane w % 32),
-    // for d = 1..ne-2 and i = d+1..k-1; slot s = dense_slot(d, i)
-    uint32_t run[1][DENSE_WORDS];
+    uint32_t lev[DENSE_MAX_K];   // level i in entry i - 1: parents | lower << 8 | upper << 16
+    // Behind the struct, slot s = dense_slot(d, i): candidates of level i after
+    // matching level d (word w of lane w % 32), for d = 1..ne-2 and i = d+1..k-1.
+    __device__ __forceinline__ uint32_t *run(uint32_t s) {
+        return reinterpret_cast<uint32_t *>(this + 1) + s * DENSE_WORDS;
+    }
 };
 // Slots for k = DENSE_MAX_K: six levels after the root, five after level 2, ...
 __host__ __device__ constexpr uint32_t dense_slot(uint32_t d, uint32_t i) {
@@ -426,11 +428,11 @@ __host__ __device__ constexpr uint32_t dense_slot(uint32_t d, uint32_t i) {
 // Slots a k-vertex plan uses: the prefix ends at level ne-2 <= k-3.
 __host__ __device__ constexpr uint32_t dense_slots(uint32_t k) { return dense_slot(k - 3, k - 1) + 1u; }
 __host__ __device__ constexpr size_t dense_warp_bytes(uint32_t slots) {
-    return sizeof(DenseWarp) + (slots - 1u) * DENSE_WORDS * sizeof(uint32_t);
+    return sizeof(DenseWarp) + slots * DENSE_WORDS * sizeof(uint32_t);
 }
 
 // Word of a segment: its ranks from `c` on (t = c - the word's first rank).
-__device__ __forceinline__ uint32_t dense_from(int t) { return t <= 0 ? 0xFFFFFFFFu : t >= 32 ? 0u : 0xFFFFFFFFu << t; }
+__device__ __forceinline__ uint32_t dense_from(int t) { return __funnelshift_lc(0u, 0xFFFFFFFFu, (uint32_t)max(t, 0)); }
 
 // A lane's view of word w: its segment and the rank of its first position.
 struct DenseLane {
@@ -443,12 +445,23 @@ __device__ __forceinline__ DenseLane dense_lane(const DenseShape &s, uint32_t w)
     l.first = (int)((w - (l.seg == 0 ? 0u : l.seg == 1 ? s.w1 : s.w2)) * 32u);
     return l;
 }
+// Elements of the lane's segment with an id <= that of the vertex whose ranks
+// are r, from the word's first on.
+__device__ __forceinline__ int dense_rank(const DenseLane &l, uint2 r) {
+    return (int)(l.seg == 0 ? r.x & 0xFFFFu : l.seg == 1 ? r.x >> 16 : r.y & 0xFFFFu) - l.first;
+}
 // Positions of the word with an id above / below that of the vertex whose
 // ranks are r (uint2 of DenseView::rank).
 __device__ __forceinline__ void dense_sides(const DenseLane &l, uint2 r, uint32_t &above, uint32_t &below) {
-    const int c = (int)(l.seg == 0 ? r.x & 0xFFFFu : l.seg == 1 ? r.x >> 16 : r.y & 0xFFFFu) - l.first;
+    const int c = dense_rank(l, r);
     above = dense_from(c);
     below = ~dense_from(c - ((r.y >> 16) == l.seg ? 1 : 0));
+}
+
+// What a level's bounds against the vertex leave of the word (f: the level's
+// entry of DenseWarp::lev, shifted by that vertex's level).
+__device__ __forceinline__ uint32_t dense_bound(uint32_t f, uint32_t above, uint32_t below) {
+    return (f & 0x100u) ? above : (f & 0x10000u) ? below : above | below;
 }
 
 // Matches level d at position p: running masks of every later level.
@@ -456,7 +469,7 @@ __device__ __forceinline__ void dense_match(DenseWarp &S, const DenseView &V, ui
     const uint32_t lane = lane_id();
     const uint32_t *r = V.rows + (size_t)p * V.s.pitch;
     const uint2 rk = __ldg(V.rank + p);
-    const bool row = (S.par[DENSE_MAX_K - 1] >> d) & 1u;
+    const bool row = (S.lev[DENSE_MAX_K - 1] >> d) & 1u;
 #pragma unroll
     for (uint32_t h = 0; h < 2; ++h) {
         const uint32_t w = lane + 32 * h;
@@ -465,12 +478,11 @@ __device__ __forceinline__ void dense_match(DenseWarp &S, const DenseView &V, ui
         uint32_t above, below;
         dense_sides(dense_lane(V.s, w), rk, above, below);
         for (uint32_t i = d + 1; i < k; ++i) {
-            uint32_t m = S.run[dense_slot(d - 1, i)][w];
-            if ((S.par[i - 1] >> d) & 1u) m &= rw;
-            if ((S.lo[i - 1] >> d) & 1u) m &= above;
-            else if ((S.up[i - 1] >> d) & 1u) m &= below;
-            else m &= above | below;
-            S.run[dense_slot(d, i)][w] = m;
+            uint32_t m = S.run(dense_slot(d - 1, i))[w];
+            const uint32_t f = S.lev[i - 1] >> d;
+            m &= (f & 1u) ? rw : 0xFFFFFFFFu;
+            m &= dense_bound(f, above, below);
+            S.run(dense_slot(d, i))[w] = m;
         }
     }
     __syncwarp();
@@ -521,14 +533,15 @@ __device__ __forceinline__ uint32_t dense_list(uint16_t *out, uint32_t x, uint32
 __device__ __forceinline__ void dense_leaf(const DevPlan &P, DenseWarp &S, const DenseView &V, uint32_t d,
                                            unsigned long long &acc, uint32_t *flags) {
     const uint32_t lane = lane_id(), y = d + 1, ne = y + 1, k = P.k;
-    const uint32_t *ym = S.run[dense_slot(d, y)];
+    const uint32_t *ym = S.run(dense_slot(d, y));
     // words the tail can have: the first segment when every tail level holds both root ends
     bool both = true;
-    for (uint32_t i = ne; i < k; ++i) both &= (S.par[i - 1] & 3u) == 3u;
+    for (uint32_t i = ne; i < k; ++i) both &= (S.lev[i - 1] & 3u) == 3u;
     const uint32_t zw = both ? V.s.w1 : V.s.w3;
     if (P.tail_mode == SGE_TAIL_SINGLE) {
-        const uint32_t *zm = S.run[dense_slot(d, ne)];
-        const bool par = (S.par[ne - 1] >> y) & 1u, lo = (S.lo[ne - 1] >> y) & 1u, up = (S.up[ne - 1] >> y) & 1u;
+        const uint32_t *zm = S.run(dense_slot(d, ne));
+        const uint32_t f = S.lev[ne - 1] >> y;
+        const bool par = f & 1u, lo = f & 0x100u, up = f & 0x10000u;
         if (!par && !lo && !up) {
             // the tail does not depend on y: |Y|·|Z| pairs less those with z = y
             uint32_t ny = 0, nz = 0, nyz = 0;
@@ -549,32 +562,35 @@ __device__ __forceinline__ void dense_leaf(const DevPlan &P, DenseWarp &S, const
         const uint32_t quads = (zw + 3u) / 4u, rq = V.s.pitch / 4u;
         const uint32_t lp = quads <= 1 ? 1u : 1u << (32 - __clz(quads - 1));
         const uint32_t ql = lane & (lp - 1), grp = lane / lp, step = 32 / lp;
-        uint4 z = make_uint4(0, 0, 0, 0);
-        if (ql < quads) z = *reinterpret_cast<const uint4 *>(zm + 4 * ql);
+        uint32_t z[4] = {0, 0, 0, 0};
+        DenseLane l[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            if (ql < quads) z[q] = zm[4 * ql + q];
+            l[q] = dense_lane(V.s, 4 * ql + q);
+        }
         const uint4 *rows = reinterpret_cast<const uint4 *>(V.rows);
+        const uint32_t flip = up ? 0xFFFFFFFFu : 0u;   // below = not from y on
         uint32_t sum = 0;
         for (uint32_t h = 0; h * 32 < V.s.pitch; ++h) {
             const uint32_t w = lane + 32 * h;
             const uint32_t n = dense_list(S.ylist, w < V.s.pitch ? ym[w] : 0u, w * 32);
             for (uint32_t b = grp; b < n; b += step) {
                 const uint32_t p = S.ylist[b];
-                uint4 m = z;
+                uint32_t m[4] = {z[0], z[1], z[2], z[3]};
                 if (par) {
                     uint4 r = make_uint4(0, 0, 0, 0);
                     if (ql < quads) r = __ldg(rows + (size_t)p * rq + ql);
-                    m.x &= r.x; m.y &= r.y; m.z &= r.z; m.w &= r.w;
+                    m[0] &= r.x; m[1] &= r.y; m[2] &= r.z; m[3] &= r.w;
                 }
                 if (lo || up) {
                     const uint2 rk = __ldg(V.rank + p);
-                    uint32_t *mw = &m.x;
+                    const uint32_t own = up ? rk.y >> 16 : 3u;   // y itself is not below y
 #pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) {
-                        uint32_t above, below;
-                        dense_sides(dense_lane(V.s, 4 * ql + q), rk, above, below);
-                        mw[q] &= lo ? above : below;
-                    }
+                    for (uint32_t q = 0; q < 4; ++q)
+                        m[q] &= dense_from(dense_rank(l[q], rk) - (own == l[q].seg ? 1 : 0)) ^ flip;
                 }
-                sum += __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+                sum += __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
             }
             __syncwarp();
         }
@@ -584,6 +600,13 @@ __device__ __forceinline__ void dense_leaf(const DevPlan &P, DenseWarp &S, const
     // CHOOSE / inclusion–exclusion: a lane per y counts the sizes S[A] of the
     // intersections of the tail levels A, then takes the plan's sum over them
     const uint32_t T = P.tail_mode == SGE_TAIL_CHOOSE ? 1u : P.T;
+    uint32_t f[DENSE_MAX_T];
+    const uint32_t *tm[DENSE_MAX_T];
+#pragma unroll
+    for (uint32_t t = 0; t < DENSE_MAX_T; ++t) {
+        f[t] = t < T ? S.lev[ne + t - 1] >> y : 0u;
+        tm[t] = S.run(dense_slot(d, ne + (t < T ? t : 0u)));
+    }
     for (uint32_t h = 0; h * 32 < V.s.pitch; ++h) {
         const uint32_t w = lane + 32 * h;
         const uint32_t n = dense_list(S.ylist, w < V.s.pitch ? ym[w] : 0u, w * 32);
@@ -593,20 +616,12 @@ __device__ __forceinline__ void dense_leaf(const DevPlan &P, DenseWarp &S, const
             const uint2 rk = __ldg(V.rank + p);
             uint32_t cnt[1u << DENSE_MAX_T] = {};
             for (uint32_t q = 0; q < zw; ++q) {
-                uint32_t above, below, z[DENSE_MAX_T] = {0, 0, 0};
+                uint32_t above, below, z[DENSE_MAX_T];
                 dense_sides(dense_lane(V.s, q), rk, above, below);
                 const uint32_t rw = __ldg(r + q);
 #pragma unroll
-                for (uint32_t t = 0; t < DENSE_MAX_T; ++t) {
-                    if (t >= T) break;
-                    const uint32_t i = ne + t;
-                    uint32_t m = S.run[dense_slot(d, i)][q];
-                    if ((S.par[i - 1] >> y) & 1u) m &= rw;
-                    if ((S.lo[i - 1] >> y) & 1u) m &= above;
-                    else if ((S.up[i - 1] >> y) & 1u) m &= below;
-                    else m &= above | below;
-                    z[t] = m;
-                }
+                for (uint32_t t = 0; t < DENSE_MAX_T; ++t)
+                    z[t] = t < T ? tm[t][q] & ((f[t] & 1u) ? rw : 0xFFFFFFFFu) & dense_bound(f[t], above, below) : 0u;
 #pragma unroll
                 for (uint32_t A = 1; A < (1u << DENSE_MAX_T); ++A)
                     cnt[A] += __popc(((A & 1u) ? z[0] : 0xFFFFFFFFu) & ((A & 2u) ? z[1] : 0xFFFFFFFFu) &
@@ -674,34 +689,33 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
         __syncwarp();
         if (lane < DENSE_MAX_K - 1) {
             const bool on = lane + 1 < k;
-            S.par[lane] = on ? P.parents[lane + 1] : 0;
-            S.lo[lane] = on ? P.lower[lane + 1] : 0;
-            S.up[lane] = on ? P.upper[lane + 1] : 0;
+            S.lev[lane] = on ? (P.parents[lane + 1] & 0xFFu) | (P.lower[lane + 1] & 0xFFu) << 8 |
+                                   (P.upper[lane + 1] & 0xFFu) << 16
+                             : 0u;
         }
         if (lane == 0) {
             uint32_t any = 0;
             for (uint32_t i = 2; i < k; ++i) any |= P.parents[i];
-            S.par[DENSE_MAX_K - 1] = (uint16_t)any;
+            S.lev[DENSE_MAX_K - 1] = any;
         }
         __syncwarp();
         {   // candidates given the root: segments and the bounds against m0, m1
-            const DenseHead hd = *V.head;
-            auto ranks = [](const uint16_t *n) { return make_uint2(n[0] | (uint32_t)n[1] << 16, n[2] | (uint32_t)n[3] << 16); };
-            const uint2 ru = ranks(hd.ucnt), rv = ranks(hd.vcnt);
+            const uint4 hd = *reinterpret_cast<const uint4 *>(V.head);
+            const uint2 ru = make_uint2(hd.x, hd.y), rv = make_uint2(hd.z, hd.w);
             for (uint32_t w = lane; w < V.s.pitch; w += 32) {
                 const DenseLane l = dense_lane(V.s, w);
-                const uint32_t valid = w < V.s.w3 ? ~dense_from((int)V.s.n[l.seg] - l.first) : 0u;
+                const uint32_t valid = w < V.s.w3 ? ~dense_from((int)(l.seg == 0 ? V.s.n[0] : l.seg == 1 ? V.s.n[1] : V.s.n[2]) - l.first) : 0u;
                 const uint32_t xu = l.seg != 2 ? valid : 0u, xv = l.seg != 1 ? valid : 0u;
                 const uint32_t x0 = po.swap ? xv : xu, x1 = po.swap ? xu : xv;
                 uint32_t gt0, lt0, gt1, lt1;
                 dense_sides(l, po.swap ? rv : ru, gt0, lt0);
                 dense_sides(l, po.swap ? ru : rv, gt1, lt1);
                 for (uint32_t i = 2; i < k; ++i) {
-                    const uint32_t pr = S.par[i - 1], lo = S.lo[i - 1], up = S.up[i - 1];
+                    const uint32_t pr = S.lev[i - 1], lo = pr >> 8, up = pr >> 16;
                     uint32_t m = ((pr & 1u) ? x0 : 0xFFFFFFFFu) & ((pr & 2u) ? x1 : 0xFFFFFFFFu);
                     m &= (lo & 1u) ? gt0 : (up & 1u) ? lt0 : (gt0 | lt0);
                     m &= (lo & 2u) ? gt1 : (up & 2u) ? lt1 : (gt1 | lt1);
-                    S.run[dense_slot(1, i)][w] = m;
+                    S.run(dense_slot(1, i))[w] = m;
                 }
             }
         }
@@ -711,14 +725,14 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
         if (ps) {
             pat = 1u << (task & ((1u << ps) - 1u));
             for (uint32_t o = 1u << ps; o < 32; o <<= 1) pat |= pat << o;
-            uint32_t *l3 = S.run[dense_slot(1, 3)];
+            uint32_t *l3 = S.run(dense_slot(1, 3));
             for (uint32_t w = lane; w < V.s.pitch; w += 32) l3[w] &= pat;
             __syncwarp();
         }
         unsigned long long acc = 0;
         bool ok = true;
         for (uint32_t p2 = c0; p2 < c1 && ok; ++p2) {   // (common neighbours are the first positions)
-            if (!((S.run[dense_slot(1, 2)][p2 >> 5] >> (p2 & 31u)) & 1u)) continue;
+            if (!((S.run(dense_slot(1, 2))[p2 >> 5] >> (p2 & 31u)) & 1u)) continue;
             dense_match(S, V, k, 2, p2);
             if (ne == 4) {
                 dense_leaf(P, S, V, 2, acc, flags);
@@ -726,7 +740,7 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
             }
             uint32_t lv = 3;
             while (true) {
-                const uint32_t p = dense_pop(S.run[dense_slot(lv - 1, lv)], V.s.pitch);
+                const uint32_t p = dense_pop(S.run(dense_slot(lv - 1, lv)), V.s.pitch);
                 if (p == DENSE_NONE) {
                     if (--lv < 3) break;
                     continue;
