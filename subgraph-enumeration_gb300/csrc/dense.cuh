@@ -19,8 +19,8 @@
 // Bound by instruction issue and L1 latency of the warp's depth-first steps;
 // the rows of a root (at most 0.5 MB) stay in L1/L2.  Kernel time, lists ->
 // rows: 78 seven-vertex patterns (16-19 edges) on 488 root edges of R-MAT 2^22
-// 1,010 -> 21 ms; 16 six-vertex patterns on 976 root edges of R-MAT 2^20
-// 20.7 -> 2.5 ms; K5 over every root of R-MAT 2^14 172 -> 87 ms.
+// 1,010 -> 17 ms; 16 six-vertex patterns on 976 root edges of R-MAT 2^20
+// 20.7 -> 2.0 ms; K5 over every root of R-MAT 2^14 172 -> 87 ms.
 //
 // Included by engine.cu inside its anonymous namespace.
 #pragma once
@@ -410,7 +410,8 @@ __global__ void __launch_bounds__(256) dense_prefix_kernel(DenseBuf D) {
 // launch's longest plan uses (dense_slots), which decides the resident warps:
 // 24 per SM with all 20 slots and counters per lane beside them, 32 for
 // seven-vertex plans with the counters in registers (78 such plans on 976 root
-// edges of R-MAT 2^22: the launch sequence 35.8 -> 33.5 ms).
+// edges of R-MAT 2^22: the launch sequence 35.8 -> 33.5 ms; then a level's masks
+// as one word and no local arrays in the loops, 32.3 ms).
 struct alignas(16) DenseWarp {
     uint16_t ylist[DENSE_MAX_U / 2];
     uint32_t lev[DENSE_MAX_K];   // level i in entry i - 1: parents | lower << 8 | upper << 16
