@@ -352,6 +352,12 @@ sge_status sge_plan_from_order_text(uint32_t k, uint32_t m, const uint32_t *edge
 
 /* Check a plan blob for internal consistency (levels, masks, tail validity). */
 sge_status sge_plan_validate(const sge_plan_blob *blob);
+/* *order_free = 1 when the plan is known to count the same instances whatever
+ * order the vertex ids have: its bounds form a stabilizer chain of the
+ * pattern's automorphisms, as every planned blob's do (labels: the pattern
+ * labels of a labeled plan, else NULL).  Such a plan may be counted with all
+ * bounds reversed; any other keeps its own direction. */
+sge_status sge_plan_order_free(const sge_plan_blob *blob, const uint32_t *labels, uint32_t *order_free);
 
 /* ---- device graph (replaces the DataGraph/CandidateSpace the join reads) ----
  * Every graph handle also builds a hub index in HBM: a neighbour bitmap for

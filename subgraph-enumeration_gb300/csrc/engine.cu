@@ -2645,6 +2645,7 @@ struct sge_plan {
     const sge_bags *bags = nullptr;  // bag relations its tail levels read (sge_plan_use_bags)
     bool has_labels = false;         // pattern labels attached (sge_plan_set_labels)
     uint32_t labels[SGE_MAX_K] = {};
+    bool order_free = false;         // counts the same under every id order (sge_plan_order_free)
 };
 
 namespace sge {
@@ -2959,9 +2960,9 @@ void drop_dense(LaunchCfg &L) {
     for (auto &d : L.dps) d.dcls = 0;
 }
 
-// Reversing every symmetry restriction keeps the count over all roots (map
-// each id x to n - 1 - x), and picks which end of the id order the candidates
-// come from.  Where low ids have the high degrees, as R-MAT and Chung-Lu
+// Reversing every symmetry restriction of a plan whose count does not depend on
+// the id order (sge_plan_order_free) keeps the count over all roots (map each id
+// x to n - 1 - x), and picks which end of the id order the candidates come from.  Where low ids have the high degrees, as R-MAT and Chung-Lu
 // generators and crawls number them, "x > m[j]" leaves the long side of every
 // list; the reversed plan scans the short one (graph_adopt compares the two
 // sides).  K4 over every root of R-MAT 2^18: 287 -> 36 ms, triangles 2.05 ->
@@ -3053,7 +3054,7 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         if (!plans[i]) return fail(SGE_BAD_INPUT, "plan %u is null", i);
         DevPlan &d = L.dps[i];
         d = plans[i]->dp;
-        if (g->mirror && mirror_ok(d, o)) mirror_plan(d);
+        if (g->mirror && plans[i]->order_free && mirror_ok(d, o)) mirror_plan(d);
         d.task_begin = total;
         const unsigned long long stride = o.root_stride > 1 ? o.root_stride : 1ull;
         const unsigned long long offs = o.root_offset;
@@ -3782,6 +3783,8 @@ sge_status sge_plan_create(const sge_plan_blob *blob, sge_plan **out) {
     sge_plan *p = new sge_plan();
     p->blob = *blob;
     to_devplan(*blob, p->dp);
+    uint32_t free_order = 0;   // (a labeled plan's depends on its labels)
+    if (!blob->labeled && sge_plan_order_free(blob, nullptr, &free_order) == SGE_OK) p->order_free = free_order != 0;
     *out = p;
     return SGE_OK;
 }
@@ -3801,12 +3804,14 @@ sge_status sge_plan_set_tuning(sge_plan *p, const sge_plan_tuning *t) {
 sge_status sge_plan_set_labels(sge_plan *p, const uint32_t *labels) {
     if (!p) return fail(SGE_BAD_INPUT, "sge_plan_set_labels: null plan");
     if (!labels) {
-        p->has_labels = false;
+        p->has_labels = p->order_free = false;
         return SGE_OK;
     }
     if (!p->blob.labeled) return fail(SGE_BAD_INPUT, "the plan was planned without labels (sge_plan_opts.vertex_labels)");
     for (uint32_t u = 0; u < p->blob.k; ++u) p->labels[u] = labels[u];
     p->has_labels = true;
+    uint32_t free_order = 0;
+    if (sge_plan_order_free(&p->blob, p->labels, &free_order) == SGE_OK) p->order_free = free_order != 0;
     return SGE_OK;
 }
 
@@ -4049,7 +4054,7 @@ sge_status sge::enumerate_rows(sge_graph *g, const sge_plan *p, uint32_t *d_out,
     DeviceGuard restore_device;
     CUDA_TRY(cudaSetDevice(g->device));
     DevPlan d = p->dp;
-    if (any_representative && g->mirror) mirror_plan(d);
+    if (any_representative && g->mirror && p->order_free) mirror_plan(d);
     d.ne = d.k;  // every level is enumerated
     d.join_style = SGE_JOIN_WCOJ;  // (the same tuples; running lists are not kept here)
     d.ntrie = 0;

@@ -737,6 +737,138 @@ sge_status sge_plan_validate(const sge_plan_blob *b) {
 
 }  // extern "C"
 
+// ---- whether a plan's bounds depend on the id order ----
+// A plan that keeps, for every instance and every order of its vertices' ids,
+// the same number of embeddings counts the same instances when all ids are
+// reversed.  Bounds from a stabilizer chain do (restrictions() above): take
+// any vertex v, bound it below (or above) every other vertex of its orbit, go
+// on with the automorphisms that fix v.  Whatever the ids, exactly |orbit|^-1
+// of the automorphisms satisfy a step.  Other bounds that sge_plan_validate
+// accepts (a wedge with its centre below one leaf only) do not.
+namespace {
+struct BoundSystem {
+    uint32_t k = 0;
+    Pattern p;
+    uint32_t less[SGE_MAX_K] = {};  // transitively closed: less[a] = vertices above a
+    int budget = 1 << 16;           // steps of either search; past it the answer is "not known"
+};
+
+// An automorphism that maps v to w and every vertex of `fixed` to itself?
+bool maps_to(BoundSystem &s, uint32_t fixed, uint32_t v, uint32_t w) {
+    if (s.p.deg(v) != s.p.deg(w) || s.p.label[v] != s.p.label[w]) return false;
+    uint8_t seq[SGE_MAX_K], map[SGE_MAX_K];
+    uint32_t n = 0, used = fixed | (1u << w), next[SGE_MAX_K] = {};
+    for (uint32_t u = 0; u < s.k; ++u)
+        if ((fixed >> u) & 1u) { seq[n] = (uint8_t)u; map[n++] = (uint8_t)u; }
+    seq[n] = (uint8_t)v;
+    map[n++] = (uint8_t)w;
+    const uint32_t given = n;
+    for (uint32_t u = 0; u < s.k; ++u)
+        if (!((fixed >> u) & 1u) && u != v) seq[n++] = (uint8_t)u;
+    auto fits = [&](uint32_t i, uint32_t c) {
+        if (s.p.deg(c) != s.p.deg(seq[i]) || s.p.label[c] != s.p.label[seq[i]]) return false;
+        for (uint32_t j = 0; j < i; ++j)
+            if (s.p.edge(seq[i], seq[j]) != s.p.edge(c, map[j])) return false;
+        return true;
+    };
+    if (!fits(given - 1, w)) return false;
+    uint32_t i = given;
+    while (i < s.k) {
+        uint32_t c = next[i];
+        while (c < s.k && (((used >> c) & 1u) || !fits(i, c))) ++c;
+        if (--s.budget < 0) return false;
+        if (c < s.k) {
+            map[i] = (uint8_t)c;
+            used |= 1u << c;
+            next[i] = c + 1;
+            if (++i < s.k) next[i] = 0;
+        } else {
+            if (i == given) return false;
+            --i;
+            used &= ~(1u << map[i]);
+        }
+    }
+    return true;
+}
+
+void close_order(uint32_t k, uint32_t *less) {
+    for (uint32_t x = 0; x < k; ++x)
+        for (uint32_t a = 0; a < k; ++a)
+            if ((less[a] >> x) & 1u) less[a] |= less[x];
+}
+
+// The bounds beyond `used` (closed) from a stabilizer chain that fixes `fixed`?
+bool is_chain(BoundSystem &s, uint32_t fixed, const uint32_t *used) {
+    bool all = true;
+    for (uint32_t a = 0; a < s.k && all; ++a) all = !(s.less[a] & ~used[a]);
+    if (all) return true;
+    for (uint32_t v = 0; v < s.k; ++v) {
+        if ((fixed >> v) & 1u) continue;
+        uint32_t others = 0, below = 0;
+        for (uint32_t w = 0; w < s.k; ++w) {
+            if (w != v && !((fixed >> w) & 1u) && maps_to(s, fixed, v, w)) others |= 1u << w;
+            if ((s.less[w] >> v) & 1u) below |= 1u << w;
+        }
+        if (--s.budget < 0) return false;
+        if (!others || ((others & ~s.less[v]) && (others & ~below))) continue;
+        uint32_t more[SGE_MAX_K];
+        for (uint32_t a = 0; a < s.k; ++a) more[a] = used[a];
+        if (!(others & ~s.less[v])) more[v] |= others;
+        else
+            for (uint32_t w = 0; w < s.k; ++w)
+                if ((others >> w) & 1u) more[w] |= 1u << v;
+        close_order(s.k, more);
+        if (is_chain(s, fixed | (1u << v), more)) return true;
+    }
+    return false;
+}
+}  // namespace
+
+extern "C" sge_status sge_plan_order_free(const sge_plan_blob *b, const uint32_t *labels, uint32_t *order_free) {
+    if (!order_free) return fail(SGE_BAD_INPUT, "sge_plan_order_free: null output");
+    *order_free = 0;
+    const sge_status st = sge_plan_validate(b);
+    if (st != SGE_OK) return st;
+    if (b->labeled && !labels) return fail(SGE_BAD_INPUT, "sge_plan_order_free: a labeled plan without labels");
+    const uint32_t k = b->k, ne = b->num_enum;
+    if (b->tail_mode == SGE_TAIL_IEP) {   // the sum over distinct tail vertices, nothing else
+        sge_plan_blob want;
+        memset(&want, 0, sizeof want);
+        set_partitions(b->tail_len, want);
+        if (b->num_partitions != want.num_partitions) return SGE_OK;
+        for (uint32_t p = 0; p < want.num_partitions; ++p) {
+            if (b->part_coef[p] != want.part_coef[p] || b->part_nblocks[p] != want.part_nblocks[p]) return SGE_OK;
+            for (uint32_t x = 0; x < want.part_nblocks[p]; ++x)
+                if (b->part_block[p][x] != want.part_block[p][x]) return SGE_OK;
+        }
+    }
+    // the pattern and its bounds over levels.  CHOOSE counts sets of candidates
+    // of its first level: that level's parents and bounds, the tail in order
+    BoundSystem s;
+    s.k = s.p.k = k;
+    for (uint32_t i = 1; i < k; ++i) {
+        const bool choose = b->tail_mode == SGE_TAIL_CHOOSE && i > ne;
+        const uint32_t l = choose ? ne : i;
+        for (uint32_t j = 0; j < i; ++j) {
+            if ((b->parents[l] >> j) & 1u) { s.p.adj[i] |= 1u << j; s.p.adj[j] |= 1u << i; }
+            if (choose && j >= ne) s.less[j] |= 1u << i;
+            if (i == 1) continue;
+            if ((b->lower[l] >> j) & 1u) s.less[j] |= 1u << i;
+            if ((b->upper[l] >> j) & 1u) s.less[i] |= 1u << j;
+        }
+    }
+    if (b->root_kind == SGE_ROOT_ASC) s.less[0] |= 2u;
+    if (b->root_kind == SGE_ROOT_DESC) s.less[1] |= 1u;
+    for (uint32_t i = 0; b->labeled && i < k; ++i)
+        s.p.label[i] = labels[b->order[b->tail_mode == SGE_TAIL_CHOOSE && i > ne ? ne : i]];
+    close_order(k, s.less);
+    for (uint32_t a = 0; a < k; ++a)
+        if ((s.less[a] >> a) & 1u) return SGE_OK;   // contradictory
+    const uint32_t none[SGE_MAX_K] = {};
+    *order_free = is_chain(s, 0, none) ? 1u : 0u;
+    return SGE_OK;
+}
+
 extern "C" sge_status sge_plan_pattern_learned(uint32_t k, uint32_t m, const uint32_t *edges,
                                                const sge_graph_stats *gs, const sge_plan_opts *opts, sge_mlp *scorer,
                                                uint32_t shortlist, sge_plan_blob *out) {

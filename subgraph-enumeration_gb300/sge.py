@@ -131,6 +131,7 @@ SIGNATURES = {
     "sge_plan_pattern": (C.c_int, [u32, u32, _P(u32), C.c_void_p, _P(PlanOpts), _P(PlanBlob)]),
     "sge_pattern_info": (C.c_int, [u32, u32, _P(u32), _P(u64), _P(u32)]),
     "sge_plan_validate": (C.c_int, [_P(PlanBlob)]),
+    "sge_plan_order_free": (C.c_int, [_P(PlanBlob), _P(u32), _P(u32)]),
     "sge_plan_from_order_text": (C.c_int, [u32, u32, _P(u32), C.c_char_p, _P(GraphStats), _P(PlanOpts),
                                            _P(PlanBlob), _P(u32)]),
     "sge_graph_stats_compute": (C.c_int, [_P(u32), _P(u32), u32, _P(GraphStats)]),
@@ -552,6 +553,15 @@ def plan_learned(pattern: PatternGraph, stats: "GraphStats", scorer: MLP, iep: b
 
 def validate_plan(b: PlanBlob) -> None:
     _check(lib().sge_plan_validate(C.byref(b)))
+
+
+def plan_order_free(b: PlanBlob, labels=None) -> bool:
+    """Whether the plan counts the same instances under every order of the ids
+    (sge_plan_order_free; labels: the pattern labels of a labeled plan)."""
+    la = None if labels is None else np.ascontiguousarray(labels, np.uint32)
+    r = u32()
+    _check(lib().sge_plan_order_free(C.byref(b), None if la is None else _u32p(la), C.byref(r)))
+    return bool(r.value)
 
 
 # ---------------------------------------------------------------- engine ----
