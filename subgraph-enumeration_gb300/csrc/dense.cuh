@@ -766,14 +766,15 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
 
 // Host: the universe class of a plan (0..3: N(m0) ∩ N(m1), N(m0), N(m1), union), -1 when the path
 // does not take it.  Level 2 must close a triangle on the root edge and every later level must touch
-// the root.  With three enumerated levels, or four and a tail whose list does not depend on the last
+// the root; plans with a level bounded above and below the same vertex stay on lists, where nothing
+// fits it (the masks take one bound per pair of levels).  With three enumerated levels, or four and a tail whose list does not depend on the last
 // of them, the rows of a root are read about once each: the list path does that without building them.
 inline int dense_class(const DevPlan &d) {
     if (d.vlab || d.ntrie || d.k > DENSE_MAX_K || d.ne < 4 || (d.parents[2] & 3u) != 3u) return -1;
     if (d.tail_mode == SGE_TAIL_IEP && d.T > DENSE_MAX_T) return -1;
     bool all0 = true, all1 = true, dep = false;
     for (uint32_t i = 2; i < d.k; ++i) {
-        if (!(d.parents[i] & 3u)) return -1;
+        if (!(d.parents[i] & 3u) || (d.lower[i] & d.upper[i])) return -1;
         all0 &= (d.parents[i] & 1u) != 0;
         all1 &= (d.parents[i] & 2u) != 0;
         dep |= i >= d.ne && ((d.parents[i] >> (d.ne - 1)) & 1u);

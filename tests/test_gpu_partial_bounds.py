@@ -60,3 +60,22 @@ def test_partial_bounds_keep_their_direction(sge, oracle, reverse):
     assert [sum(s) for s in zip(*shards)] == want
     assert counted == want and capped == want
     assert full == want and batch == want
+
+
+def test_contradictory_bounds_count_nothing(sge, oracle):
+    """Above and below the same vertex: sge_plan_validate takes it, no vertex fits."""
+    g = sge.gen_rmat(9, 3000, seed=3)
+    out = []
+    for k, edges in ((5, list(itertools.combinations(range(5), 2))), (6, list(itertools.combinations(range(6), 2)))):
+        for lv in (2, 3, k - 1):
+            b = edited(sge, k, edges, [], list(range(k)))
+            b.lower[lv] |= 2
+            b.upper[lv] |= 2
+            sge.validate_plan(b)
+            out.append(b)
+    want = [oracle.count_plan(g.offsets, g.nbrs, b, threads=0)[0] for b in out]
+    assert want == [0] * len(out)
+    with sge.Engine(g) as eng:
+        lists, _, _ = eng.count(out, max_level_capacity=eng.info()["max_degree"])
+        full, _, _ = eng.count(out)
+    assert lists == want and full == want
