@@ -42,12 +42,12 @@ __device__ __forceinline__ uint64_t splitmix64_d(uint64_t x) {
 
 // Both directions of every edge as keys src << bits | dst; a self-loop becomes
 // two all-ones keys, which no edge has (src = dst), sort last and are dropped.
-// An id >= n sets *bad.
-__global__ void directed_keys(const uint2 *edges, unsigned long long m, uint32_t n, uint32_t bits,
+// An id >= n sets *bad.  (The caller's list may start at any word: single loads.)
+__global__ void directed_keys(const uint32_t *edges, unsigned long long m, uint32_t n, uint32_t bits,
                               ulonglong2 *keys, uint32_t *bad) {
     const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    const uint32_t u = edges[i].x, v = edges[i].y;
+    const uint32_t u = edges[2 * i], v = edges[2 * i + 1];
     const unsigned long long none = bits == 32 ? ~0ull : (1ull << (2 * bits)) - 1;
     if (u >= n || v >= n) atomicOr(bad, 1u);
     if (u == v || u >= n || v >= n) keys[i] = make_ulonglong2(none, none);
@@ -207,8 +207,7 @@ sge_status sge_graph_create_from_device_edges(const uint32_t *d_edges, uint64_t 
     const unsigned ntiles = (unsigned)((nd + DEDUP_TILE - 1) / DEDUP_TILE);
     if (m) {
         CUDA_TRY(cudaMalloc(&keys.p, 8 * nd));
-        directed_keys<<<grid_for(m), 256>>>(reinterpret_cast<const uint2 *>(d_edges), m, num_vertices, bits,
-                                            keys.as<ulonglong2>(), bad.as<uint32_t>());
+        directed_keys<<<grid_for(m), 256>>>(d_edges, m, num_vertices, bits, keys.as<ulonglong2>(), bad.as<uint32_t>());
         CUDA_TRY(cudaGetLastError());
         uint32_t hbad = 0;
         CUDA_TRY(cudaMemcpy(&hbad, bad.p, 4, cudaMemcpyDeviceToHost));
