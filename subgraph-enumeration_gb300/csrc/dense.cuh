@@ -138,13 +138,26 @@ __device__ __forceinline__ uint32_t dense_tasks(uint32_t n2, uint32_t ps) {
 // Selects the dense roots: one warp per sampled root edge intersects the two
 // lists (the shorter one scanned), and the edge gets a record and arena space
 // for every class that fits and is worth it.  Bound by the list loads, as a triangle count of the sample.
+// The launch's time budget starts here (flags + 2 holds the start).
 __global__ void __launch_bounds__(256) dense_select_kernel(DevGraph g, unsigned long long root_offset,
                                                            unsigned long long root_stride, unsigned long long nedges,
-                                                           uint32_t maxdeg, DenseBuf D, uint32_t *flags) {
+                                                           uint32_t maxdeg, DenseBuf D, unsigned long long deadline_ns,
+                                                           uint32_t *flags) {
     const uint32_t lane = lane_id();
     const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long *>(flags + 2) = globaltimer_ns();
+    Ctx<MODE_PLAIN> c;
+    c.flags = flags;
+    c.deadline = deadline_ns;
+    unsigned long long t0 = 0;
+    if (lane == 0) {
+        volatile unsigned long long *slot = reinterpret_cast<volatile unsigned long long *>(flags + 2);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *slot = globaltimer_ns();
+        t0 = *slot;
+        if (!t0) t0 = globaltimer_ns();   // (block 0 has not begun)
+    }
+    c.tstart = __shfl_sync(FULL_MASK, t0, 0);
     for (unsigned long long j = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < nedges; j += nw) {
+        if (out_of_time(c)) break;
         const uint2 e = g.edges[root_offset + j * root_stride];
         const uint32_t *pu, *pv;
         uint32_t du, dv;
@@ -219,7 +232,8 @@ __device__ __forceinline__ uint32_t block_prefix256(uint32_t v, uint32_t *ws, ui
 // shared memory, then a warp per row.  A hub's row is gathered from its
 // bitmap (one load per bit, 32 bits a ballot); a shorter list is scanned and
 // each neighbour looked up in U; a long list without a bitmap is searched.
-__global__ void __launch_bounds__(256) dense_build_kernel(DevGraph g, DenseBuf D) {
+__global__ void __launch_bounds__(256) dense_build_kernel(DevGraph g, DenseBuf D, unsigned long long deadline_ns,
+                                                          uint32_t *flags) {
     __shared__ uint32_t Us[DENSE_MAX_U];         // the universe, sorted by id
     __shared__ uint32_t C[DENSE_MAX_U];          // common neighbours before index i of the shorter list; then counts
     __shared__ uint32_t Up[DENSE_MAX_U];         // the universe by position (DENSE_NONE: padding)
@@ -232,7 +246,15 @@ __global__ void __launch_bounds__(256) dense_build_kernel(DevGraph g, DenseBuf D
     const uint32_t ncls = __popc(D.need), nitems = min(D.hdr[0], D.rec_cap) * ncls * PARTS;
     while (true) {
         __syncthreads();
-        if (threadIdx.x == 0) item_s = atomicAdd(D.hdr + 1, 1u);
+        if (threadIdx.x == 0) {
+            const unsigned long long t0 = *reinterpret_cast<volatile unsigned long long *>(flags + 2);
+            if (deadline_ns && globaltimer_ns() - t0 > deadline_ns) {
+                atomicOr(flags, FLAG_TIMEOUT);
+                item_s = 0xFFFFFFFFu;   // (the count kernel then takes no task)
+            } else {
+                item_s = atomicAdd(D.hdr + 1, 1u);
+            }
+        }
         __syncthreads();
         const uint32_t item = item_s;
         if (item >= nitems) break;
@@ -662,6 +684,7 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
     const uint32_t nrec = min(D.hdr[0], D.rec_cap);
     const unsigned long long total = *reinterpret_cast<unsigned long long *>(D.hdr + 6) * D.npo;
     unsigned long long *queue = reinterpret_cast<unsigned long long *>(D.hdr + 4);
+    if (*reinterpret_cast<volatile uint32_t *>(flags) & FLAG_TIMEOUT) return;   // (rows may not be built)
     while (true) {
         unsigned long long t = 0;
         if (lane == 0) t = atomicAdd(queue, 1ull);
@@ -734,6 +757,7 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
         bool ok = true;
         for (uint32_t p2 = c0; p2 < c1 && ok; ++p2) {   // (common neighbours are the first positions)
             if (!((S.run(dense_slot(1, 2))[p2 >> 5] >> (p2 & 31u)) & 1u)) continue;
+            if (out_of_time(c)) { ok = false; break; }
             dense_match(S, V, k, 2, p2);
             if (ne == 4) {
                 dense_leaf(P, S, V, 2, acc, flags);
@@ -746,12 +770,12 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
                     if (--lv < 3) break;
                     continue;
                 }
+                if (out_of_time(c)) { ok = false; break; }
                 dense_match(S, V, k, lv, p);
                 if (lv + 2 == ne) {
                     dense_leaf(P, S, V, lv, acc, flags);
                     continue;
                 }
-                if (out_of_time(c)) { ok = false; break; }
                 ++lv;
             }
         }

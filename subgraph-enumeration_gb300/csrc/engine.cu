@@ -3269,8 +3269,9 @@ sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, ui
         dskip = D.skip;
         CUDA_TRY(cudaMemsetAsync(dense, 0, L.off_dskip + L.dedges, s));
         const unsigned sel = (unsigned)std::min<unsigned long long>((L.dedges + 7) / 8, 16ull * g->num_sms);
-        dense_select_kernel<<<sel, 256, 0, s>>>(dg, L.droot_offset, L.droot_stride, L.dedges, L.dmaxdeg, D, dflags);
-        dense_build_kernel<<<8u * g->num_sms, 256, 0, s>>>(dg, D);
+        dense_select_kernel<<<sel, 256, 0, s>>>(dg, L.droot_offset, L.droot_stride, L.dedges, L.dmaxdeg, D,
+                                             L.deadline, dflags);
+        dense_build_kernel<<<8u * g->num_sms, 256, 0, s>>>(dg, D, L.deadline, dflags);
         dense_prefix_kernel<<<1, 256, 0, s>>>(D);
         dense_count_kernel<<<(unsigned)L.dense_blocks, 128, 4 * dense_warp_bytes(L.dslots), s>>>(
             dplans, D, dcounts, H.ptime, L.deadline, dflags, L.dslots);

@@ -1,0 +1,43 @@
+"""A launch that runs out of its time budget ends soon after it.  Every root of
+R-MAT 2^20 with 16M edges, where these patterns take from a quarter of a second
+to many seconds: a budget of 1 ms has to end the call within 12 ms (a scan of
+two long lists, the unit that is not cut, is some 3 ms there)."""
+import time
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def clique(k, drop=()):
+    return [(a, b) for a in range(k) for b in range(a + 1, k) if (a, b) not in drop]
+
+
+@pytest.fixture(scope="module")
+def engine(sge):
+    with sge.Engine.rmat_device(20, 16_000_000, seed=1) as eng:
+        yield eng
+
+
+def elapsed_ms(sge, eng, b, budget):
+    t = time.perf_counter()
+    with pytest.raises(sge.SgeError) as e:
+        eng.count([b], time_budget_s=budget)
+    assert e.value.status_name == "TIMEOUT"
+    return (time.perf_counter() - t) * 1e3
+
+
+def check(sge, eng, k, edges):
+    b = sge.plan(sge.PatternGraph.from_edges(k, edges), eng, iep=False)
+    elapsed_ms(sge, eng, b, 1e-9)   # buffers
+    assert min(elapsed_ms(sge, eng, b, 1e-3) for _ in range(5)) < 12.0
+    tri = sge.plan(sge.PatternGraph.from_edges(3, clique(3)), eng)
+    assert eng.count([tri], root_stride=997)[0][0] > 0   # the handle stays usable
+
+
+# selection over every root edge, rows of up to 1 GB, deep prefixes on rows
+@pytest.mark.parametrize("k,edges", [(5, clique(5)), (6, clique(6)), (6, clique(6, [(0, 1), (2, 3), (4, 5)])),
+                                     (5, [(0, 1), (0, 2), (0, 3), (0, 4), (1, 2), (2, 3), (3, 4), (1, 4)])],
+                         ids=["k5", "k6", "octahedron", "wheel4"])
+def test_bit_rows(sge, engine, k, edges):
+    check(sge, engine, k, edges)
