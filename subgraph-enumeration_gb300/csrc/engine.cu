@@ -1776,10 +1776,11 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
         S.bp[lane] = bp - (incl - blen);
         uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
         __syncwarp();
-        uint32_t begin = 0;   // this task's part of the scan (the pair step's level is level 2)
+        uint32_t begin = 0;   // this task's part of the scan (the pair step's level is level 2), in whole
+                              // steps of 32: the loops below look at the clock by the step's number
         if (parts > 1) {
-            begin = (uint32_t)((unsigned long long)total * part / parts);
-            total = (uint32_t)((unsigned long long)total * (part + 1) / parts);
+            begin = (uint32_t)((unsigned long long)total * part / parts) & ~31u;
+            if (part + 1 < parts) total = (uint32_t)((unsigned long long)total * (part + 1) / parts) & ~31u;
         }
         // y of scan element j under candidate l, and whether level a+1 keeps it
         uint32_t l = 0;
