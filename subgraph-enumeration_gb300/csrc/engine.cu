@@ -1426,6 +1426,7 @@ __device__ __forceinline__ bool pair_rows(const DevPlan &P, WarpState &W, Ctx<M>
         while (todo) {
             const uint32_t l = __ffs(todo) - 1;
             todo &= todo - 1;
+            if (out_of_time(c)) return false;
             const int32_t h = __shfl_sync(FULL_MASK, hx, l);
             const uint32_t t = __shfl_sync(FULL_MASK, tr, l);
             uint32_t k = 0, kt = 0;
@@ -1593,6 +1594,7 @@ __device__ __forceinline__ bool pair_inline(const DevPlan &P, WarpState &W, Ctx<
         while (todo) {
             const uint32_t l = __ffs(todo) - 1;
             todo &= todo - 1;
+            if (out_of_time(c)) return false;
             const uint32_t *y_of = reinterpret_cast<const uint32_t *>(__shfl_sync(FULL_MASK, addr, l));
             const uint32_t len = __shfl_sync(FULL_MASK, blen, l), t = __shfl_sync(FULL_MASK, tr, l);
             PairProbe u = sp;

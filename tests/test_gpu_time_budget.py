@@ -41,3 +41,12 @@ def check(sge, eng, k, edges):
                          ids=["k5", "k6", "octahedron", "wheel4"])
 def test_bit_rows(sge, engine, k, edges):
     check(sge, engine, k, edges)
+
+
+# a scan per candidate of the last enumerated levels
+@pytest.mark.parametrize("k,edges", [(5, [(0, 1), (0, 2), (0, 4), (1, 3), (1, 4), (2, 3)]),
+                                     (5, [(0, 1), (0, 2), (1, 2), (1, 3), (2, 4)]),
+                                     (5, [(0, 1), (0, 2), (0, 3), (0, 4), (1, 2), (2, 3), (3, 4)])],
+                         ids=["house", "bull", "gem"])
+def test_inline_tails(sge, engine, k, edges):
+    check(sge, engine, k, edges)
