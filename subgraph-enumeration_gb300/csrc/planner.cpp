@@ -39,9 +39,10 @@ bool graph_stats(const sge_graph *g, sge_graph_stats *out);
 double sample_clustering(const uint32_t *off, const uint32_t *nb, uint32_t n);
 
 // M_j = Σ d^j in vertex order, each power by repeated multiplication.  The
-// powers of a degree are the same for every vertex that has it, so they come
-// from a table (where the largest degree keeps it in cache): per vertex one
-// row is added to the sums.  1M vertices: 20 -> 3 ms on one core.
+// powers of a degree are the same for every vertex that has it, so those of the
+// degrees below 4,096 come from a table (at most 576 KB, which a core's cache
+// holds; few vertices have more) and per vertex one row is added to the sums.
+// 1M vertices: 20 -> 3 ms on one core.
 void degree_stats(const uint32_t *off, uint32_t n, sge_graph_stats *out) {
     constexpr uint32_t J = SGE_MAX_K + 2;
     memset(out, 0, sizeof *out);
@@ -55,20 +56,17 @@ void degree_stats(const uint32_t *off, uint32_t n, sge_graph_stats *out) {
         double p = 1.0;
         for (uint32_t j = 0; j < J; ++j) { row[j] = p; p *= d; }
     };
-    double sum[J] = {};
-    if (max_deg < n / 2) {
-        std::vector<double> table(((size_t)max_deg + 1) * J);
-        for (uint32_t d = 0; d <= max_deg; ++d) powers(d, &table[(size_t)d * J]);
-        for (uint32_t v = 0; v < n; ++v) {
-            const double *row = &table[(size_t)(off[v + 1] - off[v]) * J];
-            for (uint32_t j = 0; j < J; ++j) sum[j] += row[j];
-        }
-    } else {
-        double row[J];
-        for (uint32_t v = 0; v < n; ++v) {
-            powers(off[v + 1] - off[v], row);
-            for (uint32_t j = 0; j < J; ++j) sum[j] += row[j];
-        }
+    // (no table where it would hold more degrees than there are vertices)
+    const uint32_t rows = max_deg < n / 2 ? std::min(max_deg + 1, 4096u) : 0u;
+    std::vector<double> table((size_t)rows * J);
+    for (uint32_t d = 0; d < rows; ++d) powers(d, &table[(size_t)d * J]);
+    double sum[J] = {}, own[J];
+    for (uint32_t v = 0; v < n; ++v) {
+        const uint32_t d = off[v + 1] - off[v];
+        const double *row = own;
+        if (d < rows) row = &table[(size_t)d * J];
+        else powers(d, own);
+        for (uint32_t j = 0; j < J; ++j) sum[j] += row[j];
     }
     for (uint32_t j = 0; j < J; ++j) out->moments[j] = sum[j];
 }
