@@ -43,7 +43,7 @@ def _stale(target: Path, deps: list[Path]) -> bool:
 
 def build_sge(verbose: bool = False) -> Path:
     OUT.mkdir(parents=True, exist_ok=True)
-    headers = [INC / "sge.h", CSRC / "common.hpp", CSRC / "device_util.hpp"]
+    headers = [INC / "sge.h", CSRC / "common.hpp", CSRC / "device_util.hpp", CSRC / "dense.cuh"]
     jobs = []
     objs = []
     for s in CU_SRCS:
