@@ -715,6 +715,8 @@ class Engine:
                 raise SgeError(2, f"{rows} instances exceed max_rows={max_rows}")
             out = np.zeros(max(rows, 1) * pattern.k, np.uint32)
             _check(lib().sge_match_set(self._h, ph, pattern.k, pattern.m, _u32p(e), _u32p(out), rows, C.byref(n)))
+            if n.value != rows:
+                raise SgeError(5, f"{n.value} instances enumerated, {rows} counted")
             return out[: n.value * pattern.k].reshape(n.value, pattern.k)
         finally:
             lib().sge_plan_destroy(ph)

@@ -39,3 +39,21 @@ def test_labeled_and_long_tail_plans(sge, cap):
     with sge.Engine(sge.DataGraph.from_edges(np.array([(i, i + 1) for i in range(50)]), 51)) as eng:
         assert match(sge, eng, sge.plan(k4, eng, iep=False), k4, cap)[:2] == ("OK", 0)
         assert eng.match_set(k4).shape == (0, 4)
+
+
+@pytest.mark.parametrize("more", [-1, 1])
+def test_rows_are_compared_with_the_count(sge, monkeypatch, more):
+    tri = sge.PatternGraph.from_edges(3, [(0, 1), (0, 2), (1, 2)])
+    with sge.Engine(sge.gen_chung_lu(200, 700, 2.1, 80, seed=1)) as eng:
+        count = eng.count
+        rows = len(eng.match_set(tri))
+
+        def wrong(plans, **kw):
+            c, inst, st = count(plans, **kw)
+            return c, [n + more for n in inst], st
+        monkeypatch.setattr(eng, "count", wrong)
+        with pytest.raises(sge.SgeError) as e:
+            eng.match_set(tri)
+        assert e.value.status_name == ("CUDA_ERROR" if more > 0 else "OOM")
+        monkeypatch.undo()
+        assert len(eng.match_set(tri)) == rows
