@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(128) bf16_forward_fused(const float *__restric
 
 // One batch's rows through the network and back, FT_ROWS per block: A1, A2 and
 // the gradients at Z1, Z2 for the parameter kernel, and the loss.  Row i of the
-// batch is row idx[i] of x and t (i itself when idx is null).
+// batch is row idx[i] of x and t (i itself when idx is null).  x may be X: a
+// batch that is in order already gathers onto itself, so neither is __restrict__.
 constexpr int FT_ROWS = 4, FT_THREADS = 256;
 struct FtSmem {
     float w1[FUSE_MAX][FUSE_MAX + 1], w2[FUSE_MAX][FUSE_MAX + 1];
@@ -333,10 +334,10 @@ __device__ __forceinline__ void fill_rows(float (*out)[FUSE_MAX + 1], const floa
         }
     }
 }
-__global__ void __launch_bounds__(FT_THREADS) train_rows_fused(const float *__restrict__ P, const float *__restrict__ x,
+__global__ void __launch_bounds__(FT_THREADS) train_rows_fused(const float *__restrict__ P, const float *x,
                                                                const float *__restrict__ t,
                                                                const uint32_t *__restrict__ idx, int B, int in, int hid,
-                                                               float *__restrict__ X, float *__restrict__ A1,
+                                                               float *X, float *__restrict__ A1,
                                                                float *__restrict__ A2, float *__restrict__ dZ1,
                                                                float *__restrict__ dZ2, float *__restrict__ dY,
                                                                float *__restrict__ loss) {
