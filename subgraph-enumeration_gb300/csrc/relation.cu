@@ -524,7 +524,8 @@ sge_status sort_packed(uint32_t *d_tuples, uint64_t n, uint32_t arity, const Wid
         cudaFree(a);
         cudaFree(b);
         cudaGetLastError();
-        if (arity > 1) return sort_wide(d_tuples, n, arity, w);   // (needs less at once)
+        // (128-bit keys: the wide form's are half as large)
+        if (sizeof(K) == 16 && arity > 1) return sort_wide(d_tuples, n, arity, w);
         return fail(SGE_OOM, "sge_sort_tuples: %s", cudaGetErrorString(e));
     }
     pack_kernel<K><<<grid_for(n), 256>>>(d_tuples, n, arity, w, a);
