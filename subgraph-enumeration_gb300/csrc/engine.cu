@@ -3475,9 +3475,10 @@ __global__ void __launch_bounds__(256) csr_check_kernel(const uint32_t *off, con
 __global__ void upper_parts_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, uint32_t *up,
                                    unsigned long long *sums) {
     unsigned long long su = 0, sd = 0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    // (64-bit index: v + the grid's threads may pass 2^32)
+    for (unsigned long long v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const uint32_t a = off[v], d = off[v + 1] - a;
-        const unsigned long long below = lb(adj + a, d, v), above = d - below;
+        const unsigned long long below = lb(adj + a, d, (uint32_t)v), above = d - below;
         up[v] = (uint32_t)above;
         su += above * above;
         sd += below * below;
@@ -3676,7 +3677,7 @@ sge_status sge::graph_adopt(uint32_t *d_off, uint32_t *d_adj, uint32_t n, uint64
             return cleanup(fail(SGE_OOM, "root edge scratch: %s", cudaGetErrorString(e)));
         unsigned long long *d_sums = reinterpret_cast<unsigned long long *>(up + words), sums[2] = {0, 0};
         cudaMemsetAsync(d_sums, 0, 16, g->stream);
-        upper_parts_kernel<<<std::min<unsigned>((n + 255) / 256, 8u * g->num_sms), 256, 0, g->stream>>>(d_off, d_adj, n,
+        upper_parts_kernel<<<(unsigned)std::min<uint64_t>(((uint64_t)n + 255) / 256, 8u * g->num_sms), 256, 0, g->stream>>>(d_off, d_adj, n,
                                                                                                     up, d_sums);
         sge_status st = device_exclusive_scan(up, up + n, n, g->stream);
         if (st == SGE_OK) {
