@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) dense_select_kernel(DevGraph g, unsigned 
     if (lane == 0) {
         volatile unsigned long long *slot = reinterpret_cast<volatile unsigned long long *>(flags + 2);
         if (blockIdx.x == 0 && threadIdx.x == 0) *slot = globaltimer_ns();
-        t0 = *slot;
+        if (deadline_ns) t0 = *slot;
         if (!t0) t0 = globaltimer_ns();   // (block 0 has not begun)
     }
     c.tstart = __shfl_sync(FULL_MASK, t0, 0);
@@ -247,13 +247,10 @@ __global__ void __launch_bounds__(256) dense_build_kernel(DevGraph g, DenseBuf D
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) {
-            const unsigned long long t0 = *reinterpret_cast<volatile unsigned long long *>(flags + 2);
-            if (deadline_ns && globaltimer_ns() - t0 > deadline_ns) {
-                atomicOr(flags, FLAG_TIMEOUT);
-                item_s = 0xFFFFFFFFu;   // (the count kernel then takes no task)
-            } else {
-                item_s = atomicAdd(D.hdr + 1, 1u);
-            }
+            bool late = false;
+            if (deadline_ns) late = globaltimer_ns() - *reinterpret_cast<volatile unsigned long long *>(flags + 2) > deadline_ns;
+            if (late) atomicOr(flags, FLAG_TIMEOUT);   // (the count kernel then takes no task)
+            item_s = late ? 0xFFFFFFFFu : atomicAdd(D.hdr + 1, 1u);
         }
         __syncthreads();
         const uint32_t item = item_s;
@@ -684,7 +681,7 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
     const uint32_t nrec = min(D.hdr[0], D.rec_cap);
     const unsigned long long total = *reinterpret_cast<unsigned long long *>(D.hdr + 6) * D.npo;
     unsigned long long *queue = reinterpret_cast<unsigned long long *>(D.hdr + 4);
-    if (*reinterpret_cast<volatile uint32_t *>(flags) & FLAG_TIMEOUT) return;   // (rows may not be built)
+    if (deadline_ns && (*reinterpret_cast<volatile uint32_t *>(flags) & FLAG_TIMEOUT)) return;   // (rows may not be built)
     while (true) {
         unsigned long long t = 0;
         if (lane == 0) t = atomicAdd(queue, 1ull);
