@@ -3175,9 +3175,11 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // three enumerated levels over N(m0) ∩ N(m1) with a tail inside it: a
         // root's work is the square of its list, which the share by list
         // length does not see (K4 over every root of R-MAT 2^18: one root ran
-        // 287 ms; split from 1,024 on, 36 ms).  (A split root's repeated
-        // setup would count in the instrumented kernel's totals.)
-        if (!thr && !L.want_stats && d.ne == 3 && (d.parents[2] & 3u) == 3u && (d.tail_par & 4u))
+        // 287 ms; split from 1,024 on, 36 ms).  A tail in N(m2) alone is a range
+        // per candidate, and splitting only repeats the setup (a triangle with
+        // a tail there: 8.9 ms, split 11.9).  (A split root's repeated setup
+        // would count in the instrumented kernel's totals.)
+        if (!thr && !L.want_stats && d.ne == 3 && (d.parents[2] & 3u) == 3u && (d.tail_par & 7u) == 7u)
             split_H = std::min(split_H, std::max(8u * split_S, 256u));
         // four enumerated levels and a leaf for every pair: under each level-2
         // candidate the pair step scans up to level 3's root list, so roots

@@ -1,0 +1,67 @@
+"""The automatic choices of a counting launch against the plainer ones that the
+options ask for, where those are the better: a launch that splits roots must
+not take far longer than one that splits none, nor bit rows far longer than
+lists.  Kernel times of the same process, best of several runs."""
+import itertools
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PATTERNS = {
+    "tailed_triangle": (4, [(0, 1), (0, 2), (1, 2), (2, 3)]),
+    "near5clique_8e": (5, [(0, 1), (0, 2), (0, 3), (0, 4), (1, 2), (1, 3), (1, 4), (2, 3)]),
+    "wheel4": (5, [(0, 1), (0, 2), (0, 3), (0, 4), (1, 2), (2, 3), (3, 4), (1, 4)]),
+    "k5": (5, list(itertools.combinations(range(5), 2))),
+    "octahedron": (6, [e for e in itertools.combinations(range(6), 2) if e not in ((0, 1), (2, 3), (4, 5))]),
+}
+NO_SPLIT = 1 << 30
+
+
+@pytest.fixture(scope="module")
+def engines(sge):
+    made = {}
+
+    def get(name):
+        if name not in made:
+            if name == "sparse":     # mean degree 7, hubs of a few hundred
+                g = sge.gen_chung_lu(300_000, 1_000_000, 2.3, 500, seed=6)
+            elif name == "uniform":  # degree 200, 2 shared neighbours per edge
+                e = np.random.default_rng(8).integers(0, 20_000, (2_000_000, 2))
+                g = sge.DataGraph.from_edges(e, 20_000)
+            else:
+                g = sge.gen_rmat(16, 700_001, seed=2)
+            made[name] = sge.Engine(g)
+        return made[name]
+    yield get
+    for eng in made.values():
+        eng.close()
+
+
+def best(eng, b, **kw):
+    ms, counts = [], set()
+    for _ in range(6):
+        c, _, st = eng.count([b], **kw)
+        ms.append(st["kernel_ms"])
+        counts.add(c[0])
+    assert len(counts) == 1
+    return min(ms[1:]), counts.pop()
+
+
+def compare(sge, eng, name, limit, other, exploration=False, labels=None, **kw):
+    k, edges = PATTERNS[name]
+    pl = None if labels is None else [i % labels for i in range(k)]
+    b = sge.plan(sge.PatternGraph.from_edges(k, edges), eng, iep=False, exploration=exploration, labels=pl)
+    if pl is not None:
+        kw["labels"] = [pl]
+    auto, count = best(eng, b, **kw)
+    plain, want = best(eng, b, **kw, **other)
+    assert count == want
+    assert auto <= limit * plain, f"{name}: {auto:.3f} ms, {plain:.3f} ms with {other}"
+
+
+# a tail that is a range per candidate: 1.3 to 1.6 times longer when split
+@pytest.mark.parametrize("exploration", [False, True])
+def test_tail_in_one_list_is_not_split(sge, engines, exploration):
+    compare(sge, engines("rmat"), "tailed_triangle", 1.15, dict(heavy_threshold=NO_SPLIT), exploration)
