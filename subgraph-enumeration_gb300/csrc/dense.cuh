@@ -803,6 +803,12 @@ inline int dense_class(const DevPlan &d) {
     if (d.ne == 4 && !dep) return -1;
     return all0 && all1 ? DENSE_BOTH : all0 ? DENSE_U : all1 ? DENSE_V : DENSE_UNION;
 }
+// Whether a level below the root enumerates all of N(m0) or N(m1).
+inline bool dense_wide(const DevPlan &d) {
+    for (uint32_t i = 3; i < d.ne; ++i)
+        if (d.parents[i] == 1u || d.parents[i] == 2u) return true;
+    return false;
+}
 // Whether every level whose row is read lies in N(m0) ∩ N(m1).
 inline bool dense_rows_both(const DevPlan &d) {
     uint32_t any = 0;

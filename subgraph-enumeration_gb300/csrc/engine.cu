@@ -129,6 +129,7 @@ struct DevPlan {
     uint32_t split_P3;                            // parts of each level-3 list per deferred task (1 = none)
     uint32_t split_par3;                          // level 3's parents among levels 0/1
     uint32_t split_W;                             // level-2 candidates x level-3 bound per task (0 = not used)
+    uint32_t split_list;                          // 1: a root is weighed by its level-2 list once built, not by degrees
     uint32_t pair;                                // 1: the last two enumerated levels run as one flattened step
     uint32_t pair_direct;                         // pair step may count a single-list tail per pair inline
     uint32_t epin;                                // exploration: tail level whose root-level running list is pinned
@@ -1904,11 +1905,11 @@ __device__ __forceinline__ void root_tries(const DevPlan &P, WarpState &W, Ctx<M
 // of each level-3 list (a heavy root is split into tasks over ranges of its
 // level-2 list and equal parts of the level-3 lists below them).
 // TWO: plans with two enumerated levels come here too (count_kernel takes
-// their roots 32 at a time itself).
-template <int M, bool TWO = false>
+// their roots 32 at a time itself).  defer(n) is asked once, with the length
+// of the level-2 list: true = the root is left to other tasks.
+template <int M, bool TWO = false, class F>
 __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpState &W, Ctx<M> &c, uint32_t u, uint32_t v,
-                                       uint32_t r2b = 0u, uint32_t r2e = 0xFFFFFFFFu, uint32_t p3 = 0u,
-                                       uint32_t np3 = 1u) {
+                                       uint32_t r2b, uint32_t r2e, uint32_t p3, uint32_t np3, F defer) {
     const uint32_t lane = lane_id();
     const uint32_t ne = P.ne;
     if (TWO && ne == 2) return leaf_roots(P, W, c, 1u, u, v);
@@ -1940,6 +1941,7 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
         // level 2's list is built once per root; pin it when later levels reuse it
         if (ok && ((P.pin_mask >> 2) & 1u)) pin_list(W, c, 2, W.flist[2], W.fcnt[2]);
     }
+    if (ok && defer(W.cnt[2])) ok = false;
     if (ok) {
         __syncwarp();
         if (lane == 0) {
@@ -2100,15 +2102,17 @@ __device__ __forceinline__ uint32_t level2_bound(const DevGraph &g, const DevPla
     return ub;
 }
 
-// Level-2 candidates per deferred task of a root, and whether the root is
-// deferred at all: by its level-2 bound, or, where the level below is scanned
-// once per candidate (split_W), by the two bounds' product.
+// Level-2 candidates per deferred task of a root, and whether a root with n2
+// of them (or at most that many) is deferred at all: by n2, or, where the level
+// below is scanned once per candidate (split_W), by n2 x that level's bound.
+// With split_list (automatic thresholds), n2 is the list that phase 0 has
+// built: degrees say little about it where few neighbours are shared.
 struct RootSplit {
     uint32_t S, P3;   // level-2 candidates per task; parts of what is below one of them
     bool heavy;
 };
-__device__ __forceinline__ RootSplit root_split(const DevGraph &g, const DevPlan &P, uint2 e, uint32_t b2) {
-    RootSplit r{P.split_S, P.split_P3, b2 > P.split_H};
+__device__ __forceinline__ RootSplit root_split(const DevGraph &g, const DevPlan &P, uint2 e, uint32_t n2) {
+    RootSplit r{P.split_S, P.split_P3, n2 > P.split_H};
     if (P.split_W) {
         uint32_t w = 0xFFFFFFFFu;
         if (P.split_par3 & 1u) w = min(w, __ldg(g.off + e.x + 1) - __ldg(g.off + e.x));
@@ -2116,7 +2120,7 @@ __device__ __forceinline__ RootSplit root_split(const DevGraph &g, const DevPlan
         w = max(w, 1u);
         r.S = max(1u, min(r.S, P.split_W / w));
         r.P3 = min(64u, (w + P.split_W - 1) / P.split_W);
-        r.heavy |= (unsigned long long)b2 * w > 2ull * P.split_W;
+        r.heavy |= (unsigned long long)n2 * w > 2ull * P.split_W;
     }
     return r;
 }
@@ -2126,13 +2130,13 @@ __device__ __forceinline__ RootSplit root_split(const DevGraph &g, const DevPlan
 struct HeavyBuf {
     uint32_t *cnt;             // per plan
     uint32_t *ids;             // plan p's list at p * cap
-    unsigned long long *pre;   // task-count prefix, parallel to ids
+    unsigned long long *pre;   // task-count prefix, parallel to ids; before that (split_list) the level-2 list's length
     unsigned long long *tot;   // per plan: phase-1 tasks
     unsigned long long *ptime; // per plan: warp-nanoseconds spent on its roots (both phases)
     uint32_t cap;
 };
 
-// A heavy root with level-2 bound b runs ceil(b / split_S) × split_P3 tasks.
+// A heavy root with n2 level-2 candidates (or that bound) runs ceil(n2 / S) × P3 tasks.
 // One warp per plan scans the heavy list between the two phases.
 __global__ void heavy_prefix_kernel(DevGraph g, const DevPlan *__restrict__ plans, uint32_t nplans, HeavyBuf H) {
     const uint32_t p = blockIdx.x, lane = threadIdx.x & 31u;
@@ -2145,9 +2149,9 @@ __global__ void heavy_prefix_kernel(DevGraph g, const DevPlan *__restrict__ plan
         unsigned long long tasks = 0;
         if (h < n && P.split_S) {
             const uint2 e = root_edge(g, P, H.ids[(size_t)p * H.cap + h]);
-            const uint32_t b2 = level2_bound(g, P, e);
-            const RootSplit sp = root_split(g, P, e, b2);
-            tasks = (unsigned long long)((b2 + sp.S - 1) / sp.S) * sp.P3;
+            const uint32_t n2 = P.split_list ? (uint32_t)H.pre[(size_t)p * H.cap + h] : level2_bound(g, P, e);
+            const RootSplit sp = root_split(g, P, e, n2);
+            tasks = (unsigned long long)((n2 + sp.S - 1) / sp.S) * sp.P3;
         }
         unsigned long long incl = tasks;
 #pragma unroll
@@ -2265,6 +2269,19 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
             roots += nk;
             continue;
         }
+        // puts a root off to phase 1; false: it is light, or its plan's list is full
+        auto defer = [&](unsigned long long t, uint2 e, uint32_t n2) {
+            if (!root_split(g, P, e, n2).heavy) return false;
+            uint32_t slot = 0;
+            if (lane == 0) slot = atomicAdd(H.cnt + cur, 1u);
+            slot = __shfl_sync(FULL_MASK, slot, 0);
+            if (slot >= H.cap) return false;
+            if (lane == 0) {
+                H.ids[(size_t)cur * H.cap + slot] = (uint32_t)t;
+                H.pre[(size_t)cur * H.cap + slot] = n2;
+            }
+            return true;
+        };
         for (unsigned long long t = t0; t < t1; ++t) {
             uint2 e;
             uint32_t r2b = 0, r2e = 0xFFFFFFFFu, q3 = 0, np3 = 1;
@@ -2281,7 +2298,7 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
                 const uint32_t h = lo - 1;
                 const unsigned long long local = t - pre[h];
                 e = root_edge(g, P, H.ids[(size_t)cur * H.cap + h]);
-                const RootSplit sp = root_split(g, P, e, level2_bound(g, P, e));
+                const RootSplit sp = root_split(g, P, e, 0u);
                 np3 = sp.P3;
                 q3 = (uint32_t)(local % np3);
                 r2b = (uint32_t)(local / np3) * sp.S;
@@ -2291,18 +2308,11 @@ __global__ void __launch_bounds__(COUNT_MAX_WARPS * 32, 7) count_kernel(DevGraph
                 e = root_edge(g, P, t);
                 if (!root_kept(g, P, e, labels_of<M>(P))) continue;
                 ++roots;
-                if (P.split_S && root_split(g, P, e, level2_bound(g, P, e)).heavy) {
-                    uint32_t slot = 0;
-                    if (lane == 0) slot = atomicAdd(H.cnt + cur, 1u);
-                    slot = __shfl_sync(FULL_MASK, slot, 0);
-                    if (slot < H.cap) {
-                        if (lane == 0) H.ids[(size_t)cur * H.cap + slot] = (uint32_t)t;
-                        continue;
-                    }
-                }
+                if (P.split_S && !P.split_list && defer(t, e, level2_bound(g, P, e))) continue;
             }
             if (lane == 0) W.t_root = globaltimer_ns();
-            acc += run_root<M>(P, W, c, e.x, e.y, r2b, r2e, q3, np3);
+            acc += run_root<M>(P, W, c, e.x, e.y, r2b, r2e, q3, np3,
+                               [&](uint32_t n2) { return phase == 0 && P.split_list && defer(t, e, n2); });
             if (lane == 0) atomicAdd(H.ptime + cur, globaltimer_ns() - W.t_root);
         }
     }
@@ -2599,6 +2609,7 @@ struct sge_graph {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int num_sms = 0;
     bool launched = false;     // a counting launch has run on this graph
+    bool planner_stats = false;  // stats hold the planner's moments and clustering
     bool mirror = false;       // lists are shorter below a vertex than above it (see mirror_plan)
     // hub index (neighbour bitmaps of the highest-degree vertices)
     uint32_t *d_hub_bits = nullptr;
@@ -2987,6 +2998,17 @@ void mirror_plan(DevPlan &d) {
     if (d.root_kind != SGE_ROOT_ANY) d.root_kind = d.root_kind == SGE_ROOT_ASC ? SGE_ROOT_DESC : SGE_ROOT_ASC;
 }
 
+// Common neighbours of a root edge on average: closed wedges over edges (random
+// graphs of degree 9 and 200: 0 and 2.0, a Chung-Lu graph of mean degree 7: 0.2,
+// one of degree 28: 15, ring lattices of degree 24 and 120: 16 and 88, R-MAT
+// 2^14 to 2^18: 48 to 30).  Many without planner statistics.
+double shared_neighbours(const sge_graph *g) {
+    const double *M = g->stats.moments;
+    return g->planner_stats ? g->stats.clustering * (M[2] - M[1]) / std::max(M[1], 1.0) : 1e9;
+}
+// Few of them: level-2 lists are far shorter than the degrees that bound them.
+bool few_shared(const sge_graph *g) { return shared_neighbours(g) < 4.0; }
+
 // Chooses the plans whose dense roots are counted on bitsets and lays out
 // their buffer.  The instrumented kernel (its counters are defined on lists)
 // and runs with a caller's list capacity (which lists may overflow) keep to
@@ -3166,12 +3188,22 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // 3.5, 8 -> 3.2 ms; on all 2M of them 35.6, 42.7, 79.7 ms)
         const uint32_t split_S = split3 ? 1u
             : (uint32_t)std::min<unsigned long long>(128, std::max<unsigned long long>(8, 2ull * d.ntasks / warps));
+        const uint32_t thr = tu.heavy_threshold ? tu.heavy_threshold : o.heavy_threshold;
+        // Roots weighed by the list that phase 0 has built (split_list) where
+        // that says more than the degrees: with three enumerated levels, and
+        // where edges share few neighbours.  Hubs elsewhere make work that a
+        // short list does not show (8-edge near-5-cliques on 30,000 roots of
+        // R-MAT 2^18: 10 ms by degrees, 38 by the list).
+        const bool few = few_shared(g);
         // (labels leave few of the roots: one in 256 is taken for granted)
         const double share = (double)d.ntasks * mean_deg / (double)std::max<unsigned long long>(warps, 1) /
                              (d.vlab ? 256.0 : 1.0);
-        const uint32_t thr = tu.heavy_threshold ? tu.heavy_threshold : o.heavy_threshold;
         uint32_t split_H = thr ? std::max(thr, 4u * split_S)
                                : (uint32_t)std::min(1e9, std::max(32.0, share / 4.0));
+        // Three enumerated levels and a tail that is not inside the level-2 list:
+        // a root of fewer than two tasks is not worth its setup twice.
+        const bool inner = (d.parents[2] & 3u) == 3u && (d.tail_par & 7u) == 7u;
+        if (!thr && !L.want_stats && d.ne == 3 && !inner && !d.vlab) split_H = std::max(split_H, 2u * split_S);
         // three enumerated levels over N(m0) ∩ N(m1) with a tail inside it: a
         // root's work is the square of its list, which the share by list
         // length does not see (K4 over every root of R-MAT 2^18: one root ran
@@ -3179,8 +3211,8 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // per candidate, and splitting only repeats the setup (a triangle with
         // a tail there: 8.9 ms, split 11.9).  (A split root's repeated setup
         // would count in the instrumented kernel's totals.)
-        if (!thr && !L.want_stats && d.ne == 3 && (d.parents[2] & 3u) == 3u && (d.tail_par & 7u) == 7u)
-            split_H = std::min(split_H, std::max(8u * split_S, 256u));
+        if (!thr && !L.want_stats && d.ne == 3 && inner)
+            split_H = std::min(split_H, std::max(4u * split_S, 256u));
         // four enumerated levels and a leaf for every pair: under each level-2
         // candidate the pair step scans up to level 3's root list, so roots
         // and tasks are weighed by both bounds (two triangles joined by a
@@ -3196,11 +3228,18 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
         // 21.0).  On adjacency lists such a level is cut by intersections and
         // ends far below its bound: 78 seven-vertex plans on 3,300 roots of
         // R-MAT 2^22 15.3 -> 21.5 ms, K5 less an edge 1.7 -> 11.9.
-        if (!thr && !L.want_stats && d.ne == 4 && (d.pair ? !d.pair_direct : d.ntrie != 0) && (d.parents[3] & 3u)) {
+        // Where edges share few neighbours no bag has such a root (the two
+        // triangles on 4,000 roots of a random graph of degree 200: 1.6 ms, by
+        // both bounds 3.0).
+        if (!thr && !L.want_stats && d.ne == 4 && (d.pair ? !d.pair_direct : d.ntrie != 0) && (d.parents[3] & 3u) &&
+            !(d.ntrie && few_shared(g))) {
             d.split_par3 = d.parents[3] & 3u;
             d.split_W = (uint32_t)std::min(1e9, std::max(1024.0, share * mean_deg / 500.0));
         }
-        if (d.ne >= 3 && (g->max_deg > split_H || d.split_W)) {
+        const bool by_list = !thr && !L.want_stats && ((!d.vlab && d.ne == 3) || (few && d.split_W));
+        const unsigned long long most = (unsigned long long)g->max_deg * g->max_deg;
+        if (d.ne >= 3 && (g->max_deg > split_H || (d.split_W && most > 2ull * d.split_W))) {
+            d.split_list = by_list ? 1u : 0u;
             d.split_S = split_S;
             d.split_H = split_H;
             d.split_P3 = split_P3;
@@ -3703,6 +3742,7 @@ sge_status sge::graph_adopt(uint32_t *d_off, uint32_t *d_adj, uint32_t n, uint64
         h_off = off.data();
     }
     for (uint32_t v = 0; v < n; ++v) g->max_deg = std::max(g->max_deg, h_off[v + 1] - h_off[v]);
+    g->planner_stats = planner_stats;
     if (planner_stats) {
         // the wedge sample runs on the device; the host function is kept for
         // the graphs where its draws would differ
@@ -4194,7 +4234,7 @@ __global__ void __launch_bounds__(256) count_kernel_noalloc(DevGraph g, const De
             const uint32_t v = g.adj[e];
             if (P.root_kind == SGE_ROOT_ASC && !(u < v)) continue;
             if (P.root_kind == SGE_ROOT_DESC && !(u > v)) continue;
-            acc += run_root<MODE_PLAIN, true>(P, W, c, u, v);
+            acc += run_root<MODE_PLAIN, true>(P, W, c, u, v, 0u, 0xFFFFFFFFu, 0u, 1u, [](uint32_t) { return false; });
         }
     }
     if (cur >= 0 && lane == 0 && acc) atomicAdd(counts + cur, acc * plans[cur].mult);

@@ -65,3 +65,11 @@ def compare(sge, eng, name, limit, other, exploration=False, labels=None, **kw):
 @pytest.mark.parametrize("exploration", [False, True])
 def test_tail_in_one_list_is_not_split(sge, engines, exploration):
     compare(sge, engines("rmat"), "tailed_triangle", 1.15, dict(heavy_threshold=NO_SPLIT), exploration)
+
+
+# weighed by degrees, these took 4 and 4 to 6 times as long
+@pytest.mark.parametrize("exploration", [False, True])
+@pytest.mark.parametrize("name", ["near5clique_8e", "wheel4"])
+def test_roots_weigh_what_their_list_holds(sge, engines, name, exploration):
+    lists = dict(max_level_capacity=engines("sparse").info()["max_degree"])
+    compare(sge, engines("sparse"), name, 2.0, dict(heavy_threshold=NO_SPLIT), exploration, **lists)
