@@ -2106,7 +2106,8 @@ __device__ __forceinline__ uint32_t level2_bound(const DevGraph &g, const DevPla
 // of them (or at most that many) is deferred at all: by n2, or, where the level
 // below is scanned once per candidate (split_W), by n2 x that level's bound.
 // With split_list (automatic thresholds), n2 is the list that phase 0 has
-// built: degrees say little about it where few neighbours are shared.
+// built: degrees say little about it where few neighbours are shared or few
+// carry the label.
 struct RootSplit {
     uint32_t S, P3;   // level-2 candidates per task; parts of what is below one of them
     bool heavy;
@@ -2617,6 +2618,7 @@ struct sge_graph {
     uint32_t hub_words = 0, hub_min = 0xFFFFFFFFu, hub_count = 0;
     uint64_t hub_bytes = 0;
     uint32_t *d_labels = nullptr;  // vertex labels (sge_graph_set_labels)
+    std::vector<uint32_t> label_sample;  // sorted labels of up to 4,096 vertices drawn at random
     unsigned char *d_dense = nullptr;  // dense-root records and rows
     size_t dense_bytes = 0;
 };
@@ -3008,6 +3010,8 @@ double shared_neighbours(const sge_graph *g) {
 }
 // Few of them: level-2 lists are far shorter than the degrees that bound them.
 bool few_shared(const sge_graph *g) { return shared_neighbours(g) < 4.0; }
+// Degree of a root edge's end on average.
+double end_degree(const sge_graph *g) { return g->stats.moments[2] / std::max(g->stats.moments[1], 1.0); }
 
 // Chooses the plans whose dense roots are counted on bitsets and lays out
 // their buffer.  The instrumented kernel (its counters are defined on lists)
@@ -3070,6 +3074,14 @@ void prepare_dense(const sge_graph *g, const sge_count_opts &o, LaunchCfg &L) {
     L.dense_blocks = (size_t)g->num_sms * b;
 }
 
+// Share of the vertices that carry a label, from the sample (half a vertex of
+// it where none does).
+double label_share(const sge_graph *g, uint32_t label) {
+    const auto &s = g->label_sample;
+    const auto r = std::equal_range(s.begin(), s.end(), label);
+    return std::max<double>((double)(r.second - r.first), 0.5) / (double)std::max<size_t>(s.size(), 1);
+}
+
 sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t nplans, const sge_count_opts &o,
                           size_t scratch_held, LaunchCfg &L) {
     L.nplans = nplans;
@@ -3101,6 +3113,16 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
             if (!g->d_labels) return fail(SGE_BAD_INPUT, "plan %u is labeled but the graph has no labels (sge_graph_set_labels)", i);
             d.vlab = g->d_labels;
             for (uint32_t l = 0; l < d.k; ++l) d.lab[l] = plans[i]->labels[plans[i]->blob.order[l]];
+            // A pair step costs more than it flattens where both its levels are
+            // cut to a few vertices: houses with 2 labels on a random graph of
+            // degree 9 2.8 ms, with it 3.9.  Not where the first level is a
+            // whole list, or the second a long one (the same on one of degree
+            // 200: 344 and 105; 5-cycles with 8 labels on a Chung-Lu graph of
+            // mean degree 7: 5.5 and 3.0).
+            const auto one = [&](uint32_t l) { return (d.parents[l] & (d.parents[l] - 1u)) == 0; };
+            if (d.pair && few_shared(g) && !one(d.ne - 2) &&
+                !(one(d.ne - 1) && end_degree(g) * label_share(g, d.lab[d.ne - 1]) >= 64.0))
+                d.pair = d.pair_direct = 0;
         }
         if (d.k > SGE_MAX_K) return fail(SGE_UNSUPPORTED, "plan %u has k=%u", i, d.k);
     }
@@ -3190,20 +3212,38 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
             : (uint32_t)std::min<unsigned long long>(128, std::max<unsigned long long>(8, 2ull * d.ntasks / warps));
         const uint32_t thr = tu.heavy_threshold ? tu.heavy_threshold : o.heavy_threshold;
         // Roots weighed by the list that phase 0 has built (split_list) where
-        // that says more than the degrees: with three enumerated levels, and
-        // where edges share few neighbours.  Hubs elsewhere make work that a
-        // short list does not show (8-edge near-5-cliques on 30,000 roots of
-        // R-MAT 2^18: 10 ms by degrees, 38 by the list).
+        // that says more than the degrees: with three enumerated levels, where
+        // edges share few neighbours, and for labeled plans also on graphs
+        // without hubs, where all later levels lie inside that list, and where
+        // the labels are rare and every level is cut by two lists (octahedra
+        // with 32 labels on R-MAT 2^14: 22 ms by degrees, 1.7 by the list).
+        // Hubs elsewhere make work that a short list does not show (8-edge
+        // near-5-cliques on 30,000 roots of R-MAT 2^18: 10 ms by degrees, 38 by
+        // the list; octahedra with 2 labels on a 7,100-vertex Chung-Lu graph:
+        // 102 and 340).
+        bool inside = true;
+        for (uint32_t i = 3; i < d.k; ++i) inside &= (d.parents[i] & 7u) == 7u;
         const bool few = few_shared(g);
-        // (labels leave few of the roots: one in 256 is taken for granted)
-        const double share = (double)d.ntasks * mean_deg / (double)std::max<unsigned long long>(warps, 1) /
-                             (d.vlab ? 256.0 : 1.0);
+        const double ends = d.vlab ? label_share(g, d.lab[0]) * label_share(g, d.lab[1]) : 1.0;
+        const bool own = d.vlab && (d.ne == 3 || few || inside || g->max_deg < 4.0 * end_degree(g));
+        const bool rare = d.vlab && split3 && !dense_wide(d) && ends < 1.0 / 256;
+        // (a labeled plan's list holds its label alone, unless later levels
+        // reuse it; otherwise one root in 256 is taken to carry its labels)
+        const double share = (double)d.ntasks * mean_deg / (double)std::max<unsigned long long>(warps, 1) *
+                             (!d.vlab || own ? ends : 1.0 / 256.0);
+        const double kept = own ? label_share(g, d.lab[2]) : 1.0, seen = (d.keep_full >> 2) & 1u ? kept : 1.0;
+        const double part = d.vlab && d.ne == 3 ? 16.0 : 4.0;   // of a warp's share
         uint32_t split_H = thr ? std::max(thr, 4u * split_S)
-                               : (uint32_t)std::min(1e9, std::max(32.0, share / 4.0));
+                               : (uint32_t)std::min(1e9, std::max(32.0, share * kept / part) / seen);
         // Three enumerated levels and a tail that is not inside the level-2 list:
-        // a root of fewer than two tasks is not worth its setup twice.
+        // a root of fewer than two tasks is not worth its setup twice, nor are
+        // the few roots that some labels leave (triangles with a tail, 8 labels
+        // on R-MAT 2^14: 0.8 ms, split 1.4; on 2^18 9.8 and 6.1).
         const bool inner = (d.parents[2] & 3u) == 3u && (d.tail_par & 7u) == 7u;
-        if (!thr && !L.want_stats && d.ne == 3 && !inner && !d.vlab) split_H = std::max(split_H, 2u * split_S);
+        if (!thr && !L.want_stats && d.ne == 3 && !inner) {
+            if (!d.vlab) split_H = std::max(split_H, 2u * split_S);
+            else if ((double)d.ntasks * ends < 2.0 * warps) split_H = 1u << 30;
+        }
         // three enumerated levels over N(m0) ∩ N(m1) with a tail inside it: a
         // root's work is the square of its list, which the share by list
         // length does not see (K4 over every root of R-MAT 2^18: one root ran
@@ -3236,7 +3276,7 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
             d.split_par3 = d.parents[3] & 3u;
             d.split_W = (uint32_t)std::min(1e9, std::max(1024.0, share * mean_deg / 500.0));
         }
-        const bool by_list = !thr && !L.want_stats && ((!d.vlab && d.ne == 3) || (few && d.split_W));
+        const bool by_list = !thr && !L.want_stats && (own || rare || (!d.vlab && d.ne == 3) || (few && d.split_W));
         const unsigned long long most = (unsigned long long)g->max_deg * g->max_deg;
         if (d.ne >= 3 && (g->max_deg > split_H || (d.split_W && most > 2ull * d.split_W))) {
             d.split_list = by_list ? 1u : 0u;
@@ -3869,8 +3909,13 @@ sge_status sge_graph_set_labels(sge_graph *g, const uint32_t *labels) {
     if (!labels) {
         cudaFree(g->d_labels);
         g->d_labels = nullptr;
+        g->label_sample.clear();
         return SGE_OK;
     }
+    const uint64_t some = std::min<uint64_t>(g->n, 4096);
+    g->label_sample.resize(some);
+    for (uint64_t i = 0; i < some; ++i) g->label_sample[i] = labels[splitmix64(i) % g->n];
+    std::sort(g->label_sample.begin(), g->label_sample.end());
     if (!g->d_labels) CUDA_TRY(cudaMalloc(&g->d_labels, 4ull * std::max<uint32_t>(g->n, 1)));
     CUDA_TRY(cudaMemcpy(g->d_labels, labels, 4ull * g->n, cudaMemcpyHostToDevice));
     return SGE_OK;

@@ -73,3 +73,13 @@ def test_tail_in_one_list_is_not_split(sge, engines, exploration):
 def test_roots_weigh_what_their_list_holds(sge, engines, name, exploration):
     lists = dict(max_level_capacity=engines("sparse").info()["max_degree"])
     compare(sge, engines("sparse"), name, 2.0, dict(heavy_threshold=NO_SPLIT), exploration, **lists)
+
+
+# one root in 256 taken to carry the labels: 10 to 100 times as long
+@pytest.mark.parametrize("labels", [2, 8, 32])
+@pytest.mark.parametrize("graph", ["sparse", "uniform", "rmat"])
+def test_labeled_roots_are_split_by_their_share(sge, engines, graph, labels):
+    eng = engines(graph)
+    eng.set_labels(np.random.default_rng(3).integers(0, labels, eng.info()["num_vertices"]))
+    for name in ("k5", "wheel4", "octahedron") if graph != "rmat" else ("k5",):
+        compare(sge, eng, name, 2.5, dict(heavy_threshold=NO_SPLIT), labels=labels)
