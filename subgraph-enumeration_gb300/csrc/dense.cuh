@@ -69,6 +69,7 @@ struct DenseBuf {
     unsigned long long arena_units;  // 16-byte units
     uint32_t rec_cap, npo, need;     // need: classes any plan of the launch uses
     uint32_t rows_both;              // classes whose plans only read rows of N(u) ∩ N(v)
+    uint32_t rich;                   // classes of plans that lists serve badly: rows for all roots but the smallest
 };
 
 // Segment sizes of class c and the word each segment starts at.
@@ -110,14 +111,22 @@ __device__ __forceinline__ DenseView dense_view(const DenseBuf &D, const DenseRe
 // which a root with few common neighbours and no wider universe earns back
 // only from about 8 of them on (K5 over every root of a 7,100-vertex
 // Chung-Lu graph: lists 9.2 ms, from 2 on 8.3 ms, 8 on 7.1 ms, 24 on 6.4 ms;
-// of a 1,500-vertex one: 0.73, 0.27, 0.24, 0.50 ms).  The list path knows only
-// the degrees before it starts: it splits a root between two large lists into
-// thousands of tasks even when one common neighbour is in them, and with a
-// wider universe it scans N(m0) or N(m1) below every partial match, so there
-// one common neighbour pays (78 seven-vertex patterns on R-MAT 2^22: 21 ms,
-// from 8 on 46 ms, 24 on 72 ms, lists 1,010 ms).
-__device__ __forceinline__ bool dense_worth(uint32_t c, uint32_t n2, uint32_t mindeg, uint32_t words) {
-    return n2 >= DENSE_MIN_N2 || mindeg >= DENSE_MIN_DEG || (c != DENSE_BOTH && (n2 >= 2 || words >= DENSE_MIN_WORDS));
+// of a 1,500-vertex one: 0.73, 0.27, 0.24, 0.50 ms), and not while both lists
+// are one step of a warp (a ring lattice of degree 24: 39 ms, with rows 45).
+// The list path knows only the degrees before it starts: it splits a root
+// between two large lists into thousands of tasks even when one common
+// neighbour is in them, and with a wider universe it scans N(m0) or N(m1) below
+// every partial match, so there one common neighbour pays (78 seven-vertex
+// patterns on R-MAT 2^22: 21 ms, from 8 on 46 ms, 24 on 72 ms, lists 1,010 ms).
+// Where edges share few neighbours, lists are not split and every level is cut
+// by two of them (D.rich clear), a plan matches some n2^2 / 2 prefixes, which
+// have to make up for |U| rows (octahedra and 4-wheels on a Chung-Lu graph of
+// mean degree 7: lists 1.8 and 2.1 ms, rows for all 14.7 and 15.3).
+__device__ __forceinline__ bool dense_worth(const DenseBuf &D, uint32_t c, uint32_t n2, uint32_t du, uint32_t dv,
+                                            uint32_t words) {
+    if (!((D.rich >> c) & 1u)) return n2 >= DENSE_MIN_N2 && max(du, dv) > 32u && (c == DENSE_BOTH || n2 * n2 >= 32u * words);
+    return min(du, dv) >= DENSE_MIN_DEG || (n2 >= DENSE_MIN_N2 && max(du, dv) > 32u) ||
+           (c != DENSE_BOTH && (n2 >= 2 || words >= DENSE_MIN_WORDS));
 }
 // Tasks of a record per (plan, orientation): large universes split each
 // level-2 candidate into 2^s parts of its level-3 list (the positions = q mod
@@ -185,7 +194,7 @@ __global__ void __launch_bounds__(256) dense_select_kernel(DevGraph g, unsigned 
         uint32_t have = 0;
         for (uint32_t c = 0; c < 4; ++c) {
             const uint32_t words = dense_shape(c, n2, du, dv).w3;
-            if (((D.need >> c) & 1u) && words <= DENSE_WORDS && dense_worth(c, n2, min(du, dv), words)) { units += dense_units(words); have |= 1u << c; }
+            if (((D.need >> c) & 1u) && words <= DENSE_WORDS && dense_worth(D, c, n2, du, dv, words)) { units += dense_units(words); have |= 1u << c; }
         }
         if (!have) continue;
         unsigned long long at = atomicAdd(reinterpret_cast<unsigned long long *>(D.hdr + 2), units);

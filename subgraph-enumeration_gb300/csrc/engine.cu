@@ -2962,7 +2962,7 @@ struct LaunchCfg {
     // dense roots (dense.cuh): the plans' universe classes and the layout of their buffer
     // (header | edge classes | records | order | prefix | (plan, orientation) table | rows)
     std::vector<DensePO> dpo;           // empty: every root is counted on lists
-    uint32_t dslots = 1, dneed = 0, drows_both = 0, drec_cap = 0, dmaxdeg = 0;
+    uint32_t dslots = 1, dneed = 0, drows_both = 0, drec_cap = 0, dmaxdeg = 0, drich = 0;
     unsigned long long dedges = 0, darena_units = 0, droot_offset = 0, droot_stride = 1;
     size_t dense_blocks = 0, off_dskip = 256, off_drecs = 0, off_dorder = 0, off_dpre = 0, off_dpo = 0, off_darena = 0, dense_bytes = 0;
 };
@@ -3024,6 +3024,17 @@ void prepare_dense(const sge_graph *g, const sge_count_opts &o, LaunchCfg &L) {
         DevPlan &d = L.dps[i];
         const int c = dense_class(d);
         if (c < 0) continue;
+        // Where edges share few neighbours and the list path splits no root by degrees, a
+        // root's rows are more than that ever reads of them, and selecting
+        // roots repeats the triangle count that is most of its work (K5 on a
+        // random graph of degree 200: lists 12.8, selected 16.8 ms).  Where next
+        // to none have any, selecting is the faster way to leave them out (on
+        // one of degree 9: 4.0 and 3.1 ms), and rows are for the others
+        // (dense_worth).  A plan with a level over all of N(m0) or N(m1) reads
+        // its rows all the same (prisms on a Chung-Lu graph of mean degree 7:
+        // lists 117 ms, rows 4.6).
+        const bool thin = few_shared(g) && (!d.split_S || d.split_list) && !dense_wide(d);
+        if (thin && shared_neighbours(g) >= 0.5) continue;
         d.dcls = (uint8_t)(c + 1);
         const bool both = dense_rows_both(d);
         for (uint32_t swap = 0; swap < 2; ++swap) {
@@ -3031,6 +3042,7 @@ void prepare_dense(const sge_graph *g, const sge_count_opts &o, LaunchCfg &L) {
             const uint32_t ec = dense_edge_class((uint32_t)c, swap != 0);
             L.dpo.push_back(DensePO{i, ec, swap});
             L.dneed |= 1u << ec;
+            if (!thin) L.drich |= 1u << ec;
             if (!both) L.drows_both &= ~(1u << ec);
         }
         L.droot_offset = d.root_offset;
@@ -3350,6 +3362,7 @@ sge_status enqueue_launch(sge_graph *g, const LaunchCfg &L, unsigned char *B, ui
         D.npo = (uint32_t)L.dpo.size();
         D.need = L.dneed;
         D.rows_both = L.drows_both;
+        D.rich = L.drich;
         dskip = D.skip;
         CUDA_TRY(cudaMemsetAsync(dense, 0, L.off_dskip + L.dedges, s));
         const unsigned sel = (unsigned)std::min<unsigned long long>((L.dedges + 7) / 8, 16ull * g->num_sms);

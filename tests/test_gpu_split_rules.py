@@ -83,3 +83,13 @@ def test_labeled_roots_are_split_by_their_share(sge, engines, graph, labels):
     eng.set_labels(np.random.default_rng(3).integers(0, labels, eng.info()["num_vertices"]))
     for name in ("k5", "wheel4", "octahedron") if graph != "rmat" else ("k5",):
         compare(sge, eng, name, 2.5, dict(heavy_threshold=NO_SPLIT), labels=labels)
+
+
+# rows for every root: 1.3 to 8 times as long
+@pytest.mark.parametrize("exploration", [False, True])
+@pytest.mark.parametrize("graph,name,limit", [("sparse", "octahedron", 2.0), ("sparse", "wheel4", 2.0),
+                                              ("sparse", "k5", 1.4), ("uniform", "octahedron", 1.3),
+                                              ("uniform", "k5", 1.2)])
+def test_rows_only_where_edges_share_neighbours(sge, engines, graph, name, limit, exploration):
+    eng = engines(graph)
+    compare(sge, eng, name, limit, dict(max_level_capacity=eng.info()["max_degree"]), exploration)
