@@ -385,8 +385,13 @@ __device__ __forceinline__ void trim(const uint32_t *&p, uint32_t &len, const Bo
 // What a build of the counting code holds: the instrumented counters, and
 // labeled plans and bag relations.  Most launches have neither; compiled in,
 // their branches cost the pair step registers (the 12 plans of a 7,100-vertex
-// Chung-Lu graph: 30.9 ms with them, 30.1 ms without).
-enum { MODE_FULL = 0, MODE_STATS = 1, MODE_PLAIN = 2 };
+// Chung-Lu graph: 30.9 ms with them, 30.1 ms without).  Plain launches whose
+// plans have no inline tail, or no pair step at all, or whose inline tails
+// would scan short lists (MODE_FLAT: no scan per x), leave that code out too:
+// it does not run there, but a longer body misses the instruction cache (a
+// triangle with a tail over R-MAT 2^16: 8.2 of 20 stalled cycles per
+// instruction with it).
+enum { MODE_FULL = 0, MODE_STATS = 1, MODE_PLAIN = 2, MODE_NODIRECT = 4, MODE_NOPAIR = 8, MODE_NOTRIES = 16, MODE_FLAT = 32 };
 template <int M>
 constexpr bool stats_of = (M & MODE_STATS) != 0;
 template <int M>
@@ -395,7 +400,7 @@ __device__ __forceinline__ const uint32_t *labels_of(const DevPlan &P) {
 }
 template <int M>
 __device__ __forceinline__ uint32_t ntrie_of(const DevPlan &P) {
-    return (M & MODE_PLAIN) ? 0u : P.ntrie;
+    return (M & (MODE_PLAIN | MODE_NOTRIES)) ? 0u : P.ntrie;
 }
 
 template <int M>
@@ -517,7 +522,7 @@ __device__ __forceinline__ void unpin_root(const DevPlan &P, WarpState &W, Ctx<M
     for (uint32_t j = 0; j < 2; ++j)
         if (W.pmode[j]) unpin_list(W, c, j, W.lptr[j], W.llen[j]);
     if (W.pmode[2]) {
-        if (!(M & MODE_PLAIN) && W.tpin) {
+        if (!(M & (MODE_PLAIN | MODE_NOTRIES)) && W.tpin) {
             const DevTrie &T = P.tries[P.trel[W.tpin - 1]];
             unpin_list(W, c, 2, T.val[T.nkeys] + W.toff[W.tpin - 1], W.tlen[W.tpin - 1]);
         } else if (W.hpin && P.join_style == SGE_JOIN_EXPLORATION)
@@ -1650,7 +1655,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
     // inline tail: the tail level's single list does not depend on y, so the
     // pair's count is x's count minus y itself when y is in x's range and list
     bool inl = false;
-    if (P.pair_direct) {
+    if (!(M & MODE_NODIRECT) && P.pair_direct) {
         if (lane == 0) {
             const LeafCtx lc{a, P.join_style == SGE_JOIN_EXPLORATION};
             tail_desc(P, W, *c.L, c, lc, P.ne, S.ptd);
@@ -1661,7 +1666,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
     // (a stored list, as N(m0) ∩ N(m1), is short: a scan per x would leave most
     // lanes idle, so those plans stay with the flattened step; an 8-edge
     // near-5-clique on a 7,100-vertex Chung-Lu graph: 1.0 ms, 1.3 per x)
-    if (!stats_of<M> && inl && parts == 1 && P.base[i] < 0 && S.ns + S.xpar <= 2 && (S.ns == 0 || S.slen[0] >= 64u))
+    if (!stats_of<M> && !(M & (MODE_NODIRECT | MODE_FLAT)) && inl && parts == 1 && P.base[i] < 0 && S.ns + S.xpar <= 2 && (S.ns == 0 || S.slen[0] >= 64u))
     {
         if (S.ns == 1 && S.xpar && S.stab[0] >= 0 && S.ptd.kind[0] < 3 && c.tmode == 1 && W.pmode[S.stab[0]] == 1 &&
             W.pmode[S.ptd.kind[0]] == 1 && c.g.hub_words <= c.tw && c.g.hub_min != 0xFFFFFFFFu && !labels_of<M>(P) &&
@@ -1800,7 +1805,7 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
             return keep;
         };
         // 3. flattened scan; an inline tail is summed on the spot ...
-        if (inl) {
+        if (!(M & MODE_NODIRECT) && inl) {
             for (uint32_t j0 = begin; j0 < total; j0 += 32) {
                 if (j0 && (j0 & 0x1FFFu) == 0 && out_of_time(c)) { ok = false; break; }
                 const uint32_t j = j0 + lane;
@@ -1951,7 +1956,7 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
         __syncwarp();
     }
     while (ok) {
-        if (lv == Lt && P.pair) {
+        if (!(M & MODE_NOPAIR) && lv == Lt && P.pair) {
             ok = pair_level(P, W, c, lv, acc, p3, lv == 2 ? np3 : 1u);
             if (lv == 2) break;
             --lv;
@@ -2011,7 +2016,7 @@ __device__ __forceinline__ unsigned long long run_root(const DevPlan &P, WarpSta
         }
         __syncwarp();
     }
-    if (P.pin_mask || W.hpin || (!(M & MODE_PLAIN) && W.tpin)) unpin_root(P, W, c);
+    if (P.pin_mask || W.hpin || (!(M & (MODE_PLAIN | MODE_NOTRIES)) && W.tpin)) unpin_root(P, W, c);
     if (ntrie_of<M>(P)) {
         __syncwarp();
         if (lane == 0) W.troot = 0;
@@ -3148,12 +3153,24 @@ sge_status prepare_launch(sge_graph *g, const sge_plan *const *plans, uint32_t n
     else if (o.pin_tables == 2 || !g->d_hub_bits || o.no_hub_bitmaps) { L.tmode = 2; L.tw = 512; }
     else { L.tmode = 0; L.tw = 0; }
     L.want_stats = o.collect_counters != 0;
-    bool plain = true;
+    bool plain = true, tries = false, pair = false, direct = false;
     for (auto &d : L.dps) {
         d.root_maxdeg = o.root_max_degree;
         plain &= !d.vlab && !d.ntrie;
+        tries |= d.ntrie != 0;
+        pair |= d.pair != 0;
+        direct |= d.pair_direct != 0;
     }
-    L.kern = L.want_stats ? count_kernel<MODE_STATS> : plain ? count_kernel<MODE_PLAIN> : count_kernel<MODE_FULL>;
+    // (bulls on a ring lattice of degree 120 without shared-memory tables in
+    // reach: 102 ms, 115 with the scans per x in the build)
+    const bool flat = end_degree(g) < 128.0 && L.tmode != 1;
+    L.kern = L.want_stats ? count_kernel<MODE_STATS>
+             : tries      ? count_kernel<MODE_FULL>
+             : !plain     ? (pair ? count_kernel<MODE_NOTRIES> : count_kernel<MODE_NOTRIES | MODE_NODIRECT | MODE_NOPAIR>)
+             : !pair      ? count_kernel<MODE_PLAIN | MODE_NODIRECT | MODE_NOPAIR>
+             : !direct    ? count_kernel<MODE_PLAIN | MODE_NODIRECT>
+             : flat       ? count_kernel<MODE_PLAIN | MODE_FLAT>
+                          : count_kernel<MODE_PLAIN>;
     L.use_hubs = o.no_hub_bitmaps == 0;
     // warps per block: 4 or 2, whichever keeps more warps resident per SM
     // (shared memory per warp is several KB, so smaller blocks pack better)
