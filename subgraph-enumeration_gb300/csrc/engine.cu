@@ -1665,8 +1665,12 @@ __device__ __forceinline__ bool pair_level(const DevPlan &P, WarpState &W, Ctx<M
     }
     // (a stored list, as N(m0) ∩ N(m1), is short: a scan per x would leave most
     // lanes idle, so those plans stay with the flattened step; an 8-edge
-    // near-5-clique on a 7,100-vertex Chung-Lu graph: 1.0 ms, 1.3 per x)
-    if (!stats_of<M> && !(M & (MODE_NODIRECT | MODE_FLAT)) && inl && parts == 1 && P.base[i] < 0 && S.ns + S.xpar <= 2 && (S.ns == 0 || S.slen[0] >= 64u))
+    // near-5-clique on a 7,100-vertex Chung-Lu graph: 1.0 ms, 1.3 per x.  Where
+    // the scan does not hold N(x), it is the same list for every x and pays from
+    // a longer one on: bulls on a ring lattice of degree 120, 102 ms, 118 per x;
+    // on 30,000 roots of R-MAT 2^18 188 and 65 ms)
+    if (!stats_of<M> && !(M & (MODE_NODIRECT | MODE_FLAT)) && inl && parts == 1 && P.base[i] < 0 && S.ns + S.xpar <= 2 &&
+        (S.ns == 0 || S.slen[0] >= (S.xpar ? 64u : 256u)))
     {
         if (S.ns == 1 && S.xpar && S.stab[0] >= 0 && S.ptd.kind[0] < 3 && c.tmode == 1 && W.pmode[S.stab[0]] == 1 &&
             W.pmode[S.ptd.kind[0]] == 1 && c.g.hub_words <= c.tw && c.g.hub_min != 0xFFFFFFFFu && !labels_of<M>(P) &&
