@@ -562,6 +562,13 @@ sge_status sge_sort_tuples(uint32_t *d_tuples, uint64_t n, uint32_t arity) {
     if ((!d_tuples && n) || arity == 0 || arity > MAX_ARITY) return fail(SGE_BAD_INPUT, "sge_sort_tuples: bad argument");
     if (n <= 1) return SGE_OK;
     if (n >= (1ull << 32)) return fail(SGE_UNSUPPORTED, "sge_sort_tuples: more than 2^32 rows");
+    if (arity == 1 && n <= (1ull << 20)) {
+        // a short column: its width saves less than finding it costs (100,000
+        // values of 31 bits 0.38 ms with the look, 0.28 without)
+        Widths w{};
+        w.bits[0] = 32;
+        return sort_packed<Key64>(d_tuples, n, arity, w, 32);
+    }
     uint32_t *d_or = nullptr, h_or[MAX_ARITY] = {};
     CUDA_TRY(cudaMalloc(&d_or, sizeof h_or));
     cudaError_t e = cudaMemset(d_or, 0, sizeof h_or);
