@@ -502,7 +502,6 @@ def run_rmat22(args):
     d2h = 8 * len(plans) + 4
     peak, peak_kind = peaks()
     traffic = profile_traffic("count_kernel_rmat22-sample.md")  # DRAM bytes of one step, measured by ncu
-    achieved = traffic / avg_s / 1e9 if traffic else None
     line = {
         "metric": METRIC, "value": value, "unit": "embeddings/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": sum_k / len(kernel_ms), "higher_is_better": True,
@@ -526,15 +525,13 @@ def run_rmat22(args):
         "speedup_wall": pw / lw, "speedup_kernel": pk / lk,
         "kernel_ms_without_hub_bitmaps": snh["kernel_ms"],
         "total_count": total,
-        "roofline": {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak if traffic else None, "peak_kind": peak_kind, "traffic": traffic,
-                     "dram_gbs": traffic / avg_s / 1e9 if traffic else None,
-                     "dram_frac": traffic / avg_s / 1e9 / peak if traffic else None,
+        "roofline": {"bound": "latency", "achieved": None, "peak": peak, "unit": "GB/s",
+                     "frac": None, "peak_kind": peak_kind, "traffic": traffic,
                      "alg_bytes_per_launch": sst["alg_bytes"],
                      "note": "one step = the batched launch sequence (bit rows of the dense roots: select, build, "
-                             "prefix, count; the other roots on lists: phase 0, task numbering, phase 1); achieved = "
-                             "traffic = ncu DRAM read+write of the same step (profiles/count_kernel_rmat22-sample.md) "
-                             "over the step's time. alg_bytes_per_launch is what the same counts take on lists, summed "
+                             "prefix, count; the other roots on lists: phase 0, task numbering, phase 1); traffic = "
+                             "the DRAM bytes of one step that ncu counted for profiles/count_kernel_rmat22-sample.md, "
+                             "not of this run, so no rate is derived. alg_bytes_per_launch is what the same counts take on lists, summed "
                              "by the instrumented kernel (4 B per scanned element + per probed list 4 B per probe "
                              "through a hub bitmap or pinned table, else the list as a merge consumes it, + 8 B "
                              "offsets): the bit rows replace most of it. Rows and running masks stay in L1/L2 and "

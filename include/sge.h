@@ -178,8 +178,9 @@ typedef struct sge_count_opts {
     uint32_t collect_counters;  /* 1: run the instrumented kernel (set_ops, alg_bytes, partial matches) */
     uint32_t heavy_threshold;   /* 0 = auto (a quarter of a warp's share of the launch's level-2
                                    candidates, at least 32; less where a root's work grows with the
-                                   square of that list, and by the bounds of levels 2 and 3 together
-                                   where level 3 is scanned once per candidate); otherwise roots whose
+                                   square of that list, and by levels 2 and 3 together where level 3 is
+                                   scanned once per candidate; the level-2 list itself is weighed or its
+                                   bound, whichever tells more of the work); otherwise roots whose
                                    level-2 list may exceed it are deferred to a second launch that
                                    splits each into tasks of one level-2 candidate and a part of its
                                    level-3 list (or, where level 3 is not enumerated, of 8 to 128 level-2

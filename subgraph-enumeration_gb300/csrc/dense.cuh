@@ -20,7 +20,7 @@
 // the rows of a root (at most 0.5 MB) stay in L1/L2.  Kernel time, lists ->
 // rows: 78 seven-vertex patterns (16-19 edges) on 488 root edges of R-MAT 2^22
 // 1,010 -> 17 ms; 16 six-vertex patterns on 976 root edges of R-MAT 2^20
-// 20.7 -> 2.0 ms; K5 over every root of R-MAT 2^14 172 -> 87 ms.
+// 20.7 -> 2.0 ms; K5 over every root of R-MAT 2^14 172 -> 97 ms.
 //
 // Included by engine.cu inside its anonymous namespace.
 #pragma once
