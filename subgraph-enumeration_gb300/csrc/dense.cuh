@@ -763,6 +763,8 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
         bool ok = true;
         for (uint32_t p2 = c0; p2 < c1 && ok; ++p2) {   // (common neighbours are the first positions)
             if (!((S.run(dense_slot(1, 2))[p2 >> 5] >> (p2 & 31u)) & 1u)) continue;
+            // (the leaves under one candidate's part, a few hundred at most, are not
+            // cut: a look at the clock at each cost 0.4 % of a batch)
             if (out_of_time(c)) { ok = false; break; }
             dense_match(S, V, k, 2, p2);
             if (ne == 4) {
@@ -776,12 +778,12 @@ __global__ void __launch_bounds__(128, 8) dense_count_kernel(const DevPlan *__re
                     if (--lv < 3) break;
                     continue;
                 }
-                if (out_of_time(c)) { ok = false; break; }
                 dense_match(S, V, k, lv, p);
                 if (lv + 2 == ne) {
                     dense_leaf(P, S, V, lv, acc, flags);
                     continue;
                 }
+                if (out_of_time(c)) { ok = false; break; }
                 ++lv;
             }
         }
